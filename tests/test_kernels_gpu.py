@@ -516,6 +516,33 @@ def test_argmax_takes_the_first_of_a_tie(ops):
     assert got.tolist() == torch.argmax(logits, dim=-1).tolist() and got[2].item() == 5
 
 
+@pytest.mark.parametrize("vocab", [37, 4093, 20011])
+@pytest.mark.parametrize("levels", [0, 9])
+def test_sampling_by_every_route(ops, vocab, levels):
+    """top_k around the sizes at which the draw changes its way (few candidates that one block finishes, more
+    than it holds, more than the bound allows), alone and with top_p, and top_p over more tokens than a block
+    lists; `levels`: logits of so many values, so that ties reach over every limit (a tie at the k-th largest is
+    kept whole). One of the rows holds an infinite logit and one starts off 16 bytes."""
+    cases = [(1, 1.0), (8, 0.5), (9, 1.0), (50, 0.95), (480, 1.0), (700, 0.9), (2048, 0.7), (2049, 1.0), (0, 0.6), (0, 0.995)]
+    rows = len(cases)
+    logits = rand(rows, vocab + 1, scale=2.0, seed=vocab)[:, 1:]
+    if levels:
+        logits = (logits.float() * 0.5).round().clamp(-levels, levels)
+    logits = logits.float().clone()
+    logits[3, vocab // 2] = float("inf")
+    wide = torch.empty(rows, vocab + 3, device="cuda")  # rows of another stride, off 16 bytes
+    strided = wide[:, 2: 2 + vocab]
+    strided.copy_(logits)
+    dev = lambda v, dt: torch.tensor(v, dtype=dt, device="cuda")
+    args = (dev([0.7] * rows, torch.float32), dev([k for k, _ in cases], torch.int32), dev([p for _, p in cases], torch.float32),
+            dev([0.0, 0.02] * (rows // 2), torch.float32), dev(list(range(rows)), torch.int64), dev([5] * rows, torch.int64))
+    finite = [r for r in range(rows) if r != 3]
+    expect = kernel_refs.sample(logits[finite], *(a[finite] for a in args)).tolist()
+    got = ops.sample(logits.clone(), *args)
+    assert got[finite].tolist() == expect
+    assert ops.sample(strided, *args).tolist() == got.tolist()
+
+
 def test_sampling_keeps_exactly_the_filtered_set(ops):
     """Many draws never leave the set that top_k/top_p/min_p keep, and reach all of it."""
     vocab = 300
