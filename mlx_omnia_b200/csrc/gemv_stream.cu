@@ -152,14 +152,24 @@ __device__ __forceinline__ int tile_row(int tile, int r, int n, int inner) {
   return row < n ? row : -1;
 }
 
+// Grouped form: the matrices of many experts one under another, and a list of (expert, first sorted row, rows)
+// made on the device, each entry of at most NT * 8 rows. A block's run of tiles goes through the entries' matrices
+// one after another; tiles that share a fetch of the activations belong to one entry.
+struct Grouped {
+  const int* entries;  // [count, 3]
+  const int* count;
+  const int* source;  // sorted row r reads activation row source[r] (null: r)
+  int per_entry;      // tiles of a matrix
+};
+
 // NT: activation tiles of 8 rows (1 for m <= 8, 2 for m <= 16).
 __host__ __device__ constexpr size_t partial_bytes(int nt) { return sizeof(float) * CONSUMER_WARPS * GROUP_TILES * TILE_ROWS * (nt * 8 + 1); }
 
-template <int NT, int EPI, bool PENDING>
+template <int NT, int EPI, bool PENDING, bool GROUPED>
 __global__ void __launch_bounds__(THREADS, 1)
 gemv_stream_kernel(const bf16* __restrict__ a, const __grid_constant__ CUtensorMap map_w, void* __restrict__ out,
                    int m, int n, int k, int inner, int tiles, float multiplier, float cap, float second, const PendingStep pending,
-                   int* __restrict__ err) {
+                   const Grouped grouped, int follows, int* __restrict__ err) {
   extern __shared__ __align__(128) unsigned char smem[];
   unsigned char* ring = smem;
   float (*partial)[GROUP_TILES * TILE_ROWS][NT * 8 + 1] =
@@ -184,6 +194,11 @@ gemv_stream_kernel(const bf16* __restrict__ a, const __grid_constant__ CUtensorM
   }
   __syncthreads();
 
+  if (GROUPED) {
+    // The list comes from a kernel before the one before (`follows` says so) or from the one before.
+    if (!follows) pdl_wait();
+    tiles = __ldcg(grouped.count) * grouped.per_entry;
+  }
   // This block's tiles: a contiguous run, sizes differing by at most one between blocks. They
   // are worked on in groups of GROUP_TILES: for every 1024 columns, the stages of all tiles of
   // the group follow one another, so a warp fetches its activations of those columns once per
@@ -192,19 +207,29 @@ gemv_stream_kernel(const bf16* __restrict__ a, const __grid_constant__ CUtensorM
   const int my_tiles = base + ((int)blockIdx.x < extra ? 1 : 0);
   const int tile0 = blockIdx.x * base + min((int)blockIdx.x, extra);
   const int chunks = (k + STAGE_COLS - 1) / STAGE_COLS;
+  // How many tiles are worked on together from tile `first` of the run on.
+  auto together = [&](int first) {
+    const int count = min(GROUP_TILES, my_tiles - first);
+    return GROUPED ? min(count, grouped.per_entry - (tile0 + first) % grouped.per_entry) : count;
+  };
 
   if (warp == CONSUMER_WARPS) {
     // ---- producer: needs nothing from the kernel before, so it does not wait for it ----
     int s = 0, phase = 1, in_flight = 0;
     bool ok = true;
-    for (int first = 0; first < my_tiles && ok; first += GROUP_TILES) {
-      const int count = min(GROUP_TILES, my_tiles - first);
+    for (int first = 0, count; first < my_tiles && ok; first += count) {
+      count = together(first);
+      int matrix0 = 0, in_matrix = tile0 + first;  // the matrix's first row, and the tile's place in it
+      if (GROUPED) {
+        matrix0 = __ldcg(grouped.entries + 3 * (in_matrix / grouped.per_entry)) * n;
+        in_matrix %= grouped.per_entry;
+      }
       for (int c = 0; c < chunks && ok; ++c)
         for (int i = 0; i < count; ++i) {
           if (lane == 0) ok = mbar_wait(empty0 + 8 * s, phase, abort_flag);
           ok = __shfl_sync(0xffffffffu, ok, 0);
           if (!ok) break;
-          const int tile = tile0 + first + i;
+          const int tile = in_matrix + i;
           // Lane i copies box i of the stage: half i / BOXES_ACROSS (rows g, then rows g + 8) and
           // 256 columns. A box that starts outside the matrix is not copied (its rows and columns
           // are masked by the consumers); one that straddles an edge is filled with zeros there.
@@ -214,11 +239,12 @@ gemv_stream_kernel(const bf16* __restrict__ a, const __grid_constant__ CUtensorM
           const unsigned live = __ballot_sync(0xffffffffu, copies);
           if (lane == 0) mbar_expect_tx(full0 + 8 * s, (uint32_t)__popc(live) * BOX_BYTES);
           __syncwarp();
-          if (copies) tma_load_2d(smem_u32(ring + s * STAGE_BYTES + lane * BOX_BYTES), &map_w, full0 + 8 * s, x, y);
+          if (copies) tma_load_2d(smem_u32(ring + s * STAGE_BYTES + lane * BOX_BYTES), &map_w, full0 + 8 * s, x, matrix0 + y);
           in_flight = min(in_flight + 1, STAGES);
           if (++s == STAGES) s = 0, phase ^= 1;
         }
     }
+    if (GROUPED && follows) pdl_wait();  // (a block without tiles, or with few, comes here at once)
     pdl_launch_dependents();
     if (!ok && lane == 0) {
       // Giving up: the copies already issued must land before the block's shared memory is released.
@@ -236,11 +262,21 @@ gemv_stream_kernel(const bf16* __restrict__ a, const __grid_constant__ CUtensorM
     const int g = lane >> 2, t = lane & 3;
     const bf16* arow[NT];
     bool alive[NT];
+    int first_row = 0;  // GROUPED: the entry's first sorted row (m: its rows), of the tiles whose activations are fetched
+    auto rows_of = [&](int first) {
+      if (GROUPED) {
+        const int* entry = grouped.entries + 3 * ((tile0 + first) / grouped.per_entry);
+        first_row = __ldcg(entry + 1);
+        m = __ldcg(entry + 2);
+      }
 #pragma unroll
-    for (int j = 0; j < NT; ++j) {
-      alive[j] = 8 * j + g < m;
-      arow[j] = a + (size_t)(alive[j] ? 8 * j + g : 0) * k;
-    }
+      for (int j = 0; j < NT; ++j) {
+        alive[j] = 8 * j + g < m;
+        int row = alive[j] ? 8 * j + g : 0;
+        if (GROUPED) row = grouped.source ? __ldcg(grouped.source + first_row + row) : first_row + row;
+        arow[j] = a + (size_t)row * k;
+      }
+    };
     const uint4 zero = make_uint4(0, 0, 0, 0);
     const int in_stage = warp * WARP_COLS + 8 * t;  // this thread's first column within a stage
     if (PENDING) {
@@ -255,7 +291,7 @@ gemv_stream_kernel(const bf16* __restrict__ a, const __grid_constant__ CUtensorM
       }
       consumer_sync();
     }
-    pdl_wait();  // the activations come from the kernel before
+    if (!GROUPED || follows) pdl_wait();  // the activations come from the kernel before
     // From here on every earlier kernel is complete, so the next kernel's blocks may move in beside
     // this one (never more than two kernels overlap). Activations are read through L2 (__ldcg): a
     // block that started while an earlier kernel was still running must not find lines in L1 that
@@ -356,11 +392,16 @@ gemv_stream_kernel(const bf16* __restrict__ a, const __grid_constant__ CUtensorM
         }
     };
     uint4 av[KBLOCKS][NT], av_next[KBLOCKS][NT];
-    if (my_tiles > 0) fetch(0, av_next);
+    if (my_tiles > 0) {
+      rows_of(0);
+      fetch(0, av_next);
+    }
     bool ok = true;
     int s = 0, phase = 0;
-    for (int first = 0; first < my_tiles && ok; first += GROUP_TILES) {
-      const int count = min(GROUP_TILES, my_tiles - first);
+    for (int first = 0, count; first < my_tiles && ok; first += count) {
+      count = together(first);
+      const int in_matrix = GROUPED ? (tile0 + first) % grouped.per_entry : tile0 + first;
+      const int out_row = first_row, out_m = m;
       float acc[GROUP_TILES][NT][4];
 #pragma unroll
       for (int i = 0; i < GROUP_TILES; ++i)
@@ -372,12 +413,17 @@ gemv_stream_kernel(const bf16* __restrict__ a, const __grid_constant__ CUtensorM
 #pragma unroll
           for (int j = 0; j < NT; ++j) av[h][j] = av_next[h][j];
         // The next columns' activations (the first columns again when another group follows).
-        if (c + 1 < chunks || first + GROUP_TILES < my_tiles) fetch(c + 1 < chunks ? c + 1 : 0, av_next);
+        if (c + 1 < chunks) {
+          fetch(c + 1, av_next);
+        } else if (first + count < my_tiles) {
+          if (GROUPED && in_matrix + count == grouped.per_entry) rows_of(first + count);
+          fetch(0, av_next);
+        }
         const int col0 = c * STAGE_COLS + in_stage;
 #pragma unroll
         for (int i = 0; i < GROUP_TILES; ++i) {
           if (i >= count) break;
-          const int tile = tile0 + first + i;
+          const int tile = in_matrix + i;
           const bool lo_live = tile_row<EPI>(tile, g, n, inner) >= 0, hi_live = tile_row<EPI>(tile, g + 8, n, inner) >= 0;
           ok = mbar_wait(full0 + 8 * s, phase, abort_flag);
           if (!ok) break;
@@ -418,8 +464,8 @@ gemv_stream_kernel(const bf16* __restrict__ a, const __grid_constant__ CUtensorM
       const int out_rows = EPI == EPI_SWIGLU ? 8 : TILE_ROWS;
       for (int idx = threadIdx.x; idx < count * out_rows * NT * 8; idx += CONSUMERS) {
         const int token = idx / (count * out_rows), rest = idx % (count * out_rows);
-        const int i = rest / out_rows, r = rest % out_rows, tile = tile0 + first + i;
-        if (token >= m) continue;
+        const int i = rest / out_rows, r = rest % out_rows, tile = in_matrix + i;
+        if (token >= out_m) continue;
         float v = 0.f;
 #pragma unroll
         for (int s2 = 0; s2 < CONSUMER_WARPS; ++s2) v += partial[s2][i * TILE_ROWS + r][token];
@@ -429,11 +475,12 @@ gemv_stream_kernel(const bf16* __restrict__ a, const __grid_constant__ CUtensorM
           for (int s2 = 0; s2 < CONSUMER_WARPS; ++s2) up += partial[s2][i * TILE_ROWS + 8 + r][token];
           const int col = tile * 8 + r;
           if (col >= inner) continue;
-          // The two halves are rounded to bfloat16 first, as a separate product would round them.
-          const float gate = __bfloat162float(__float2bfloat16_rn(v));
-          up = __bfloat162float(__float2bfloat16_rn(up));
+          // The two halves are rounded to bfloat16 first, as a separate product would round them (the experts' other
+          // kernels round the unit's result only, and so does the grouped form).
+          const float gate = GROUPED ? v : __bfloat162float(__float2bfloat16_rn(v));
+          if (!GROUPED) up = __bfloat162float(__float2bfloat16_rn(up));
           // `cap` says which unit (gated_unit in common.cuh), `multiplier` is the clamped one's slope.
-          reinterpret_cast<bf16*>(out)[(size_t)token * inner + col] = __float2bfloat16_rn(gated_unit(gate, up, multiplier, cap));
+          reinterpret_cast<bf16*>(out)[(size_t)(out_row + token) * inner + col] = __float2bfloat16_rn(gated_unit(gate, up, multiplier, cap));
         } else {
           const int col = tile * TILE_ROWS + r;
           if (col >= n) continue;
@@ -459,7 +506,7 @@ gemv_stream_kernel(const bf16* __restrict__ a, const __grid_constant__ CUtensorM
                 v = gelu_erf(z);
               }
             }
-            reinterpret_cast<bf16*>(out)[(size_t)token * n + col] = __float2bfloat16_rn(v);
+            reinterpret_cast<bf16*>(out)[(size_t)(out_row + token) * n + col] = __float2bfloat16_rn(v);
           }
         }
       }
@@ -507,9 +554,10 @@ constexpr size_t fixed_most() {
          (PENDING ? sizeof(bf16) * NT * 8 * (size_t)(PENDING_MAX_K + PENDING_PAD) + sizeof(float) * 2 * PENDING_MAX_K : 0);
 }
 
-template <int NT, int EPI, bool PENDING>
+template <int NT, int EPI, bool PENDING, bool GROUPED = false>
 int launch(const bf16* a, const bf16* w, void* out, int m, int n, int k, int inner, float multiplier, float cap,
-           float second, const PendingStep& pending, int* err, cudaStream_t stream) {
+           float second, const PendingStep& pending, int* err, cudaStream_t stream, const Grouped& grouped = Grouped{},
+           int matrices = 1, int follows = 0) {
   const size_t fixed = (size_t)STAGES * STAGE_BYTES + ((partial_bytes(NT) + 15) & ~(size_t)15);
   const size_t smem = fixed + (PENDING ? sizeof(bf16) * NT * 8 * (size_t)(k + PENDING_PAD) + sizeof(float) * 2 * k : 0);
   constexpr size_t most = fixed_most<NT, PENDING>();
@@ -519,17 +567,19 @@ int launch(const bf16* a, const bf16* w, void* out, int m, int n, int k, int inn
     cudaError_t e = cudaGetDevice(&device);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(gemv_stream_kernel<NT, EPI, PENDING>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+      e = cudaFuncSetAttribute(gemv_stream_kernel<NT, EPI, PENDING, GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
     if (e != cudaSuccess) {
       sms = 0;
       return (int)e;
     }
   }
   CUtensorMap map_w;
-  if (!make_map(&map_w, w, n, k)) return (int)cudaErrorInvalidValue;
+  if (!make_map(&map_w, w, matrices * n, k)) return (int)cudaErrorInvalidValue;
   const int tiles = EPI == EPI_SWIGLU ? (inner + 7) / 8 : (n + TILE_ROWS - 1) / TILE_ROWS;
-  launch_pdl(gemv_stream_kernel<NT, EPI, PENDING>, min(tiles, sms), THREADS, smem, stream, a, map_w, out, m, n, k, inner,
-             tiles, multiplier, cap, second, pending, err);
+  Grouped list = grouped;
+  list.per_entry = tiles;
+  launch_pdl(gemv_stream_kernel<NT, EPI, PENDING, GROUPED>, GROUPED ? sms : min(tiles, sms), THREADS, smem, stream, a, map_w, out, m,
+             n, k, inner, tiles, multiplier, cap, second, pending, list, follows, err);
   return OMNIA_LAUNCH_RESULT();
 }
 
@@ -587,4 +637,34 @@ extern "C" int omnia_gemv_stream_pending(const float* x, float* x_out, const voi
     return launch_rows<EPI_SOFTCAP, true>(nullptr, wp, out, m, n, k, 0, 1.f, cap, 0.f, pending, err, stream);
   if (epilogue != EPI_STORE) return (int)cudaErrorInvalidValue;
   return launch_rows<EPI_STORE, true>(nullptr, wp, out, m, n, k, 0, 1.f, 0.f, 0.f, pending, err, stream);
+}
+
+// The products of a step's chosen experts (moe.cu), whose rows are few: the sorted rows of every entry of the list
+// `entries` [*count, 3] = (expert, first sorted row, at most `entry_rows` rows: 8 or 16) times that expert's matrix of
+// w [experts, n, k]. dual: n = 2 inner, gate rows then up rows, out [rows, inner] the unit that `limit` and `alpha` name;
+// otherwise out [rows, n], with limit 5 behind the exact GELU. follows != 0: the list was made before the kernel in front
+// of this one began, so the weights need not wait for that kernel.
+//
+// Bound by the weights of the experts in use, each read once. mma.sync tiles of 64 x 64 fed by 64-byte pieces of rows
+// (moe.cu's other product) reach 3.3 TB/s on them; this stream of 4 KB boxes is the dense products' own. 8 rows, 4 of 32
+// experts of 2,048 x 1,536 each: 78 and 61 us for the two products (each with its wait for the kernel before), 46 and 30 so.
+extern "C" int omnia_gemv_stream_grouped(const void* a, const int* source, const void* w, void* out, const int* entries,
+                                         const int* count, int entry_rows, int n, int k, int experts, int dual, float alpha,
+                                         float limit, int follows, int* err, cudaStream_t stream) {
+  if (n == 0 || experts == 0) return 0;
+  if ((entry_rows != 8 && entry_rows != 16) || k % 8 != 0 || k <= 0 || (dual && n % 2) || (long long)n * experts > 0x7fffffffLL)
+    return (int)cudaErrorInvalidValue;
+  if (((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15) != 0) return (int)cudaErrorInvalidValue;
+  const bf16* ap = (const bf16*)a;
+  const bf16* wp = (const bf16*)w;
+  const Grouped list{entries, count, source, 0};
+  const PendingStep none{};
+  if (dual)
+    return entry_rows == 8
+               ? launch<1, EPI_SWIGLU, false, true>(ap, wp, out, 8, n, k, n / 2, alpha, limit, 0.f, none, err, stream, list, experts, follows)
+               : launch<2, EPI_SWIGLU, false, true>(ap, wp, out, 16, n, k, n / 2, alpha, limit, 0.f, none, err, stream, list, experts, follows);
+  if (limit != 0.f && limit != 5.f) return (int)cudaErrorInvalidValue;
+  return entry_rows == 8
+             ? launch<1, EPI_STORE, false, true>(ap, wp, out, 8, n, k, 0, 1.f, limit, 0.f, none, err, stream, list, experts, follows)
+             : launch<2, EPI_STORE, false, true>(ap, wp, out, 16, n, k, 0, 1.f, limit, 0.f, none, err, stream, list, experts, follows);
 }

@@ -1917,6 +1917,11 @@ MOE_TCGEN05_PAIRS = 1024
 grouped products run on the tcgen05 kernel (tiles of 128 rows of one expert each; fewer rows an expert
 would leave most of every tile empty); below, on the mma.sync kernel with tiles of 64 rows."""
 
+MOE_STREAM_PAIRS = 8
+"""Up to this many pairs an expert on average (or 16 rows, which give no expert more than 16 pairs) the bfloat16 grouped
+products stream the weights as a decode step's dense products do, in entries of 8 or 16 rows: an expert with more rows
+than that has its matrix read again for the next entry, which above this average happens often."""
+
 
 def moe_experts(h: torch.Tensor, router: torch.Tensor | None, correction: torch.Tensor | None, gate_up: torch.Tensor,
                 down: torch.Tensor, top: int, step: StepContext | None = None,
@@ -1966,7 +1971,8 @@ def moe_experts(h: torch.Tensor, router: torch.Tensor | None, correction: torch.
         tensor_cores = h.dtype == torch.bfloat16 and hidden % 8 == 0 and inner % 8 == 0
     if tcgen05 is None:
         tcgen05 = tensor_cores and pairs >= MOE_TCGEN05_PAIRS and pairs >= 64 * experts
-    tile_rows = 128 if tcgen05 else MOE_TILE_ROWS
+    streamed = tensor_cores and not tcgen05 and (rows <= 16 or pairs <= MOE_STREAM_PAIRS * experts)
+    tile_rows = 128 if tcgen05 else (8 if rows <= 8 else 16) if streamed else MOE_TILE_ROWS
     max_tiles = min(pairs, -(-pairs // tile_rows) + experts)
     def chosen() -> tuple:
         """The choices, and every chosen expert's output."""
@@ -2013,6 +2019,16 @@ def moe_experts(h: torch.Tensor, router: torch.Tensor | None, correction: torch.
                            _ptr(tile_count), max_tiles, alpha, limit, err, _stream()), "gemm_tcgen05_grouped")
             _check(grouped(_ptr(act), _ptr(down), _ptr(out), pairs, hidden, inner, experts, 0, _ptr(tiles),
                            _ptr(tile_count), max_tiles, 1.0, 0.0, err, _stream()), "gemm_tcgen05_grouped")
+        elif streamed:
+            stream = _function("gemv_stream", "omnia_gemv_stream_grouped",
+                               [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
+                                c_float, c_float, c_int, c_void_p, c_void_p])
+            err = _ptr(error_word(device))
+            _check(stream(_ptr(h if sorted_rows is None else sorted_rows), _ptr(source) if sorted_rows is None else None,
+                          _ptr(gate_up), _ptr(act), _ptr(tiles), _ptr(tile_count), tile_rows, gate_up.shape[1], hidden, experts,
+                          int(dual), alpha, limit, 0, err, _stream()), "gemv_stream_grouped")
+            _check(stream(_ptr(act), None, _ptr(down), _ptr(out), _ptr(tiles), _ptr(tile_count), tile_rows, hidden, inner,
+                          experts, 0, 1.0, 0.0, 1, err, _stream()), "gemv_stream_grouped")
         else:
             product = _function("moe", "omnia_moe_product",
                                 [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int,

@@ -327,6 +327,38 @@ def test_table_routed_clamped_experts(dtype, tensor_cores, rows, hidden, inner, 
     ops.raise_on_error(CUDA)
 
 
+@pytest.mark.parametrize("rows,hidden,inner,experts,top", [(1, 1048, 88, 9, 4), (8, 136, 1032, 9, 2), (9, 2056, 8, 5, 3),
+                                                           (16, 264, 24, 2, 1), (17, 128, 72, 40, 4), (61, 1024, 200, 33, 4)])
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("skewed", [False, True])
+def test_streamed_experts(rows, hidden, inner, experts, top, gated, skewed):
+    """Few rows an expert: entries of 8 and of 16 rows, matrices that are no multiple of a tile or of a stage, more
+    blocks than tiles, and (`skewed`: every token the same experts) experts whose rows take several entries. A row is
+    rounded to bfloat16 between the two products and behind them: a part in 2^9 each time."""
+    g = torch.Generator().manual_seed(rows * 7 + experts)
+    bf, vocab = torch.bfloat16, 29
+    h = torch.randn(rows, hidden, generator=g).to(bf)
+    table = torch.stack([torch.randperm(experts, generator=g)[:top] for _ in range(vocab)]).to(torch.int32)
+    ids = torch.full((rows,), 3) if skewed else torch.randint(0, vocab, (rows,), generator=g)
+    up = (torch.randn(experts, (1 + gated) * inner, hidden, generator=g) * hidden ** -0.5).to(bf)
+    down = (torch.randn(experts, hidden, inner, generator=g) * inner ** -0.5).to(bf)
+    got = ops.moe_experts(h.to(CUDA), None, None, up.to(CUDA), down.to(CUDA), top, None, table=table.to(CUDA),
+                          token_ids=ids.to(torch.int32).to(CUDA), alpha=1.702 if gated else 1.0, limit=0.8 if gated else 0.0,
+                          activation=None if gated else "gelu_erf")
+    want = torch.zeros(rows, hidden, dtype=F64)
+    for t in range(rows):
+        for e in table[ids[t]].tolist():
+            z = up[e].to(F64) @ h[t].to(F64)
+            if gated:
+                gate, part = z[:inner].clamp(max=0.8), z[inner:].clamp(-0.8, 0.8)
+                z = gate * torch.sigmoid(1.702 * gate) * (part + 1.0)
+            else:
+                z = torch.nn.functional.gelu(z)
+            want[t] += down[e].to(F64) @ z / top
+    assert rel(got, want) < 1e-2
+    ops.raise_on_error(CUDA)
+
+
 # ---- the engine -----------------------------------------------------------------------------
 
 
