@@ -275,7 +275,7 @@ union SampleWork {  // used one after the other
 //    it, so it is out. The histograms count what is left, and after the first digit only a list of it.
 // Where a bound leaves too much (k above 2,048, ties by the thousand, an infinite maximum) the radix selection
 // over all logits stands. 64 rows of 151,936 logits, top_k 50, top_p 0.95: 146 us with the selection over all logits,
-44 so (a cluster of eight blocks a row is 512 blocks, two to an SM: 1.7 rounds of them).
+// 44 so (a cluster of eight blocks a row is 512 blocks, two to an SM: 1.7 rounds of them).
 __global__ void __cluster_dims__(SAMPLE_CLUSTER, 1, 1) __launch_bounds__(SAMPLE_THREADS, 2)
 sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice, int cached,
               const float* __restrict__ temperature, const int* __restrict__ top_k,
