@@ -11,8 +11,10 @@
 //   warp 1   allocates tensor memory (both blocks); in the leader its elected lane waits for a
 //            drained accumulator, issues four MMAs per full stage, and tcgen05.commit (multicast to
 //            both blocks) frees the stage in both and, after the last step, signals "accumulator full"
-//   warps 2-5  (both blocks) read their block's 128 accumulator rows, apply the epilogue, store, and
-//            arrive on the leader's "accumulator empty" barrier
+//   warps 2-9  (both blocks) read their block's 128 accumulator rows, two warps to 32 rows, each half of the
+//            columns, apply the epilogue, store, and arrive on the leader's "accumulator empty" barrier. (The last
+//            tiles' epilogues overlap no product: one wave of tiles, 2,048 deep, takes 23.3 us with four such warps
+//            and 20.7 with eight.)
 // Blocks are persistent (one per SM); clusters take tiles round-robin; two accumulators in tensor
 // memory let the epilogue of one tile run while the next is multiplied. Epilogues: 0 store
 // bfloat16; 1 SwiGLU: the leader stages 128 gate rows of w, its peer the matching 128 up rows, the
@@ -38,7 +40,8 @@ typedef __nv_bfloat16 bf16;
 constexpr int BLOCK_M = 128;
 constexpr int BLOCK_K = 64;   // 128 bytes of bfloat16: one swizzle row
 constexpr int UMMA_K = 16;
-constexpr int THREADS = 192;  // producer warp, MMA warp, four epilogue warps
+constexpr int EPI_WARPS = 8;
+constexpr int THREADS = 64 + 32 * EPI_WARPS;  // producer warp, MMA warp, epilogue warps
 constexpr uint32_t WAIT_LIMIT = 1u << 20;
 
 enum { EPI_STORE = 0, EPI_SWIGLU = 1, EPI_SOFTCAP = 2, EPI_QKV = 3 };
@@ -117,10 +120,12 @@ __device__ __forceinline__ void tmem_load32(uint32_t addr, uint32_t* v) {
 
 
 constexpr int STAGES = 6;
-// The accumulator's columns, TILE_N, are 256 or 192 (a template parameter): the narrower tile is for
-// shapes whose 256-wide tiles leave the last wave of clusters mostly idle (12,288 columns of
-// gate|up at 2,048 rows: 384 tiles on 74 clusters are six waves, the last with 14 tiles; 512 tiles of
-// 192 are seven waves of three quarters the length). Each block stages TILE_N / 2 rows of w.
+// The accumulator has 256 columns whatever the shape: an instruction of 256 rows takes some 80 ns with 256, 192, 128 or
+// 64 columns alike (a wave of tiles 2,048 deep 10.4 / 12.2 / 10.0 / 9.6 us), so narrower tiles only add waves
+// (2,048 x 12,288 x 2,048: 86 us with tiles of 192, whose last wave is fuller, 78 with 256; x 24,576 x 4,096: 313 and 280).
+// Clusters of two pairs that share a's rows by multicast, a quarter less out of L2, measured the same a wave (and the
+// device holds 33 of them, 66 pairs of 74). Each block stages TILE_N / 2 rows of w.
+constexpr uint32_t TILE_N = 256;
 constexpr uint32_t A_BYTES = BLOCK_M * BLOCK_K * sizeof(bf16);
 constexpr uint32_t ACC_STRIDE = 256;                                // tensor-memory columns between the two accumulators
 constexpr uint32_t TMEM_COLS = 512;                                 // a power of two, as allocations must be
@@ -185,16 +190,17 @@ __device__ __forceinline__ int tile_column(int index, const QkvParts& parts) {
   return column;
 }
 
-template <int EPI, uint32_t TILE_N>
+template <int EPI>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                          void* __restrict__ out, int m, int n, int k, int pair_offset, float multiplier,
-                         float cap, int m_tiles, int n_tiles, const QkvParts parts, int* err) {
+                         float cap, int m_tiles, int n_tiles, const QkvParts parts, const int* __restrict__ group_tiles,
+                         const int* __restrict__ group_count, int group_rows, int* err) {
   constexpr int TILE_COLS = EPI == EPI_SWIGLU ? TILE_N / 2 : TILE_N;
   constexpr uint32_t HALF_N = TILE_N / 2;                           // rows of w a block stages
   constexpr uint32_t B_BYTES = HALF_N * BLOCK_K * sizeof(bf16);
   constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-  static_assert(TILE_N % 32 == 0 && TILE_N <= ACC_STRIDE && STAGE_BYTES % 1024 == 0, "tile width");
+  static_assert(TILE_N <= ACC_STRIDE && STAGE_BYTES % 1024 == 0, "tile width");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* tiles = reinterpret_cast<unsigned char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = reinterpret_cast<uint64_t*>(tiles + STAGES * STAGE_BYTES);
@@ -208,7 +214,6 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   const bool leader = rank == 0;
   const int cluster_id = blockIdx.x >> 1, clusters = gridDim.x >> 1;
   const int k_blocks = (k + BLOCK_K - 1) / BLOCK_K;
-  const int total_tiles = m_tiles * n_tiles;
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
   const uint32_t acc_full0 = smem_u32(bars + 2 * STAGES), acc_empty0 = smem_u32(bars + 2 * STAGES + 2);
 
@@ -219,7 +224,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(acc_full0 + 8 * b, 1);   // the leader's commit, multicast
-      mbar_init(acc_empty0 + 8 * b, 8);  // one arrival per epilogue warp of either block
+      mbar_init(acc_empty0 + 8 * b, 2 * EPI_WARPS);  // one arrival per epilogue warp of either block
     }
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -237,6 +242,17 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   // (the launch is a programmatic dependent launch); from here on its results are read.
   pdl_wait();
   pdl_launch_dependents();
+  // Grouped: the list's length is what a kernel before this one wrote; m_tiles is then its capacity.
+  if (group_tiles != nullptr) m_tiles = min(*group_count, m_tiles);
+  const int total_tiles = m_tiles * n_tiles;
+  // Row tile `mt`: its first row, how many of its 256 rows are its own, and where its weight rows begin.
+  auto row_tile = [&](int mt, int& m0, int& rows, int& w0) {
+    if (group_tiles != nullptr) {
+      w0 = group_tiles[3 * mt] * group_rows, m0 = group_tiles[3 * mt + 1], rows = group_tiles[3 * mt + 2];
+    } else {
+      w0 = 0, m0 = mt * 2 * BLOCK_M, rows = 2 * BLOCK_M;
+    }
+  };
 
   if (warp == 0) {
     // ---- producer (both blocks) -------------------------------------------------------------
@@ -244,8 +260,11 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       uint32_t it = 0;
       bool ok = true;
       for (int tile = cluster_id; tile < total_tiles && ok; tile += clusters) {
-        const int m0 = (tile % m_tiles) * 2 * BLOCK_M + rank * BLOCK_M, n0 = tile_column<EPI>(tile / m_tiles, parts) * TILE_COLS;
-        const int w_row = EPI == EPI_SWIGLU ? (leader ? n0 : pair_offset + n0) : n0 + (int)rank * (int)HALF_N;
+        int m0, tile_rows, w0;
+        row_tile(tile % m_tiles, m0, tile_rows, w0);
+        m0 += rank * BLOCK_M;
+        const int n0 = tile_column<EPI>(tile / m_tiles, parts) * TILE_COLS;
+        const int w_row = w0 + (EPI == EPI_SWIGLU ? (leader ? n0 : pair_offset + n0) : n0 + (int)rank * (int)HALF_N);
         for (int kb = 0; kb < k_blocks; ++kb, ++it) {
           const int s = it % STAGES;
           ok = mbar_wait(empty0 + 8 * s, ((it / STAGES) & 1) ^ 1, abort_flag);
@@ -288,13 +307,16 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       }
     }
   } else {
-    // ---- epilogue (both blocks; warps 2..5 own accumulator rows 32 * (warp % 4) .. + 31) ----------
-    const int quarter = warp & 3;
+    // ---- epilogue (both blocks; a warp takes accumulator rows 32 * (warp % 4) .. + 31) ----------
+    const int quarter = warp & 3, half_of = (warp - 2) >> 2;  // whose rows, and which half of the columns
     uint32_t local = 0;
     bool ok = true;
     for (int tile = cluster_id; tile < total_tiles && ok; tile += clusters, ++local) {
-      const int m0 = (tile % m_tiles) * 2 * BLOCK_M + rank * BLOCK_M, n0 = tile_column<EPI>(tile / m_tiles, parts) * TILE_COLS;
-      const int row = m0 + quarter * 32 + lane;
+      int m0, tile_rows, w0;
+      row_tile(tile % m_tiles, m0, tile_rows, w0);
+      const int n0 = tile_column<EPI>(tile / m_tiles, parts) * TILE_COLS;
+      const int in_tile = rank * BLOCK_M + quarter * 32 + lane;
+      const int row = in_tile < tile_rows ? m0 + in_tile : m;  // m: not one of the tile's own
       const uint32_t buf = local % ACC_BUFS, round = local / ACC_BUFS;
       ok = mbar_wait(acc_full0 + 8 * buf, round & 1, abort_flag);
       if (!ok) break;
@@ -303,35 +325,41 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
       if (EPI == EPI_SWIGLU) {
         bf16* dst = reinterpret_cast<bf16*>(out) + (size_t)row * pair_offset + n0;
 #pragma unroll 1
-        for (int c = 0; c < (int)TILE_N / 2; c += 32) {
+        for (int c = half_of * (int)TILE_N / 4; c < (half_of + 1) * (int)TILE_N / 4; c += 32) {
           uint32_t gate[32], up[32];
           tmem_load32(lane_base + c, gate);
           tmem_load32(lane_base + TILE_N / 2 + c, up);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-          if (row < m) {
+          if (row >= m) continue;
+          __nv_bfloat162 unit[16];
 #pragma unroll
-            for (int j = 0; j < 32; j += 2) {
-              float v[2];
+          for (int j = 0; j < 32; j += 2) {
+            float v[2];
 #pragma unroll
-              for (int e = 0; e < 2; ++e) {
-                // Both halves are rounded to bfloat16 first, as a separate product would round them.
-                const float g = __bfloat162float(__float2bfloat16_rn(__uint_as_float(gate[j + e])));
-                const float u = __bfloat162float(__float2bfloat16_rn(__uint_as_float(up[j + e])));
-                // cap > 0: the clamped unit (gate below cap, up within +-cap and moved by one, slope `multiplier`).
-                const float gc = cap > 0.f ? fminf(g, cap) : g;
-                const float uc = cap > 0.f ? fminf(fmaxf(u, -cap), cap) + 1.f : u;
-                // cap -1: the gate through a relu; cap -2: through the tanh form of GELU, g sigmoid(2 a).
-                const float z = cap < OMNIA_UNIT_RELU ? 1.5957691216057308f * (g + 0.044715f * g * g * g) : multiplier * gc;
-                v[e] = cap == OMNIA_UNIT_RELU ? fmaxf(g, 0.f) * u : __fdividef(gc, 1.f + __expf(-z)) * uc;
-              }
-              const int col = n0 + c + j;
-              if (col + 1 < pair_offset && (pair_offset & 1) == 0) {
-                *reinterpret_cast<__nv_bfloat162*>(dst + c + j) = __floats2bfloat162_rn(v[0], v[1]);
-              } else {
-                if (col < pair_offset) dst[c + j] = __float2bfloat16_rn(v[0]);
-                if (col + 1 < pair_offset) dst[c + j + 1] = __float2bfloat16_rn(v[1]);
-              }
+            for (int e = 0; e < 2; ++e) {
+              // Both halves are rounded to bfloat16 first, as a separate product would round them.
+              const float g = __bfloat162float(__float2bfloat16_rn(__uint_as_float(gate[j + e])));
+              const float u = __bfloat162float(__float2bfloat16_rn(__uint_as_float(up[j + e])));
+              // cap > 0: the clamped unit (gate below cap, up within +-cap and moved by one, slope `multiplier`).
+              const float gc = cap > 0.f ? fminf(g, cap) : g;
+              const float uc = cap > 0.f ? fminf(fmaxf(u, -cap), cap) + 1.f : u;
+              // cap -1: the gate through a relu; cap -2: through the tanh form of GELU, g sigmoid(2 a).
+              const float z = cap < OMNIA_UNIT_RELU ? 1.5957691216057308f * (g + 0.044715f * g * g * g) : multiplier * gc;
+              v[e] = cap == OMNIA_UNIT_RELU ? fmaxf(g, 0.f) * u : __fdividef(gc, 1.f + __expf(-z)) * uc;
             }
+            unit[j / 2] = __floats2bfloat162_rn(v[0], v[1]);
+          }
+          // 16 bytes a store: every lane has a row of its own, so a store is 32 requests whatever it carries.
+          if (n0 + c + 32 <= pair_offset && (pair_offset & 7) == 0) {
+#pragma unroll
+            for (int j = 0; j < 16; j += 4)
+              *reinterpret_cast<uint4*>(dst + c + 2 * j) =
+                  make_uint4(*reinterpret_cast<uint32_t*>(&unit[j]), *reinterpret_cast<uint32_t*>(&unit[j + 1]),
+                             *reinterpret_cast<uint32_t*>(&unit[j + 2]), *reinterpret_cast<uint32_t*>(&unit[j + 3]));
+          } else {
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (n0 + c + j < pair_offset) dst[c + j] = (j & 1) ? unit[j / 2].y : unit[j / 2].x;
           }
         }
       } else if (EPI == EPI_QKV) {
@@ -350,7 +378,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
           }
         };
 #pragma unroll 1
-        for (int seg = 0; seg < (int)TILE_N && n0 + seg < n; seg += d) {
+        for (int seg = half_of * (int)TILE_N / 2; seg < (half_of + 1) * (int)TILE_N / 2 && n0 + seg < n; seg += d) {
           const int col0 = n0 + seg;
           // Whose head this is: 0 q, 1 k, 2 v, 3 neither. (The same for every thread of the block.)
           int kind = 3, head = 0;
@@ -422,7 +450,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
         }
       } else {
 #pragma unroll 1
-        for (int c = 0; c < (int)TILE_N; c += 32) {
+        for (int c = half_of * (int)TILE_N / 2; c < (half_of + 1) * (int)TILE_N / 2; c += 32) {
           uint32_t acc[32];
           tmem_load32(lane_base + c, acc);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -437,6 +465,12 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             }
           } else {
             bf16* dst = reinterpret_cast<bf16*>(out) + (size_t)row * n + n0 + c;
+            // cap 5: the exact GELU of the product, as bfloat16 would hold it (a separate kernel would read it so).
+            if (cap == 5.f) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j)
+                acc[j] = __float_as_uint(gelu_erf(__bfloat162float(__float2bfloat16_rn(__uint_as_float(acc[j])))));
+            }
             if (n0 + c + 32 <= n && (n & 7) == 0) {
 #pragma unroll
               for (int j = 0; j < 32; j += 8) {
@@ -512,51 +546,36 @@ bool make_map(CUtensorMap* map, const void* base, int rows, int k, int box_rows)
 
 int sm_count() { return omnia_sm_count(); }
 
-// Tiles of the output for accumulators of `tile_n` columns.
-template <int EPI>
-long long tile_count(int m, int n, int pair_offset, int tile_n, int* m_tiles, int* n_tiles) {
-  const int cols = EPI == EPI_SWIGLU ? pair_offset : n;
-  const int tile_cols = EPI == EPI_SWIGLU ? tile_n / 2 : tile_n;
-  *n_tiles = (cols + tile_cols - 1) / tile_cols;
-  *m_tiles = (m + 2 * BLOCK_M - 1) / (2 * BLOCK_M);
-  return (long long)*n_tiles * *m_tiles;
-}
+// The grouped product's list of row tiles, on the device; `rows`: of the weights of one group.
+struct Groups {
+  const int* tiles;
+  const int* count;
+  int most, rows, experts;
+};
 
-template <int EPI, uint32_t TILE_N>
-int launch_width(const void* a, const void* w, void* out, int m, int n, int k, int pair_offset, float multiplier,
-                 float cap, const QkvParts& parts, int* err, cudaStream_t stream) {
+template <int EPI>
+int launch(const void* a, const void* w, void* out, int m, int n, int k, int pair_offset, float multiplier,
+           float cap, int* err, cudaStream_t stream, const QkvParts& parts = QkvParts{}, const Groups& groups = Groups{}) {
   constexpr uint32_t STAGE_BYTES = A_BYTES + (TILE_N / 2) * BLOCK_K * sizeof(bf16);
+  const bool grouped = groups.tiles != nullptr;
   CUtensorMap map_a, map_b;
-  if (!make_map(&map_a, a, m, k, BLOCK_M) || !make_map(&map_b, w, n, k, (int)(TILE_N / 2)))
+  if (!make_map(&map_a, a, m, k, BLOCK_M) || !make_map(&map_b, w, grouped ? groups.experts * n : n, k, (int)(TILE_N / 2)))
     return (int)cudaErrorInvalidValue;
   constexpr size_t smem = (size_t)STAGES * STAGE_BYTES + 1024 + 256;
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<EPI, TILE_N>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(gemm_tcgen05_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  int m_tiles, n_tiles;
-  const long long total = tile_count<EPI>(m, n, pair_offset, (int)TILE_N, &m_tiles, &n_tiles);
+  const int cols = EPI == EPI_SWIGLU ? pair_offset : n, tile_cols = (int)(EPI == EPI_SWIGLU ? TILE_N / 2 : TILE_N);
+  const int n_tiles = (cols + tile_cols - 1) / tile_cols, m_tiles = grouped ? groups.most : (m + 2 * BLOCK_M - 1) / (2 * BLOCK_M);
+  const long long total = (long long)n_tiles * m_tiles;
   const int pairs = sm_count() / 2;
   const int clusters = (int)(total < pairs ? total : pairs);  // one persistent block per SM
-  launch_pdl(gemm_tcgen05_pair_kernel<EPI, TILE_N>, 2 * clusters, THREADS, smem, stream,
-             map_a, map_b, out, m, n, k, pair_offset, multiplier, cap, m_tiles, n_tiles, parts, err);
+  launch_pdl(gemm_tcgen05_pair_kernel<EPI>, 2 * clusters, THREADS, smem, stream, map_a, map_b, out, m, n, k, pair_offset,
+             multiplier, cap, m_tiles, n_tiles, parts, groups.tiles, groups.count, groups.rows, err);
   return OMNIA_LAUNCH_RESULT();
-}
-
-// The width whose waves of tiles take the least time: waves x width, 256 on a tie.
-template <int EPI>
-int launch(const void* a, const void* w, void* out, int m, int n, int k, int pair_offset, float multiplier,
-           float cap, int* err, cudaStream_t stream) {
-  const QkvParts parts = {};
-  const int pairs = sm_count() / 2;
-  int mt, nt;
-  const long long wide = (tile_count<EPI>(m, n, pair_offset, 256, &mt, &nt) + pairs - 1) / pairs * 256;
-  const long long narrow = (tile_count<EPI>(m, n, pair_offset, 192, &mt, &nt) + pairs - 1) / pairs * 192;
-  if (narrow < wide) return launch_width<EPI, 192>(a, w, out, m, n, k, pair_offset, multiplier, cap, parts, err, stream);
-  return launch_width<EPI, 256>(a, w, out, m, n, k, pair_offset, multiplier, cap, parts, err, stream);
 }
 
 }  // namespace
@@ -595,5 +614,23 @@ extern "C" int omnia_gemm_tcgen05_pair_qkv(const void* a, const void* w, void* o
     return (int)cudaErrorInvalidValue;
   const QkvParts parts = {head_dim, q_col, k_col, v_col, nq, nkv, eps, (const float2*)angles, slots, (bf16*)q_out,
                           (bf16*)pages, page_size, num_slots};
-  return launch_width<EPI_QKV, 256>(a, w, out, m, n, k, 0, 1.f, 0.f, parts, err, stream);
+  return launch<EPI_QKV>(a, w, out, m, n, k, 0, 1.f, 0.f, err, stream, parts);
+}
+
+// The grouped product of routed experts: a [m, k] rows sorted by expert; w [experts, n, k]; tiles
+// [max_tiles, 3] = (expert, first row, rows <= 256) and tile_count [1] in device memory. epilogue 0:
+// out [m, n] = a w_e^T (cap 5: its exact GELU); 1: n = 2 * inner (gate rows, then up rows), out [m, inner] = silu(gate) * up, or with
+// cap > 0 the clamped unit (the sigmoid's slope in `multiplier`), with cap -1 relu(gate) * up, -2 tanh-GELU(gate) * up.
+extern "C" int omnia_gemm_tcgen05_pair_grouped(const void* a, const void* w, void* out, int m, int n, int k, int experts,
+                                               int epilogue, const int* tiles, const int* tile_count, int max_tiles,
+                                               float multiplier, float cap, int* err, cudaStream_t stream) {
+  if (m == 0 || n == 0 || max_tiles == 0) return 0;
+  if (k <= 0 || k % 8 != 0 || ((uintptr_t)a & 15) || ((uintptr_t)w & 15) || experts < 1) return (int)cudaErrorInvalidValue;
+  const Groups groups = {tiles, tile_count, max_tiles, n, experts};
+  if (epilogue == EPI_SWIGLU) {
+    if (n % 2) return (int)cudaErrorInvalidValue;
+    return launch<EPI_SWIGLU>(a, w, out, m, n, k, n / 2, cap > 0.f ? multiplier : 1.f, cap, err, stream, QkvParts{}, groups);
+  }
+  if (epilogue != EPI_STORE || (cap != 0.f && cap != 5.f)) return (int)cudaErrorInvalidValue;
+  return launch<EPI_STORE>(a, w, out, m, n, k, 0, 1.f, cap, err, stream, QkvParts{}, groups);
 }

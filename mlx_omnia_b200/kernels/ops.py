@@ -852,12 +852,12 @@ def _pair_pays(rows: int, n: int, k: int, epilogue: int, sms: int) -> bool:
     if epilogue == 1:
         # gate|up with SwiGLU: tiles of 128 output columns, 128 rows to an SM or 256 to a pair. What
         # decides is how many waves of tiles each kernel runs (measured, 12,288 weight rows of 2,048:
-        # some 10 us and 14 a wave for one SM, 8 and 13 a wave for a pair; 264 / 512 / 768 / 896 rows:
-        # 24 / 38 / 38 / 51 us against 30 / 31 / 35 / 46).
+        # some 10 us and 14 a wave for one SM, 9 and 11 a wave for a pair; 512 / 1,082 rows: 38 / 53.5 us
+        # against 29.6 / 52).
         tiles = -(-(n // 2) // 128)
         one = -(-(-(-rows // 128) * tiles) // sms)
         two = -(-(-(-rows // 256) * tiles) // (sms // 2))
-        return 8 + 13 * two < 10 + 14 * one
+        return 9 + 11 * two < 10 + 14 * one
     tiles = -(-rows // 256) * -(-n // 256)
     return tiles * -(-k // 64) >= 64 * (sms // 2)
 
@@ -1917,6 +1917,11 @@ MOE_TCGEN05_PAIRS = 1024
 grouped products run on the tcgen05 kernel (tiles of 128 rows of one expert each; fewer rows an expert
 would leave most of every tile empty); below, on the mma.sync kernel with tiles of 64 rows."""
 
+MOE_PAIR_ROWS = 112
+"""From this many pairs an expert on average the grouped products take tiles of 256 rows, two SMs to a tile: such a tile
+brings in a third less than two of 128 rows, which are bound by what they pull out of L2 (19 us a wave of tiles 2,048
+deep against 10.5), and an expert of 113 to 256 rows fills one. With fewer rows most experts need one tile of either."""
+
 MOE_STREAM_PAIRS = 8
 """Up to this many pairs an expert on average (or 16 rows, which give no expert more than 16 pairs) the bfloat16 grouped
 products stream the weights as a decode step's dense products do, in entries of 8 or 16 rows: an expert with more rows
@@ -1972,7 +1977,8 @@ def moe_experts(h: torch.Tensor, router: torch.Tensor | None, correction: torch.
     if tcgen05 is None:
         tcgen05 = tensor_cores and pairs >= MOE_TCGEN05_PAIRS and pairs >= 64 * experts
     streamed = tensor_cores and not tcgen05 and (rows <= 16 or pairs <= MOE_STREAM_PAIRS * experts)
-    tile_rows = 128 if tcgen05 else (8 if rows <= 8 else 16) if streamed else MOE_TILE_ROWS
+    pair = tcgen05 and pairs >= MOE_PAIR_ROWS * experts
+    tile_rows = (256 if pair else 128) if tcgen05 else (8 if rows <= 8 else 16) if streamed else MOE_TILE_ROWS
     max_tiles = min(pairs, -(-pairs // tile_rows) + experts)
     def chosen() -> tuple:
         """The choices, and every chosen expert's output."""
@@ -2011,7 +2017,8 @@ def moe_experts(h: torch.Tensor, router: torch.Tensor | None, correction: torch.
                 fn = _function("moe", "omnia_moe_gather", [c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p])
                 _check(fn(_ptr(h), _ptr(source), _ptr(offsets[experts:]), _ptr(sorted_rows), pairs, hidden, _code(h.dtype),
                           _stream()), "moe_gather")
-            grouped = _function("gemm_tcgen05", "omnia_gemm_tcgen05_grouped",
+            grouped = _function(*(("gemm_tcgen05_pair", "omnia_gemm_tcgen05_pair_grouped") if pair else
+                                  ("gemm_tcgen05", "omnia_gemm_tcgen05_grouped")),
                                 [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_int,
                                  c_float, c_float, c_void_p, c_void_p])
             err = _ptr(error_word(device))
