@@ -687,11 +687,12 @@ def paged_attention(q: torch.Tensor | None, kv: KVView, step: StepContext, scale
     # Requests that bring a single token take the split-key decode kernel, in a decode-only step
     # (all of them, no index list: the shape a captured graph replays) and in a mixed step alike.
     single, longest = (None, step.max_seq_len) if step.decode_only else _single_token_requests(step, q.device)
-    if step.decode_only or single is not None:
+
+    def single_tokens(beside: bool) -> None:
         count = step.num_seqs if step.decode_only else single.shape[0]
-        longest = width_bucket(-(-longest // kv.page_size)) * kv.page_size
-        chunk, warps = decode_plan(count, nkv, longest, sm_count(q.device))
-        max_chunks = -(-longest // chunk)
+        held = width_bucket(-(-longest // kv.page_size)) * kv.page_size
+        chunk, warps = decode_plan(count, nkv, held, sm_count(q.device))
+        max_chunks = -(-held // chunk)
         part_o, part_ml, tickets = _step_buffers(step, q.device, {
             "attention_part_o": (count * nq * max_chunks * d, torch.float32, False),
             "attention_part_ml": (count * nq * max_chunks * 2, torch.float32, False),
@@ -700,7 +701,8 @@ def paged_attention(q: torch.Tensor | None, kv: KVView, step: StepContext, scale
                        [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                         c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                         c_float, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p,
-                        c_int, c_int, c_void_p, c_int, c_float, c_float, c_float, c_float, c_int, c_void_p, c_void_p], defines)
+                        c_int, c_int, c_void_p, c_int, c_float, c_float, c_float, c_float, c_int, c_int, c_void_p, c_void_p],
+                       defines)
         p = projection
         fused = (None, 0, 0, 0, 0, -1.0, None, None) if p is None else (
             _ptr(p.rows), p.rows.shape[1], p.q_col, p.k_col, p.v_col, -1.0 if p.eps is None else p.eps,
@@ -708,10 +710,14 @@ def paged_attention(q: torch.Tensor | None, kv: KVView, step: StepContext, scale
         _check(fn(None if p is not None else _ptr(q), _ptr(kv.pages), _ptr(kv.block_table), _ptr(step.cu_seqlens),
                   _ptr(step.seq_lens), _ptr(single), count, _ptr(part_o), _ptr(part_ml), _ptr(tickets), chunk,
                   max_chunks, gate_ptr, gate_stride, _ptr(out), max_pages, num_pages, nq, nkv, kv.page_size,
-                  kv.window or 0, scale, warps, *fused, 1, keep, _ptr(sink), run, softcap, *last, err, _stream()),
+                  kv.window or 0, scale, warps, *fused, 1, keep, _ptr(sink), run, softcap, *last, int(beside), err, _stream()),
                "attention_decode")
-        if step.decode_only or all(n == 1 for n in step.q_lens):
-            return out
+
+    if step.decode_only or (single is not None and all(n == 1 for n in step.q_lens)):
+        single_tokens(False)
+        return out
+    # A mixed step launches its prompts' kernel first (its few long blocks take their places), then the single tokens'
+    # beside it: neither reads what the other writes.
     if tcgen05_attention_supported(q.dtype, nq, nkv, d, kv.page_size):
         per_block = 128 // (nq // nkv)
         sms = sm_count(q.device)
@@ -731,6 +737,8 @@ def paged_attention(q: torch.Tensor | None, kv: KVView, step: StepContext, scale
             _check(fn(_ptr(q), tokens, _ptr(kv.pages), _ptr(kv.block_table), _ptr(step.cu_seqlens), _ptr(step.seq_lens),
                       _ptr(work), work.shape[0], gate_ptr, gate_stride, _ptr(out), max_pages, num_pages, nq, nkv,
                       kv.page_size, kv.window or 0, scale, err, _stream()), "attention_prefill_tcgen05_wide")
+            if single is not None:
+                single_tokens(True)
             return out
         work = _prefill_work_flat(step, per_block, 64, nkv, kv.window or 0, q.device, prefill_places(sms) if plain else 0,
                                   run)
@@ -749,6 +757,8 @@ def paged_attention(q: torch.Tensor | None, kv: KVView, step: StepContext, scale
                   _ptr(work), work.shape[0], gate_ptr, gate_stride, _ptr(out), _ptr(partial), _ptr(tickets), max_pages,
                   num_pages, nq, nkv, kv.page_size, kv.window or 0, scale, keep, _ptr(sink), run, softcap, *last, err, _stream()),
                "attention_prefill_tcgen05")
+        if single is not None:
+            single_tokens(True)
         return out
     tokens_per_block = 64 // (nq // nkv)
     work = _prefill_work(step, tokens_per_block, q.device)
@@ -759,6 +769,8 @@ def paged_attention(q: torch.Tensor | None, kv: KVView, step: StepContext, scale
     _check(fn(_ptr(q), _ptr(kv.pages), _ptr(kv.block_table), _ptr(step.cu_seqlens), _ptr(step.seq_lens), _ptr(work),
               work.shape[0], gate_ptr, gate_stride, _ptr(out), max_pages, num_pages, nq, nkv, kv.page_size,
               kv.window or 0, scale, keep, _ptr(sink), run, softcap, *last, err, _stream()), "attention_prefill")
+    if single is not None:
+        single_tokens(True)
     return out
 
 

@@ -205,6 +205,36 @@ def test_paged_attention(ops, dtype, nq, nkv, d, page, window):
     ops.raise_on_error(q.device)
 
 
+@pytest.mark.parametrize("nq,nkv,d,page,window", [(16, 8, 128, 16, None), (4, 2, 16, 4, None), (6, 3, 64, 16, 500)])
+@pytest.mark.parametrize("q_lens,seq_lens", [([1, 256, 1, 1], [4000, 256, 9, 700]), ([300, 1], [1300, 1]),
+                                             ([1] * 11 + [17, 2], [1 + 331 * i for i in range(11)] + [17, 900])])
+def test_single_tokens_beside_prompts(ops, nq, nkv, d, page, window, q_lens, seq_lens):
+    """A mixed step's two attention kernels run side by side: the rows of each are what they are when its requests
+    come alone, and the same bits run after run."""
+    step = step_of(q_lens, seq_lens)
+    pages, table = make_kv(seq_lens, nkv, d, page, torch.bfloat16, 8 + sum(-(-n // page) for n in seq_lens), seed=3)
+    pages.normal_(generator=torch.Generator(device="cuda").manual_seed(4))
+    q = rand(step.num_tokens, nq, d, dtype=torch.bfloat16, seed=11)
+    gate = rand(step.num_tokens, nq * d, dtype=torch.bfloat16, seed=12)
+
+    def view(keep):
+        return KVView(pages, table[keep], torch.zeros(1, dtype=torch.int64, device="cuda"), page, window)
+
+    every = list(range(len(q_lens)))
+    first = ops.paged_attention(q, view(every), step, d ** -0.5, gate=gate)
+    close(first, kernel_refs.paged_attention(q, view(every), step, d ** -0.5, gate=gate), torch.bfloat16)
+    for _ in range(20):
+        assert torch.equal(ops.paged_attention(q, view(every), step, d ** -0.5, gate=gate), first)
+    starts = [sum(q_lens[:s]) for s in every]
+    for single in (True, False):
+        keep = [s for s in every if (q_lens[s] == 1) == single]
+        rows = torch.tensor([starts[s] + i for s in keep for i in range(q_lens[s])], device="cuda")
+        alone = ops.paged_attention(q[rows], view(keep), step_of([q_lens[s] for s in keep], [seq_lens[s] for s in keep]),
+                                    d ** -0.5, gate=gate[rows])
+        close(alone, first[rows], torch.bfloat16)
+    ops.raise_on_error(q.device)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("nq,nkv,d,page,window", [(6, 3, 128, 16, 33), (16, 8, 64, 16, 20), (6, 3, 128, 16, None),
                                                    (4, 2, 128, 32, 100), (8, 1, 24, 8, 16), (5, 5, 40, 4, 70)])
