@@ -864,12 +864,13 @@ def _pair_pays(rows: int, n: int, k: int, epilogue: int, sms: int) -> bool:
     if epilogue == 1:
         # gate|up with SwiGLU: tiles of 128 output columns, 128 rows to an SM or 256 to a pair. What
         # decides is how many waves of tiles each kernel runs (measured, 12,288 weight rows of 2,048:
-        # some 10 us and 14 a wave for one SM, 9 and 11 a wave for a pair; 512 / 1,082 rows: 38 / 53.5 us
-        # against 29.6 / 52).
+        # some 10 us and 14 a wave for one SM, 9 and 11 a wave for a pair; 512 / 1,082 rows: 38 / 53 us
+        # against 29.6 / 52). A pair's wave counts as 12: where pairs run one wave more than a few, what they gain
+        # depends on the depth (1,082 rows of 4,096: 90 us against 93), and one SM keeps those.
         tiles = -(-(n // 2) // 128)
         one = -(-(-(-rows // 128) * tiles) // sms)
         two = -(-(-(-rows // 256) * tiles) // (sms // 2))
-        return 9 + 11 * two < 10 + 14 * one
+        return 9 + 12 * two < 10 + 14 * one
     tiles = -(-rows // 256) * -(-n // 256)
     return tiles * -(-k // 64) >= 64 * (sms // 2)
 
