@@ -159,7 +159,7 @@ class CacheManager:
             elif need.state is not None:
                 self.state[entry] = slots_of(need.state)
                 if need.initial_state is not None:
-                    self.initial_state[entry] = need.initial_state.to(need.state.dtype).to(device)
+                    self.initial_state[entry] = need.initial_state.to(need.state.dtype).to(device).expand(need.state.shape).contiguous()
             if getattr(need, "block_state", None):
                 self.block_state[entry] = {name: slots_of(spec) for name, spec in need.block_state.items()}
         # State that belongs to the model and to no schedule entry (an embedding that looks at the token before).
@@ -172,23 +172,25 @@ class CacheManager:
         the mixer's `initial_state()` where it gave one, zeros everywhere else."""
         if not slots or not (self.state or self.block_state or self.model_state):
             return
-        index = None
-        for tensor in self.model_state.values():
-            if index is None:
-                index = torch.as_tensor(slots, device=tensor.device)
-            tensor.index_fill_(0, index, 0)
+        held: list[tuple[torch.Tensor, torch.Tensor | None]] = [(t, None) for t in self.model_state.values()]
         for entry in sorted(set(self.state) | set(self.block_state)):
-            held = self.state.get(entry)
-            tensors = list(held.values()) if isinstance(held, dict) else ([held] if held is not None else [])
-            tensors += list(self.block_state.get(entry, {}).values())
-            for tensor in tensors:
-                if index is None:
-                    index = torch.as_tensor(slots, device=tensor.device)
-                initial = self.initial_state.get(entry) if tensor is held else None
-                if initial is None:
-                    tensor.index_fill_(0, index, 0)
-                else:
-                    tensor[index] = initial
+            own = self.state.get(entry)
+            if isinstance(own, dict):
+                held += [(t, None) for t in own.values()]
+            elif own is not None:
+                held.append((own, self.initial_state.get(entry)))
+            held += [(t, None) for t in self.block_state.get(entry, {}).values()]
+        if held and held[0][0].is_cuda:
+            from mlx_omnia_b200.kernels import ops
+
+            ops.fill_slots(held, slots)
+            return
+        index = torch.as_tensor(slots)
+        for tensor, initial in held:
+            if initial is None:
+                tensor.index_fill_(0, index, 0)
+            else:
+                tensor[index] = initial
 
     # -- sizes -----------------------------------------------------------------------
     @staticmethod

@@ -811,6 +811,28 @@ def gather_rows(src: torch.Tensor, rows: torch.Tensor) -> torch.Tensor:
     return out
 
 
+FILL_TENSORS, FILL_SLOTS = 32, 128  # of one launch (elementwise.cu)
+
+
+def fill_slots(tensors: list[tuple[torch.Tensor, torch.Tensor | None]], slots: list[int]) -> None:
+    """In place: rows `slots` of every tensor of the list (contiguous, of whatever type) become the tensor beside it
+    (a row's shape, the same type, contiguous), or zeros where there is none."""
+    fn = _function("elementwise", "omnia_fill_slots", [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p])
+    for t, start in tensors:
+        if not t.is_contiguous() or any(not 0 <= s < t.shape[0] for s in slots) or \
+                start is not None and (start.shape != t.shape[1:] or start.dtype != t.dtype or not start.is_contiguous()):
+            raise KernelError("fill_slots takes contiguous tensors, slots inside them, and a row of the same shape and type")
+    tensors = [(t, start) for t, start in tensors if t[0].numel()]
+    for i in range(0, len(tensors), FILL_TENSORS):
+        part = tensors[i: i + FILL_TENSORS]
+        to = (c_void_p * len(part))(*(t.data_ptr() for t, _ in part))
+        start = (c_void_p * len(part))(*(_ptr(x) for _, x in part))
+        size = (c_longlong * len(part))(*(t[0].numel() * t.element_size() for t, _ in part))
+        for j in range(0, len(slots), FILL_SLOTS):
+            some = (c_int * len(slots[j: j + FILL_SLOTS]))(*slots[j: j + FILL_SLOTS])
+            _check(fn(to, start, size, len(part), some, len(some), _stream()), "fill_slots")
+
+
 SKINNY_ROWS = 16
 """Up to this many activation rows, bfloat16 products run on the weight-streaming kernel."""
 

@@ -417,6 +417,26 @@ def test_swiglu_softcap_gather(ops, dtype):
     assert torch.equal(ops.gather_rows(z, rows), kernel_refs.gather_rows(z, rows))
 
 
+@pytest.mark.parametrize("tensors,slots", [(1, 1), (3, 2), (33, 5), (2, 130)])
+def test_fill_slots(ops, tensors, slots):
+    """Chosen rows become the given row or zeros, whatever a row's size in bytes; the rest stays."""
+    shapes = [((7,), torch.bfloat16), ((3, 5), torch.float32), ((64, 128), torch.float32), ((2, 8), torch.bfloat16), ((), torch.int32)]
+    total = slots + 40
+    chosen = torch.randperm(total, generator=torch.Generator().manual_seed(slots))[:slots].tolist()
+    held, want = [], []
+    for i in range(tensors):
+        shape, dtype = shapes[i % len(shapes)]
+        t = (rand(total, *shape, seed=i) * 9).to(dtype)
+        start = None if i % 3 else (rand(*shape, seed=100 + i) * 9).to(dtype)
+        held.append((t, start))
+        want.append(t.clone())
+        want[-1][chosen] = torch.zeros_like(t[0]) if start is None else start
+    ops.fill_slots(held, chosen)
+    assert all(torch.equal(t, w) for (t, _), w in zip(held, want))
+    with pytest.raises(ops.KernelError, match="slots inside"):
+        ops.fill_slots(held, [total])
+
+
 def test_linear_is_true_float32(ops):
     a, w = rand(33, 517, seed=1), rand(129, 517, seed=2)
     expect = (a.double() @ w.double().t()).float()
