@@ -420,7 +420,7 @@ def test_swiglu_softcap_gather(ops, dtype):
 @pytest.mark.parametrize("tensors,slots", [(1, 1), (3, 2), (33, 5), (2, 130)])
 def test_fill_slots(ops, tensors, slots):
     """Chosen rows become the given row or zeros, whatever a row's size in bytes; the rest stays."""
-    shapes = [((7,), torch.bfloat16), ((3, 5), torch.float32), ((64, 128), torch.float32), ((2, 8), torch.bfloat16), ((), torch.int32)]
+    shapes = [((7,), torch.bfloat16), ((3, 5), torch.float32), ((64, 128), torch.float32), ((2, 8), torch.bfloat16), ((1,), torch.int32)]
     total = slots + 40
     chosen = torch.randperm(total, generator=torch.Generator().manual_seed(slots))[:slots].tolist()
     held, want = [], []
