@@ -20,8 +20,8 @@
 // spends most of its instructions there: what the loaders do per element decides the kernel's pace. A token's partial sums stay in registers until its run is done,
 // so the shuffles that add them up are off the chain from token to token, which is one fused
 // multiply-add a row. The state, the decay and every sum stay float32. It serves decode steps (one
-// token a request) and prompts' portions of any length alike; the order of a column's additions does
-// not depend on how a prompt was cut.
+// token a request), float32, and portions too short or heads too odd for lightning_chunk.cu; the order of a
+// column's additions does not depend on how such portions were cut.
 //
 // Compiled per key width: -DLIGHTNING_DK=<DK>.
 #include "common.cuh"

@@ -287,6 +287,32 @@ def test_decayed_state_over_portions_and_slots(dtype, H, dk, dv, parts):
     ops.raise_on_error(CUDA)
 
 
+@pytest.mark.parametrize("H,dk,dv", [(3, 128, 128), (2, 16, 16), (2, 64, 48), (1, 256, 32), (40, 32, 64), (2, 48, 32)])
+@pytest.mark.parametrize("lens", [(1, 16, 17, 33), (127, 128), (129, 300, 5), (2048,)])
+def test_decayed_state_in_chunks(H, dk, dv, lens):
+    """The chunked recurrence and the one that goes token by token, from the same states: they have the same operands
+    (activated and rounded alike) and differ by the order of float32 sums, a few 2^-24 of the largest entry; the
+    states carry over, nobody else's slot is touched, rows that start on odd places are taken."""
+    g = torch.Generator().manual_seed(dk + dv + len(lens))
+    width = 2 * H * dk + 2 * H * dv
+    proj = (torch.randn(sum(lens), width + 3, generator=g) * 1.5).to(torch.bfloat16).to(CUDA)
+    decay = torch.tensor(([1.0, 0.999, 0.5, 0.0] + [0.97] * H)[:H] if H > 1 else [0.995], device=CUDA)
+    w = (1.0 + 0.2 * torch.randn(H * dv, generator=g)).to(CUDA)
+    slots = list(range(len(lens), 0, -1))
+    start = torch.randn(len(lens) + 2, H, dk, dv, generator=g).to(CUDA) * 5
+    step = Batch(list(lens), [7] * len(lens), slots)
+    states, outs = [], []
+    for chunked in (False, True):
+        S = start.clone()
+        outs.append(ops.lightning_attention(proj, 3, 3 + H * dk, 3 + 2 * H * dk, 3 + 2 * H * dk + H * dv, H, dk, dv, decay, w, 1e-5,
+                                            S, step, chunked=chunked))
+        states.append(S)
+    assert torch.equal(states[1][0], start[0]) and torch.equal(states[1][-1], start[-1])
+    assert rel(states[1], states[0]) < 5e-6
+    assert rel(outs[1], outs[0]) <= 2.0 ** -7  # a rounding to bfloat16 may fall the other way: one unit of its last place
+    ops.raise_on_error(CUDA)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("rows", [3, 40, 400])
 def test_relu_gated_unit(dtype, rows):
