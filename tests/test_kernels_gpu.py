@@ -71,6 +71,21 @@ def test_rmsnorm_and_add_rmsnorm(ops, dtype, rows, hidden):
             close(h1, h2, dtype)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("rows,hidden", [(601, 72), (600, 1028), (593, 2048), (700, 4100), (592, 8192)])
+def test_residual_step_of_many_rows(ops, dtype, rows, hidden):
+    """The kernel that reads the norms' weights late, at widths that fill its threads and that do not."""
+    x = rand(rows, hidden, scale=3.0, seed=1)
+    branch = rand(rows, hidden, dtype=dtype, scale=0.3, seed=3)
+    wb, wo = 1 + rand(hidden, scale=0.1, seed=4), 1 + rand(hidden, scale=0.1, seed=5)
+    for args in [(wb, 1e-6, wo, 1e-5), (None, None, wo, 1e-5), (wb, 1e-6, None, None), (None, 1e-6, None, 1e-5)]:
+        x1, x2 = x.clone(), x.clone()
+        h1, h2 = ops.add_rmsnorm(x1, branch, *args), kernel_refs.add_rmsnorm(x2, branch, *args)
+        close(x1, x2, torch.float32)
+        if h2 is not None:
+            close(h1, h2, dtype)
+
+
 def make_kv(tokens, nkv, d, page_size, dtype, num_pages, seed=0):
     """A cache view with one request per row of `tokens` (a list of lengths): random page
     placement, every other page poisoned with huge values."""
@@ -415,6 +430,17 @@ def test_swiglu_softcap_gather(ops, dtype):
     close(ops.softcap(z, 2.0, None), kernel_refs.softcap(z, 2.0, None), torch.float32)
     rows = torch.tensor([6, 0, 3, 3], dtype=torch.int32, device="cuda")
     assert torch.equal(ops.gather_rows(z, rows), kernel_refs.gather_rows(z, rows))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("rows,inner", [(1, 8), (17, 2048), (33, 2056), (3, 20000), (5, 12)])
+def test_gated_units_and_soft_cap_by_sixteen_bytes(ops, dtype, rows, inner):
+    gu = rand(rows, 2 * inner, dtype=dtype, scale=3.0)
+    close(ops.swiglu(gu), kernel_refs.swiglu(gu), dtype)
+    g, u = gu[:, :inner].float().clamp(max=2.0), gu[:, inner:].float().clamp(-2.0, 2.0)
+    close(ops.clamped_glu(gu, 1.7, 2.0), (g * torch.sigmoid(1.7 * g) * (u + 1)).to(dtype), dtype)
+    for z in (gu, gu.flatten()[1:]):  # on sixteen bytes, and not
+        close(ops.softcap(z, 0.5, 20.0), kernel_refs.softcap(z, 0.5, 20.0), torch.float32, scale=10)
 
 
 @pytest.mark.parametrize("tensors,slots", [(1, 1), (3, 2), (33, 5), (2, 130)])
