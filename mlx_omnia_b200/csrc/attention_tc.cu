@@ -341,7 +341,8 @@ attention_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pa
     __syncthreads();
   }
   cp_async_wait<0>();
-  pdl_launch_dependents();  // the cache is read: the next kernel may begin its preamble
+  pdl_launch_dependents();  // the cache is read: the next kernel may begin its preamble (and in a mixed step the decode
+                            // kernel, `beside`: never ahead of the wait)
 
   // Normalise, gate, store.
 #pragma unroll
@@ -553,7 +554,8 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
   // tokens were written in earlier steps), so the block's start and its first loads of the cache
   // run while that kernel finishes. Every block waits before it leaves, also one with nothing to do.
   // `beside`: the kernel before this one is the same step's attention of longer entries, which lets this one begin once
-  // it has itself waited for what both read. The two share no output, so the blocks run beside it; those that merge
+  // it has itself waited for what both read (every block of the three prompts' kernels triggers behind its own wait, and
+  // the caller says `beside` only where that kernel has blocks). The two share no output, so the blocks run beside it; those that merge
   // (every request has them) wait for it before they leave, so this grid does not end ahead of it and whoever comes
   // next comes after both. The others leave at once: a waiting block would keep its place from one with work to do.
   // Eight single tokens of up to 4,096 positions and 256 of a prompt: 27 us and 21 us one after the other, 30 so (40

@@ -154,7 +154,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   // (the launch is a programmatic dependent launch); from here on its results are read.
   OMNIA_TRACE_BLOCK(2);
   pdl_wait();
-  pdl_launch_dependents();
+  pdl_launch_dependents();  // never ahead of the wait (see attention_tc.cu, `beside`)
   OMNIA_TRACE_BLOCK(3);
 
   if ((warp >= WARP_K && warp < WARP_K + FEEDERS) || (warp >= WARP_V && warp < WARP_V + FEEDERS)) {

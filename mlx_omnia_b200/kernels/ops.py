@@ -713,7 +713,9 @@ def paged_attention(q: torch.Tensor | None, kv: KVView, step: StepContext, scale
                   kv.window or 0, scale, warps, *fused, 1, keep, _ptr(sink), run, softcap, *last, int(beside), err, _stream()),
                "attention_decode")
 
-    if step.decode_only or (single is not None and all(n == 1 for n in step.q_lens)):
+    # `beside` leaves the wait for the kernel that wrote q and the cache to the prompts' kernel in front: only where that
+    # one has blocks, which takes an entry of several tokens (one of none has no block, and its launch is nothing).
+    if step.decode_only or (single is not None and all(n <= 1 for n in step.q_lens)):
         single_tokens(False)
         return out
     # A mixed step launches its prompts' kernel first (its few long blocks take their places), then the single tokens'

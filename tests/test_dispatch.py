@@ -1,6 +1,13 @@
 """Host-side choices of the kernel dispatcher that need no GPU."""
 
+from types import SimpleNamespace
+
+import numpy as np
+import pytest
+import torch
+
 from mlx_omnia_b200.kernels import ops
+from mlx_omnia_b200.parts.base import KVView
 
 
 def test_width_bucket_keeps_three_bits_and_is_its_own_fixed_point():
@@ -219,3 +226,33 @@ def test_lightning_parts_divide_the_columns_and_fit_a_block():
     # One prompt of 16 heads: blocks for three quarters of the SMs, not two blocks an SM for the rest.
     assert ops.lightning_parts(1, 16, 128, 148) == 8
     assert ops.lightning_parts(64, 16, 128, 148) == 2
+
+
+@pytest.mark.parametrize("d,page", [(64, 16), (16, 4)])  # prompts on tcgen05 and on mma.sync
+@pytest.mark.parametrize("q_lens,beside", [([1, 4, 1], 1), ([1, 0, 1], 0), ([0, 1], 0), ([0, 1, 2], 1), ([1, 1], 0)])
+def test_single_tokens_run_beside_a_prompts_kernel_only_where_there_is_one(monkeypatch, d, page, q_lens, beside):
+    """The single tokens' attention leaves its wait to the prompts' kernel in front of it, so it may do that only
+    behind a launch that has blocks: an entry of no tokens gives that kernel none."""
+    calls = []
+
+    def function(library, name, argtypes, defines=None):
+        def call(*args):
+            assert len(args) == len(argtypes)
+            calls.append((name, args))
+            return 0
+        return call
+
+    monkeypatch.setattr(ops, "_function", function)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    monkeypatch.setattr(ops, "_ints_to_device", lambda values, device: torch.from_numpy(np.ascontiguousarray(values)))
+    monkeypatch.setattr(ops, "error_word", lambda device: torch.zeros(1, dtype=torch.int32))
+    monkeypatch.setattr(ops, "_step_buffers", lambda step, device, wanted: [torch.zeros(1)] * len(wanted))
+    held = [300 + n for n in q_lens]
+    step = SimpleNamespace(num_seqs=len(q_lens), q_lens=q_lens, seq_lens_host=held, max_seq_len=max(held), decode_only=False,
+                           workspace=None, cu_seqlens=torch.zeros(4), seq_lens=torch.zeros(3), positions=torch.zeros(9))
+    kv = KVView(torch.zeros(2, 2, 2, page, d, dtype=torch.bfloat16), torch.zeros(len(q_lens), 100, dtype=torch.int32), None, page, None)
+    ops.paged_attention(torch.zeros(sum(q_lens), 4, d, dtype=torch.bfloat16), kv, step, 1.0)
+    launched = [name for name, _ in calls if "part_floats" not in name]
+    assert launched[-1] == "omnia_attention_decode_tc" and len(launched) == 1 + beside
+    assert calls[-1][1][-3] == beside and (not beside or "prefill" in launched[0])
