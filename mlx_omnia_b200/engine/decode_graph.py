@@ -242,6 +242,8 @@ class MixedGraphs:
     def run(self, key: tuple, entries, copy: bool = True) -> torch.Tensor:
         runner = self.runner
         for entry in entries:
+            if not entry.tokens:
+                raise ValueError(f"request {entry.request.request_id!r} brings no tokens to this step")
             if any(not 0 <= w < len(entry.tokens) for w in entry.want):
                 raise ValueError(f"request {entry.request.request_id!r}: a wanted place lies outside its tokens")
         starts = runner.take_pages(entries)

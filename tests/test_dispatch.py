@@ -256,3 +256,14 @@ def test_single_tokens_run_beside_a_prompts_kernel_only_where_there_is_one(monke
     launched = [name for name, _ in calls if "part_floats" not in name]
     assert launched[-1] == "omnia_attention_decode_tc" and len(launched) == 1 + beside
     assert calls[-1][1][-3] == beside and (not beside or "prefill" in launched[0])
+
+
+def test_a_replayed_mixed_step_refuses_an_entry_without_tokens():
+    """As an uncaptured step does, and before any page is taken."""
+    from mlx_omnia_b200.engine.decode_graph import MixedGraphs
+    from mlx_omnia_b200.engine.step import StepEntry
+
+    graphs = MixedGraphs(SimpleNamespace(cache=SimpleNamespace(groups=[], page_size=16, capacity_tokens=lambda: 0)))
+    entries = [StepEntry(SimpleNamespace(request_id=name), tokens, []) for name, tokens in (("a", [1, 2]), ("b", []))]
+    with pytest.raises(ValueError, match="'b' brings no tokens"):
+        graphs.run(("a shape",), entries)
