@@ -2039,6 +2039,8 @@ def moe_experts(h: torch.Tensor, router: torch.Tensor | None, correction: torch.
     device = h.device
     if step is None:
         step = _NoStep()
+    if (tensor_cores or tcgen05) and h.dtype != torch.bfloat16:
+        raise KernelError(f"the experts' products on the tensor cores take bfloat16, not {h.dtype}")
     if tensor_cores is None:
         tensor_cores = h.dtype == torch.bfloat16 and hidden % 8 == 0 and inner % 8 == 0
     if tcgen05 is None:

@@ -267,3 +267,21 @@ def test_a_replayed_mixed_step_refuses_an_entry_without_tokens():
     entries = [StepEntry(SimpleNamespace(request_id=name), tokens, []) for name, tokens in (("a", [1, 2]), ("b", []))]
     with pytest.raises(ValueError, match="'b' brings no tokens"):
         graphs.run(("a shape",), entries)
+
+
+@pytest.mark.parametrize("rows", [1, 16, 17, 600])
+def test_experts_on_the_tensor_cores_take_bfloat16_only(monkeypatch, rows):
+    """Every kernel that a step of so many rows would choose reads its operands as bfloat16."""
+    monkeypatch.setattr(ops, "_function", lambda *a: lambda *args: 0)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops, "error_word", lambda device: torch.zeros(1, dtype=torch.int32))
+    monkeypatch.setattr(ops, "_step_buffers", lambda step, device, wanted: [torch.zeros(1, dtype=torch.int32)] * len(wanted))
+
+    def experts(dtype):
+        return ops.moe_experts(torch.zeros(rows, 16, dtype=dtype), None, None, torch.zeros(3, 16, 16, dtype=dtype),
+                               torch.zeros(3, 16, 8, dtype=dtype), 2, None, tensor_cores=True, token_ids=torch.zeros(rows, dtype=torch.int32),
+                               table=torch.zeros(5, 2, dtype=torch.int32))
+
+    assert experts(torch.bfloat16).shape == (rows, 16)
+    with pytest.raises(ops.KernelError, match="bfloat16"):
+        experts(torch.float32)
