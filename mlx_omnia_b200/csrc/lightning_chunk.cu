@@ -16,6 +16,12 @@
 // 5.8e-7; with running sums 2e-6 both), after 128: 7.6e-8 and 6.5e-8 (6.0e-8 and 1.8e-7). The powers of the decay are
 // made in float64 and rounded once.
 //
+// That holds for finite numbers of ordinary size. Where something is infinite or NaN (or overflows on its way through a
+// product, or as a bfloat16), a chunk's products would carry it to tokens that come before it, since a weight of zero
+// times it is NaN, and would make NaN of an infinity taken apart. Whatever went in, an output or the last state that is
+// not finite comes of it; the block then walks its tokens once more, one by one as lightning.cu does, from the state in
+// memory, which it writes only at its end. (The parts of a number below 2^-109 lose bits to bfloat16's smallest exponent.)
+//
 // A block owns LIGHTNING_COLS value columns of one head of one request and walks its chunks in order; a column of S
 // needs no other column. Warp w has 16 of the chunk's tokens for the first three products (the tokens dealt so that the
 // two warps of a scheduler have equal shares of the triangle) and 16 of the state's rows for the last, whose float32
@@ -167,20 +173,24 @@ lightning_chunk_kernel(const bf16* __restrict__ rows, int H, int dv, const float
   const int m0 = (warp / CW) * MPW, c0 = (warp % CW) * NTW * 8;
   float S[MPW][NTW][4];
   float* mine = S_state + ((size_t)state_slots[seq] * H + head) * N * dv + col0 + c0 + 2 * t4;
+  auto read_state = [&]() {
 #pragma unroll
-  for (int m = 0; m < MPW; ++m)
+    for (int m = 0; m < MPW; ++m)
 #pragma unroll
-    for (int nt = 0; nt < NTW; ++nt)
+      for (int nt = 0; nt < NTW; ++nt)
 #pragma unroll
-      for (int side = 0; side < 2; ++side) {
-        float2 v = make_float2(0.f, 0.f);
-        if (m0 + m < MT) v = *reinterpret_cast<const float2*>(mine + (size_t)((m0 + m) * 16 + g + 8 * side) * dv + nt * 8);
-        S[m][nt][2 * side] = v.x, S[m][nt][2 * side + 1] = v.y;
-      }
+        for (int side = 0; side < 2; ++side) {
+          float2 v = make_float2(0.f, 0.f);
+          if (m0 + m < MT) v = *reinterpret_cast<const float2*>(mine + (size_t)((m0 + m) * 16 + g + 8 * side) * dv + nt * 8);
+          S[m][nt][2 * side] = v.x, S[m][nt][2 * side + 1] = v.y;
+        }
+  };
+  read_state();
 
   const int tile = WARPS == 8 && warp >= 4 ? 11 - warp : warp, row0 = tile * 16;
   const int chunks = (end - begin + L - 1) / L;
   fetch(begin, min(L, end - begin), 0);
+  float probe = 0.f;  // NaN once something this thread made was not finite
   for (int c = 0; c < chunks; ++c) {
     const int t0 = begin + c * L, n = min(L, end - t0), b = c & 1;
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -294,8 +304,10 @@ lightning_chunk_kernel(const bf16* __restrict__ rows, int H, int dv, const float
         if (r >= n) continue;
         float* out = o_raw + (size_t)(t0 + r) * H * dv + head * dv + col0 + 2 * t4;
 #pragma unroll
-        for (int nt = 0; nt < NT; ++nt)
+        for (int nt = 0; nt < NT; ++nt) {
           *reinterpret_cast<float2*>(out + nt * 8) = make_float2(acc[nt][2 * side], acc[nt][2 * side + 1]);
+          probe = fmaf(acc[nt][2 * side + 1], 0.f, fmaf(acc[nt][2 * side], 0.f, probe));
+        }
       }
     }
     const float kept = power[n];
@@ -336,6 +348,60 @@ lightning_chunk_kernel(const bf16* __restrict__ rows, int H, int dv, const float
           }
         }
       }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < MPW; ++m)
+#pragma unroll
+    for (int nt = 0; nt < NTW; ++nt)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) probe = fmaf(S[m][nt][e], 0.f, probe);
+  if (__syncthreads_or(probe != 0.f)) {
+    constexpr int SHARES = WARPS / CW;           // warps that hold rows of a column
+    float* sums = reinterpret_cast<float*>(Ws);  // [2][SHARES][COLS], of alternate tokens
+    const bf16 *Kc = stage0, *Qc = Kc + L * NROW, *Vc = Qc + L * NROW;
+    const float d = decay[head];
+    read_state();
+#pragma unroll 1
+    for (int t0 = begin; t0 < end; t0 += L) {
+      const int n = min(L, end - t0);
+      fetch(t0, n, 0);
+      asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+      __syncthreads();
+#pragma unroll 1
+      for (int i = 0; i < n; ++i) {
+        float* share = sums + ((i & 1) * SHARES + warp / CW) * COLS + c0 + 2 * t4;
+#pragma unroll
+        for (int nt = 0; nt < NTW; ++nt) {
+          const float2 v = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(Vc + i * XROW + c0 + nt * 8 + 2 * t4));
+          float2 o = make_float2(0.f, 0.f);
+#pragma unroll
+          for (int m = 0; m < MPW; ++m)
+#pragma unroll
+            for (int side = 0; side < 2; ++side) {
+              if (m0 + m >= MT) continue;
+              const int at = i * NROW + (m0 + m) * 16 + g + 8 * side;
+              const float k = __bfloat162float(Kc[at]), q = __bfloat162float(Qc[at]);
+              float* s = S[m][nt] + 2 * side;
+              s[0] = fmaf(k, v.x, d * s[0]), s[1] = fmaf(k, v.y, d * s[1]);
+              o.x = fmaf(s[0], q, o.x), o.y = fmaf(s[1], q, o.y);
+            }
+#pragma unroll
+          for (int w = 4; w < 32; w <<= 1) {
+            o.x += __shfl_xor_sync(0xffffffffu, o.x, w);
+            o.y += __shfl_xor_sync(0xffffffffu, o.y, w);
+          }
+          if (g == 0) *reinterpret_cast<float2*>(share + nt * 8) = o;
+        }
+        __syncthreads();
+        if (tid < COLS) {
+          float o = 0.f;
+#pragma unroll
+          for (int w = 0; w < SHARES; ++w) o += sums[((i & 1) * SHARES + w) * COLS + tid];
+          o_raw[(size_t)(t0 + i) * H * dv + head * dv + col0 + tid] = o;
+        }
+      }
+      __syncthreads();  // the stage and the sums may be written again
     }
   }
 #pragma unroll

@@ -313,6 +313,85 @@ def test_decayed_state_in_chunks(H, dk, dv, lens):
     ops.raise_on_error(CUDA)
 
 
+@pytest.mark.parametrize("H,dk,dv", [(2, 128, 64), (1, 16, 48), (1, 256, 32), (2, 48, 32)])
+@pytest.mark.parametrize("what", ["infinite v", "nan k", "infinite q", "infinite state", "nan state", "product too large", "v too small"])
+def test_what_is_not_finite_in_a_chunk_stays_where_it_belongs(H, dk, dv, what):
+    """A value that is infinite or NaN, and a product of operands that overflows where the recurrence itself does
+    not, reach the tokens, columns and state entries that they reach token by token, and no others; the numbers
+    around them stay what they are. Bounds as in the test above."""
+    g = torch.Generator().manual_seed(dk + len(what))
+    lens, t = (300, 150), 45  # the second block of 32 keys of the first chunk, and of the other entry's
+    width = 2 * H * dk + 2 * H * dv
+    proj = torch.randn(sum(lens), width, generator=g) * 1.5
+    q, k, v = proj[:, : H * dk], proj[:, H * dk: 2 * H * dk], proj[:, 2 * H * dk: 2 * H * dk + H * dv]
+    start = torch.randn(3, H, dk, dv, generator=g) * 5
+    if what == "infinite v":
+        v[t, 3] = v[lens[0] + t, 7] = float("inf")
+    elif what == "nan k":
+        k[t, 5] = float("nan")
+    elif what == "infinite q":
+        q[t, 5] = float("inf")
+    elif what == "infinite state":
+        start[1, 0, 2, 3], start[1, 0, 4, 5] = float("inf"), float("-inf")
+    elif what == "nan state":
+        start[2, 0, 1, 1] = float("nan")
+    elif what == "product too large":  # q . k overflows, S = k v^T and S^T q do not
+        q[t], k[t], v[t] = 1e15, 1e25, 1e-30
+    else:
+        q[t], k[t], v[t] = 1e-20, 1e-20, 1e30
+    proj, start = proj.to(torch.bfloat16).to(CUDA), start.to(CUDA)
+    decay = torch.tensor([0.97, 0.5][:H], device=CUDA)
+    w = torch.ones(H * dv, device=CUDA)
+    states, outs = [], []
+    for chunked in (False, True):
+        S = start.clone()
+        outs.append(ops.lightning_attention(proj, 0, H * dk, 2 * H * dk, 2 * H * dk + H * dv, H, dk, dv, decay, w, 1e-5, S,
+                                            Batch(list(lens), [7, 9], [1, 2]), chunked=chunked))
+        states.append(S)
+    for (one, other), bound in ((states, 5e-6), (outs, 2.0 ** -7)):
+        finite = torch.isfinite(one)
+        assert torch.equal(torch.isnan(one), torch.isnan(other))
+        assert torch.equal(one[torch.isinf(one)], other[torch.isinf(one)]) and torch.equal(finite, torch.isfinite(other))
+        assert rel(torch.where(finite, other, 0.0), torch.where(finite, one, 0.0)) <= bound
+    assert bool(torch.isfinite(outs[1][:t]).all()) == (what != "infinite state")
+    ops.raise_on_error(CUDA)
+
+
+@pytest.mark.parametrize("H,dk,dv,tokens", [(2, 128, 32, 300), (1, 16, 16, 129), (1, 256, 32, 200), (1, 64, 48, 700)])
+def test_chunked_recurrence_against_64_bits(H, dk, dv, tokens):
+    """The carried state in 64 bits, from activations that round to the same bfloat16 whoever takes the exponential.
+    A chunk of L tokens rounds the float32 state once for its decay and once for each of L / 16 sums of products
+    (whose operands are exact to 24 bits): at most (1 + L / 16) 2^-24 a chunk, and what a chunk adds fades with the
+    decay like the rest of the state."""
+    g = torch.Generator().manual_seed(dk * tokens)
+    width = 2 * H * dk + 2 * H * dv
+    proj = (torch.randn(tokens, width, generator=g) * 1.5).to(torch.bfloat16).double()
+    act = proj * torch.sigmoid(proj)
+    firm = (act * (1 + 2.0 ** -14)).to(torch.bfloat16) == (act * (1 - 2.0 ** -14)).to(torch.bfloat16)
+    proj = torch.where(firm, proj, 0.0)
+    act = torch.where(firm, act, 0.0).to(torch.bfloat16).double()
+    decay = torch.tensor([0.999, 0.9][:H])
+    S = torch.randn(1, H, dk, dv, generator=g)
+    want = S[0].double().clone()
+    q, k = (act[:, i * H * dk: (i + 1) * H * dk].reshape(tokens, H, dk) for i in (0, 1))
+    v = act[:, 2 * H * dk: 2 * H * dk + H * dv].reshape(tokens, H, dv)
+    o = torch.empty(tokens, H, dv, dtype=torch.float64)
+    for t in range(tokens):
+        want = decay.double()[:, None, None] * want + k[t][:, :, None] * v[t][:, None, :]
+        o[t] = torch.einsum("hkv,hk->hv", want, q[t])
+    S = S.to(CUDA)
+    out = ops.lightning_attention(proj.to(torch.bfloat16).to(CUDA), 0, H * dk, 2 * H * dk, 2 * H * dk + H * dv, H, dk, dv,
+                                  decay.to(CUDA), torch.ones(H * dv, device=CUDA), 1e-5, S, Batch([tokens], [0], [0]), chunked=True)
+    chunk = 128 if dk <= 128 else 64
+    error = float((S[0].double().cpu() - want).norm() / want.norm())
+    assert error <= -(-tokens // chunk) * (1 + chunk // 16) * 2.0 ** -24, error
+    gate = torch.sigmoid(proj[:, 2 * H * dk + H * dv:])
+    flat = o.reshape(tokens, H * dv)
+    normed = flat * torch.rsqrt(flat.square().mean(-1, keepdim=True) + 1e-5) * gate
+    assert rel(out.double().cpu(), normed) <= 2.0 ** -7
+    ops.raise_on_error(CUDA)
+
+
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("rows", [3, 40, 400])
 def test_relu_gated_unit(dtype, rows):
