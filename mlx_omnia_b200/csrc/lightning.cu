@@ -20,8 +20,8 @@
 // spends most of its instructions there: what the loaders do per element decides the kernel's pace. A token's partial sums stay in registers until its run is done,
 // so the shuffles that add them up are off the chain from token to token, which is one fused
 // multiply-add a row. The state, the decay and every sum stay float32. It serves decode steps (one
-// token a request), float32, and portions too short or heads too odd for lightning_chunk.cu; the order of a
-// column's additions does not depend on how such portions were cut.
+// token a request, in a mixed step too), float32, and portions too short or heads too odd for lightning_chunk.cu; the order
+// of a column's additions does not depend on how such portions were cut.
 //
 // Compiled per key width: -DLIGHTNING_DK=<DK>.
 #include "common.cuh"
@@ -47,7 +47,8 @@ template <typename T, int P>
 __global__ void __launch_bounds__(LIGHTNING_THREADS) lightning_recurrence_kernel(
     const T* __restrict__ proj, int stride, int q_col, int k_col, int v_col, int H, int dv, int cols, int parts,
     int column_threads, const float* __restrict__ decay, float* __restrict__ S_state,
-    const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* __restrict__ o_raw) {
+    const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, const int* __restrict__ entries,
+    float* __restrict__ o_raw) {
   pdl_wait();
   pdl_launch_dependents();
   constexpr int DK = LIGHTNING_DK;
@@ -63,7 +64,8 @@ __global__ void __launch_bounds__(LIGHTNING_THREADS) lightning_recurrence_kernel
   constexpr bool EXACT = P * R == DK;       // every thread's R rows are rows of S: nothing to guard
   extern __shared__ __align__(16) float shared[];
   const int half = 2 * TC * VROW + TC * cols;  // floats of one buffer: q [TC][VROW] | k [TC][VROW] | v [TC][cols]
-  const int head = blockIdx.x / parts, part = blockIdx.x % parts, seq = blockIdx.y;
+  const int head = blockIdx.x / parts, part = blockIdx.x % parts;
+  const int seq = entries ? entries[blockIdx.y] : blockIdx.y;
   const int col0 = part * cols;
   const int begin = cu_seqlens[seq], end = cu_seqlens[seq + 1];
   if (end <= begin) return;
@@ -272,15 +274,16 @@ extern "C" int omnia_lightning_dk(void) { return LIGHTNING_DK; }
 // proj: the projected rows [tokens, stride] with q at q_col, k at k_col (heads * DK each) and v at
 // v_col (heads * dv); decay float32 [heads]; S_state float32 [slots, heads, DK, dv], updated in place;
 // o_raw float32 [tokens, heads * dv] receives the unnormed outputs. parts: runs of columns a head is
-// cut into (dv must divide into them; a run of at most 384 columns, 96 for four threads a column).
+// cut into (dv must divide into them; a run of at most 384 columns, 96 for four threads a column). entries: the `count`
+// requests whose tokens are walked (null: the first `count`, all of the step's).
 extern "C" int omnia_lightning_recurrence(const void* proj, int stride, int q_col, int k_col, int v_col, int H, int dv,
                                           int parts, const float* decay, float* S_state, const int* cu_seqlens,
-                                          const int* state_slots, int num_seqs, float* o_raw, int dtype,
-                                          cudaStream_t stream) {
-  if (num_seqs == 0) return 0;
+                                          const int* state_slots, const int* entries, int count, float* o_raw,
+                                          int dtype, cudaStream_t stream) {
+  if (count == 0) return 0;
   if (H < 1 || dv < 1 || parts < 1 || dv % parts != 0) return (int)cudaErrorInvalidValue;
   const int cols = dv / parts;
-  const dim3 grid(H * parts, num_seqs);
+  const dim3 grid(H * parts, count);
 #define OMNIA_LIGHTNING_LAUNCH(P)                                                                              \
   do {                                                                                                         \
     constexpr int R = (LIGHTNING_DK + P - 1) / P;                                                              \
@@ -292,7 +295,7 @@ extern "C" int omnia_lightning_recurrence(const void* proj, int stride, int q_co
     const int column_threads = (cols * P + 31) / 32 * 32;                                                      \
     launch_pdl(lightning_recurrence_kernel<T, P>, grid, dim3(column_threads + LIGHTNING_LOADERS), smem, stream, \
                (const T*)proj, stride, q_col, k_col, v_col, H, dv, cols, parts, column_threads, decay, S_state, \
-               cu_seqlens, state_slots, o_raw);                                                                \
+               cu_seqlens, state_slots, entries, o_raw);                                                               \
   } while (0)
   // Threads a column: as many as leave each at least four rows of S and fit the block. A column's
   // threads share out its rows, so more of them shorten what a token costs a warp; their partial sums

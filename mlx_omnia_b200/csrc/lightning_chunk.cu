@@ -96,13 +96,16 @@ __device__ __forceinline__ void split(float u, float v, uint32_t* part) {
   }
 }
 
-// q | k | v of the projected rows, silu in float32, rounded to bfloat16 as lightning.cu does: rows [tokens, 2 heads DK + heads dv].
+// q | k | v of the listed requests' projected rows, silu in float32, rounded to bfloat16 as lightning.cu does: rows [tokens,
+// 2 heads DK + heads dv].
 __global__ void lightning_act_kernel(const bf16* __restrict__ proj, int stride, int q_col, int k_col, int v_col, int qk, int width,
-                                     long long pieces, bf16* __restrict__ rows) {
+                                     const int* __restrict__ cu_seqlens, const int* __restrict__ entries, bf16* __restrict__ rows) {
   pdl_wait();
   pdl_launch_dependents();
-  const int across = width / 8;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < pieces; i += gridDim.x * (long long)blockDim.x) {
+  const int across = width / 8, seq = entries ? entries[blockIdx.y] : blockIdx.y;
+  const long long last = (long long)cu_seqlens[seq + 1] * across;
+  for (long long i = (long long)cu_seqlens[seq] * across + blockIdx.x * (long long)blockDim.x + threadIdx.x; i < last;
+       i += gridDim.x * (long long)blockDim.x) {
     const int c = (int)(i % across) * 8;
     const bf16* src = proj + (i / across) * stride + (c < qk ? q_col + c : c < 2 * qk ? k_col + c - qk : v_col + c - 2 * qk);
     uint4 piece;
@@ -124,7 +127,8 @@ __global__ void lightning_act_kernel(const bf16* __restrict__ proj, int stride, 
 
 __global__ void __launch_bounds__(THREADS, 1)
 lightning_chunk_kernel(const bf16* __restrict__ rows, int H, int dv, const float* __restrict__ decay, float* __restrict__ S_state,
-                       const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, float* __restrict__ o_raw) {
+                       const int* __restrict__ cu_seqlens, const int* __restrict__ state_slots, const int* __restrict__ entries,
+                       float* __restrict__ o_raw) {
   extern __shared__ __align__(16) unsigned char chunk_smem[];
   bf16* stage0 = reinterpret_cast<bf16*>(chunk_smem);  // two stages of [L][NROW] k, [L][NROW] q, [L][XROW] v
   constexpr int STAGE = L * (2 * NROW + XROW);
@@ -132,7 +136,7 @@ lightning_chunk_kernel(const bf16* __restrict__ rows, int H, int dv, const float
   bf16* Ws = Ss + 3 * N * XROW;   // [3][L][XROW] the weighted v in three parts
   float* power = reinterpret_cast<float*>(Ws + 3 * L * XROW);  // [L + 1] the decay's powers
 
-  const int parts = dv / COLS, head = blockIdx.x / parts, col0 = (blockIdx.x % parts) * COLS, seq = blockIdx.y;
+  const int parts = dv / COLS, head = blockIdx.x / parts, col0 = (blockIdx.x % parts) * COLS;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t4 = lane & 3, mat = lane >> 3, r8 = lane & 7;
   for (int i = tid; i <= L; i += THREADS) {
@@ -144,6 +148,7 @@ lightning_chunk_kernel(const bf16* __restrict__ rows, int H, int dv, const float
   }
   pdl_wait();
   pdl_launch_dependents();
+  const int seq = entries ? entries[blockIdx.y] : blockIdx.y;
   const int begin = cu_seqlens[seq], end = cu_seqlens[seq + 1];
   if (end <= begin) return;
   const int row_stride = 2 * H * N + H * dv;
@@ -417,13 +422,14 @@ lightning_chunk_kernel(const bf16* __restrict__ rows, int H, int dv, const float
 
 }  // namespace
 
-// As omnia_lightning_recurrence (lightning.cu) for bfloat16 rows; `rows` is room for [tokens, 2 H DK + H dv] bfloat16 on 16
-// bytes, dv a multiple of LIGHTNING_COLS.
-extern "C" int omnia_lightning_chunk(const void* proj, int stride, int q_col, int k_col, int v_col, int H, int dv, int tokens,
+// As omnia_lightning_recurrence (lightning.cu) for bfloat16 rows, of the `count` requests that `entries` lists (null: of the
+// first `count`), the longest of which brings `longest` tokens; `rows` is room for [the step's tokens, 2 H DK + H dv]
+// bfloat16 on 16 bytes, dv a multiple of LIGHTNING_COLS.
+extern "C" int omnia_lightning_chunk(const void* proj, int stride, int q_col, int k_col, int v_col, int H, int dv, int longest,
                                      void* rows, const float* decay, float* S_state, const int* cu_seqlens,
-                                     const int* state_slots, int num_seqs, float* o_raw, cudaStream_t stream) {
-  if (num_seqs == 0 || tokens == 0) return 0;
-  if (H < 1 || dv < COLS || dv % COLS || tokens < 0 || (((uintptr_t)rows | (uintptr_t)S_state | (uintptr_t)o_raw) & 15))
+                                     const int* state_slots, const int* entries, int count, float* o_raw, cudaStream_t stream) {
+  if (count == 0 || longest == 0) return 0;
+  if (H < 1 || dv < COLS || dv % COLS || count < 0 || longest < 0 || (((uintptr_t)rows | (uintptr_t)S_state | (uintptr_t)o_raw) & 15))
     return (int)cudaErrorInvalidValue;
   int device = 0;
   static bool configured[64] = {};
@@ -435,10 +441,10 @@ extern "C" int omnia_lightning_chunk(const void* proj, int stride, int q_col, in
     configured[device] = true;
   }
   const int width = 2 * H * N + H * dv;
-  const long long pieces = (long long)tokens * (width / 8), most = 8LL * omnia_sm_count();
-  launch_pdl(lightning_act_kernel, dim3((unsigned)((pieces + 255) / 256 < most ? (pieces + 255) / 256 : most)), dim3(256), 0, stream,
-             (const bf16*)proj, stride, q_col, k_col, v_col, H * N, width, pieces, (bf16*)rows);
-  launch_pdl(lightning_chunk_kernel, dim3(H * (dv / COLS), num_seqs), dim3(THREADS), smem_bytes(L), stream, (const bf16*)rows, H, dv,
-             decay, S_state, cu_seqlens, state_slots, o_raw);
+  const long long blocks = ((long long)longest * (width / 8) + 255) / 256, most = (8LL * omnia_sm_count() + count - 1) / count;
+  launch_pdl(lightning_act_kernel, dim3((unsigned)(blocks < most ? blocks : most), count), dim3(256), 0, stream, (const bf16*)proj,
+             stride, q_col, k_col, v_col, H * N, width, cu_seqlens, entries, (bf16*)rows);
+  launch_pdl(lightning_chunk_kernel, dim3(H * (dv / COLS), count), dim3(THREADS), smem_bytes(L), stream, (const bf16*)rows, H, dv,
+             decay, S_state, cu_seqlens, state_slots, entries, o_raw);
   return OMNIA_LAUNCH_RESULT();
 }

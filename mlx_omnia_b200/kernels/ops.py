@@ -1447,17 +1447,30 @@ def lightning_parts(requests: int, heads: int, dv: int, sms: int) -> int:
 
 
 LIGHTNING_CHUNK_TOKENS = 32
-"""From this many tokens of the longest entry on the chunked recurrence runs (where it applies): 16 heads of 128, 16 tokens
-9.1 us against 9.4 token by token, 32 tokens 8.8 against 13.2, 64: 8.6 against 19.9."""
+"""Requests that bring this many tokens run chunked (where that applies), the others token by token in a launch of their
+own: a block of the chunked kernel has an SM to itself, and which kernel a request takes does not depend on its
+neighbours. 16 heads of 128, one request: 16 tokens 9.1 us against 9.4 token by token, 32 tokens 8.8 against 13.2, 64:
+8.6 against 19.9."""
 
 
-def lightning_chunk_columns(requests: int, heads: int, dk: int, dv: int, dtype: torch.dtype, longest: int, sms: int) -> int:
-    """Value columns a block of the chunked recurrence takes, or 0 where that kernel does not apply (float32, widths its
-    tiles do not fit) or its chunks would be nearly empty: 32, or 16 where heads are no multiple of 32 wide or 32 would
-    leave half the SMs idle."""
-    if dtype != torch.bfloat16 or dk % 16 or dk > 256 or dv % 16 or longest < LIGHTNING_CHUNK_TOKENS:
+def lightning_chunk_columns(requests: int, heads: int, dk: int, dv: int, dtype: torch.dtype, sms: int) -> int:
+    """Value columns a block of the chunked recurrence of `requests` requests takes, or 0 where that kernel does not apply
+    (float32, widths its tiles do not fit): 32, or 16 where heads are no multiple of 32 wide or 32 would leave half the
+    SMs idle."""
+    if dtype != torch.bfloat16 or dk % 16 or dk > 256 or dv % 16:
         return 0
     return 16 if dv % 32 or 2 * requests * heads * (dv // 32) <= sms else 32
+
+
+def _lightning_requests(step: StepContext, long: bool, device: torch.device) -> tuple[torch.Tensor | None, int]:
+    """The requests that run chunked (`long`) or token by token: their indices (None: all of the step's) and how many."""
+    def build(step: StepContext) -> np.ndarray:
+        return np.asarray([s for s, n in enumerate(step.q_lens) if (n >= LIGHTNING_CHUNK_TOKENS) == long], dtype=np.int32)
+
+    count = sum((n >= LIGHTNING_CHUNK_TOKENS) == long for n in step.q_lens)
+    if count in (0, step.num_seqs):
+        return None, count
+    return _step_list(step, ("lightning_requests", long), build, device), count
 
 
 def lightning_attention(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, gate_col: int, heads: int, dk: int,
@@ -1468,33 +1481,39 @@ def lightning_attention(proj: torch.Tensor, q_col: int, k_col: int, v_col: int, 
     from q_col, k_col (heads * dk each) and v_col (heads * dv); per head S <- decay_h S + k v^T,
     o = S^T q; then one RMS norm over a token's heads side by side (weight [heads * dv], `eps`) and the
     gate sigmoid(columns from gate_col). The recurrence runs token by token, a head's columns cut into `parts` runs,
-    or (`chunked` None: where it pays, unless parts are named) in chunks on the tensor cores with the same operands
-    and float32 sums. -> [tokens, heads * dv]"""
+    or (`chunked` None: for the requests it pays for, unless parts are named; True: for all) in chunks on the tensor cores
+    with the same operands and float32 sums. -> [tokens, heads * dv]"""
     tokens, stride = proj.shape
     width = heads * dv
+    sms = sm_count(proj.device)
     o_raw = torch.empty(tokens, width, dtype=torch.float32, device=proj.device)
     out = torch.empty(tokens, width, dtype=proj.dtype, device=proj.device)
-    cols = 0
-    if chunked or (chunked is None and parts is None):
-        longest = LIGHTNING_CHUNK_TOKENS if chunked else step.max_q_len
-        cols = lightning_chunk_columns(step.num_seqs, heads, dk, dv, proj.dtype, longest, sm_count(proj.device))
-        if chunked and not cols:
+    entries = long_entries = None
+    count, long_count, longest = step.num_seqs, 0, step.max_q_len
+    if chunked:
+        count, long_count = 0, count
+    elif chunked is None and parts is None and longest >= LIGHTNING_CHUNK_TOKENS and \
+            lightning_chunk_columns(1, heads, dk, dv, proj.dtype, sms):
+        (entries, count), (long_entries, long_count) = (_lightning_requests(step, long, proj.device) for long in (False, True))
+    if long_count:
+        cols = lightning_chunk_columns(long_count, heads, dk, dv, proj.dtype, sms)
+        if not cols:
             raise KernelError(f"the chunked recurrence does not take keys of {dk} and values of {dv} in {proj.dtype}")
-    if cols:
         rows = torch.empty(tokens, 2 * heads * dk + width, dtype=proj.dtype, device=proj.device)
         fn = _function("lightning_chunk", "omnia_lightning_chunk",
                        [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
-                        c_int, c_void_p, c_void_p], {"LIGHTNING_DK": dk, "LIGHTNING_COLS": cols})
-        _check(fn(_ptr(proj), stride, q_col, k_col, v_col, heads, dv, tokens, _ptr(rows), _ptr(decay), _ptr(S),
-                  _ptr(step.cu_seqlens), _ptr(step.state_slots), step.num_seqs, _ptr(o_raw), _stream()), "lightning_chunk")
-    else:
+                        c_void_p, c_int, c_void_p, c_void_p], {"LIGHTNING_DK": dk, "LIGHTNING_COLS": cols})
+        _check(fn(_ptr(proj), stride, q_col, k_col, v_col, heads, dv, longest, _ptr(rows), _ptr(decay), _ptr(S),
+                  _ptr(step.cu_seqlens), _ptr(step.state_slots), _ptr(long_entries), long_count, _ptr(o_raw), _stream()),
+               "lightning_chunk")
+    if count:
         if parts is None:
-            parts = lightning_parts(step.num_seqs, heads, dv, sm_count(proj.device))
+            parts = lightning_parts(count, heads, dv, sms)
         fn = _function("lightning", "omnia_lightning_recurrence",
                        [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p, c_void_p,
-                        c_int, c_void_p, c_int, c_void_p], {"LIGHTNING_DK": dk})
+                        c_void_p, c_int, c_void_p, c_int, c_void_p], {"LIGHTNING_DK": dk})
         _check(fn(_ptr(proj), stride, q_col, k_col, v_col, heads, dv, parts, _ptr(decay), _ptr(S), _ptr(step.cu_seqlens),
-                  _ptr(step.state_slots), step.num_seqs, _ptr(o_raw), _code(proj.dtype), _stream()), "lightning_recurrence")
+                  _ptr(step.state_slots), _ptr(entries), count, _ptr(o_raw), _code(proj.dtype), _stream()), "lightning_recurrence")
     fn = _function("lightning", "omnia_lightning_out",
                    [c_void_p, c_void_p, c_int, c_void_p, c_float, c_int, c_int, c_void_p, c_int, c_void_p],
                    {"LIGHTNING_DK": dk})

@@ -313,6 +313,34 @@ def test_decayed_state_in_chunks(H, dk, dv, lens):
     ops.raise_on_error(CUDA)
 
 
+@pytest.mark.parametrize("H,dk,dv", [(3, 128, 128), (2, 16, 16), (2, 5, 16)])
+@pytest.mark.parametrize("order", [1, -1])
+def test_short_and_long_requests_of_one_step_keep_their_own_kernels(H, dk, dv, order):
+    """A step of single tokens, short and long portions: every request's rows and state are, bit for bit, what a step
+    of its own kind alone gives (the same number of columns a block, so the same order of additions)."""
+    g = torch.Generator().manual_seed(dk)
+    lens = [1, 31, 32, 1, 200, 5, 130][::order]
+    width = 2 * H * dk + 2 * H * dv
+    proj = (torch.randn(sum(lens), width, generator=g) * 1.5).to(torch.bfloat16).to(CUDA)
+    start = torch.randn(len(lens), H, dk, dv, generator=g).to(CUDA)
+    decay, w = torch.tensor([0.97, 0.5, 0.999][:H], device=CUDA), (1 + 0.2 * torch.randn(H * dv, generator=g)).to(CUDA)
+
+    def run(keep):
+        S, at = start.clone(), [sum(lens[:s]) for s in keep]
+        rows = torch.cat([proj[a: a + lens[s]] for a, s in zip(at, keep)])
+        out = ops.lightning_attention(rows, 0, H * dk, 2 * H * dk, 2 * H * dk + H * dv, H, dk, dv, decay, w, 1e-5, S,
+                                      Batch([lens[s] for s in keep], None, list(keep)))
+        return out.split([lens[s] for s in keep]), S
+
+    outs, S = run(range(len(lens)))
+    kinds = [list(range(len(lens)))] if dk % 16 else [[s for s, n in enumerate(lens) if (n >= 32) == long] for long in (False, True)]
+    for keep in kinds:
+        alone, S_alone = run(keep)
+        for s, out in zip(keep, alone):
+            assert torch.equal(out, outs[s]) and torch.equal(S[s], S_alone[s]), lens[s]
+    ops.raise_on_error(CUDA)
+
+
 @pytest.mark.parametrize("H,dk,dv", [(2, 128, 64), (1, 16, 48), (1, 256, 32), (2, 48, 32)])
 @pytest.mark.parametrize("what", ["infinite v", "nan k", "infinite q", "infinite state", "nan state", "product too large", "v too small"])
 def test_what_is_not_finite_in_a_chunk_stays_where_it_belongs(H, dk, dv, what):

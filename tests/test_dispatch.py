@@ -285,3 +285,28 @@ def test_experts_on_the_tensor_cores_take_bfloat16_only(monkeypatch, rows):
     assert experts(torch.bfloat16).shape == (rows, 16)
     with pytest.raises(ops.KernelError, match="bfloat16"):
         experts(torch.float32)
+
+
+@pytest.mark.parametrize("q_lens,short,long", [([1] * 31 + [32], list(range(31)), [31]), ([64, 1, 31, 40], [1, 2], [0, 3]),
+                                               ([32, 100], None, "all"), ([1, 5, 31], "all", None), ([0, 32, 1], [0, 2], [1])])
+def test_chunked_recurrence_takes_the_requests_that_bring_a_chunk(monkeypatch, q_lens, short, long):
+    """Single tokens and short portions stay with the token kernel whoever shares their step."""
+    calls = {}
+    monkeypatch.setattr(ops, "_function", lambda library, name, argtypes, defines=None:
+                        lambda *args: calls.update({name: args}) or 0)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    lists = {}
+    monkeypatch.setattr(ops, "_ints_to_device", lambda values, device: lists.setdefault(len(lists), torch.from_numpy(values)))
+    step = SimpleNamespace(num_seqs=len(q_lens), q_lens=q_lens, max_q_len=max(q_lens), workspace=None,
+                           cu_seqlens=torch.zeros(9), state_slots=torch.zeros(9))
+    ops.lightning_attention(torch.zeros(sum(q_lens), 320, dtype=torch.bfloat16), 0, 64, 128, 192, 4, 16, 16, torch.ones(4),
+                            torch.ones(64), 1e-5, torch.zeros(4, 4, 16, 16), step)
+    held = {t.data_ptr(): t.tolist() for t in lists.values()}
+    for name, at, want in (("omnia_lightning_recurrence", 12, short), ("omnia_lightning_chunk", 13, long)):
+        if want is None:
+            assert name not in calls
+            continue
+        entries, count = calls[name][at: at + 2]
+        assert count == (len(q_lens) if want == "all" else len(want))
+        assert entries is None if want == "all" else held[entries] == want
