@@ -16,7 +16,8 @@
 
 #define SAMPLE_THREADS 512
 #define SAMPLE_CLUSTER 8
-#define SAMPLE_LIST 4096  // entries of a block's list of what can still be chosen
+#define SAMPLE_LIST 4096  // entries of a block's list of what can still be chosen, where shared memory has room for them
+#define SAMPLE_SENT 128   // candidates that a block sends to block 0 at most
 
 __device__ __forceinline__ unsigned int order_key(float v) {
   // Monotone map float -> uint: larger float, larger key.
@@ -85,11 +86,36 @@ __device__ ArgMax block_argmax(ArgMax a, ArgMax* scratch) {
 // and every block walks the sum from the top to the bin that holds the threshold. Counts are
 // integers and probability mass is added in fixed point (2^-40), so the sums do not depend on
 // their order and a seeded run repeats bit for bit.
+struct SampleHistogram {
+  unsigned int count[256];
+  unsigned int limb[3][256];  // the mass in three limbs
+};
+// What the whole row's draw comes down to once the top_k bound of the cluster has left few candidates:
+// each block sends its own to block 0, which finishes alone, a candidate a thread.
+struct SampleSent {
+  float s[SAMPLE_CLUSTER][SAMPLE_SENT];
+  int i[SAMPLE_CLUSTER][SAMPLE_SENT];
+};
+struct SampleFew {  // of each candidate, to be compared with every other
+  unsigned int key[SAMPLE_THREADS];
+  unsigned long long mass[SAMPLE_THREADS];
+};
+struct SampleGroups {
+  unsigned int largest[SAMPLE_THREADS / 2];   // of each group
+  unsigned int above[2][SAMPLE_THREADS / 2];  // how many groups of each half are larger
+};
 struct SampleShared {
-  unsigned int count[256];           // this block's histogram of the pass
-  unsigned int limb[3][256];         // its mass in three limbs of 16 bits (32-bit atomics; at most 2^15 additions)
-  unsigned int total_count[2][256];  // the cluster's, of alternate passes: every block adds into every block's
-  unsigned int total_limb[2][3][256];  // the cluster's mass in three limbs of 20 bits (32-bit remote atomics)
+  SampleHistogram even;  // the cluster's, of the first pass and every other: every block adds into every block's
+                         // (limbs of 20 bits: 32-bit remote atomics)
+  union {                // one after the other, and the histograms last: 16 KB here cost a block its place on an SM
+    struct {
+      SampleHistogram own;  // this block's histogram of the pass (limbs of 16 bits: 32-bit atomics, at most 2^15 additions)
+      SampleHistogram odd;  // the cluster's, of the passes in between
+    };
+    SampleGroups groups;
+    SampleSent sent;  // (block 0's, written by all)
+    SampleFew few;
+  };
   ArgMax first_best, draw_best;      // this block's candidates, read by the whole cluster
   ArgMax ascratch[33];
   unsigned int digit;                // the bin a pass settled on
@@ -97,8 +123,10 @@ struct SampleShared {
   unsigned long long mass;           // this block's whole mass; where block 0 finishes alone, the kept mass
   unsigned int bound;                // this block's bound on the keys that top_k can keep
   unsigned int listed;               // elements listed or sent
-  unsigned int sent[SAMPLE_CLUSTER]; // how many each block sent
+  unsigned int sent_count[SAMPLE_CLUSTER];  // how many each block sent
+  __device__ SampleHistogram& total(int buf) { return buf ? odd : even; }
 };
+static_assert(sizeof(SampleSent) <= 2 * sizeof(SampleHistogram) && sizeof(SampleFew) <= 2 * sizeof(SampleHistogram), "sizes");
 
 __device__ __forceinline__ unsigned long long fixed_mass(float e) { return __float2ull_rn(e * 1099511627776.f); }
 
@@ -118,21 +146,22 @@ template <bool MASS, typename Item>
 __device__ __forceinline__ void histogram_pass(SampleShared& sh, int buf, int n, unsigned int prefix, int shift,
                                                Item item) {
   for (int b = threadIdx.x; b < 256; b += blockDim.x) {
-    sh.count[b] = 0u;
-    sh.limb[0][b] = sh.limb[1][b] = sh.limb[2][b] = 0u;
-    sh.total_count[buf ^ 1][b] = 0u;  // the next pass's totals: nobody adds to them before this pass's barrier
-    sh.total_limb[buf ^ 1][0][b] = sh.total_limb[buf ^ 1][1][b] = sh.total_limb[buf ^ 1][2][b] = 0u;
+    SampleHistogram& next = sh.total(buf ^ 1);
+    sh.own.count[b] = 0u;
+    sh.own.limb[0][b] = sh.own.limb[1][b] = sh.own.limb[2][b] = 0u;
+    next.count[b] = 0u;  // the next pass's totals: nobody adds to them before this pass's barrier
+    next.limb[0][b] = next.limb[1][b] = next.limb[2][b] = 0u;
   }
   __syncthreads();
   unsigned int held = 256u, held_count = 0u;  // 256: nothing held yet
   unsigned long long held_mass = 0ull;
   // A lane's mass is below 2^47 (fewer than 2^6 elements of less than 2^41 each).
   auto flush = [&](unsigned int bin, unsigned int count, unsigned long long mass) {
-    atomicAdd(&sh.count[bin], count);
+    atomicAdd(&sh.own.count[bin], count);
     if (MASS) {
-      atomicAdd(&sh.limb[0][bin], (unsigned int)(mass & 0xFFFFu));
-      atomicAdd(&sh.limb[1][bin], (unsigned int)((mass >> 16) & 0xFFFFu));
-      atomicAdd(&sh.limb[2][bin], (unsigned int)(mass >> 32));
+      atomicAdd(&sh.own.limb[0][bin], (unsigned int)(mass & 0xFFFFu));
+      atomicAdd(&sh.own.limb[1][bin], (unsigned int)((mass >> 16) & 0xFFFFu));
+      atomicAdd(&sh.own.limb[2][bin], (unsigned int)(mass >> 32));
     }
   };
   for (int j = threadIdx.x; j < n; j += blockDim.x) {
@@ -165,11 +194,11 @@ __device__ __forceinline__ void histogram_pass(SampleShared& sh, int buf, int n,
       mass = (unsigned long long)p0 + ((unsigned long long)p1 << 16) + ((unsigned long long)p2 << 32);
     }
     if ((threadIdx.x & 31) == 0) {
-      atomicAdd(&sh.count[reference], count);
+      atomicAdd(&sh.own.count[reference], count);
       if (MASS) {  // a warp's mass is below 2^52: the top limb takes what is above 32 bits
-        atomicAdd(&sh.limb[0][reference], (unsigned int)(mass & 0xFFFFu));
-        atomicAdd(&sh.limb[1][reference], (unsigned int)((mass >> 16) & 0xFFFFu));
-        atomicAdd(&sh.limb[2][reference], (unsigned int)(mass >> 32));
+        atomicAdd(&sh.own.limb[0][reference], (unsigned int)(mass & 0xFFFFu));
+        atomicAdd(&sh.own.limb[1][reference], (unsigned int)((mass >> 16) & 0xFFFFu));
+        atomicAdd(&sh.own.limb[2][reference], (unsigned int)(mass >> 32));
       }
     }
   } else if (held_count) {
@@ -184,18 +213,18 @@ __device__ __forceinline__ void cluster_totals(cooperative_groups::cluster_group
                                                bool mass) {
   __syncthreads();
   for (int b = threadIdx.x; b < 256; b += blockDim.x) {
-    const unsigned int c = sh.count[b];
+    const unsigned int c = sh.own.count[b];
     if (c == 0u) continue;
-    const unsigned long long m = (unsigned long long)sh.limb[0][b] + ((unsigned long long)sh.limb[1][b] << 16) +
-                                 ((unsigned long long)sh.limb[2][b] << 32);
+    const unsigned long long m = (unsigned long long)sh.own.limb[0][b] + ((unsigned long long)sh.own.limb[1][b] << 16) +
+                                 ((unsigned long long)sh.own.limb[2][b] << 32);
 #pragma unroll
     for (unsigned int r = 0; r < SAMPLE_CLUSTER; ++r) {
-      SampleShared* other = cluster.map_shared_rank(&sh, r);
-      atomicAdd(&other->total_count[buf][b], c);
+      SampleHistogram& other = cluster.map_shared_rank(&sh, r)->total(buf);
+      atomicAdd(&other.count[b], c);
       if (mass && m) {  // a block's mass of a bin is below 2^58; eight blocks' limbs stay below 2^23
-        atomicAdd(&other->total_limb[buf][0][b], (unsigned int)(m & 0xFFFFFu));
-        atomicAdd(&other->total_limb[buf][1][b], (unsigned int)((m >> 20) & 0xFFFFFu));
-        atomicAdd(&other->total_limb[buf][2][b], (unsigned int)(m >> 40));
+        atomicAdd(&other.limb[0][b], (unsigned int)(m & 0xFFFFFu));
+        atomicAdd(&other.limb[1][b], (unsigned int)((m >> 20) & 0xFFFFFu));
+        atomicAdd(&other.limb[2][b], (unsigned int)(m >> 40));
       }
     }
   }
@@ -207,14 +236,15 @@ __device__ __forceinline__ void cluster_totals(cooperative_groups::cluster_group
 // it. Leaves the bin and what lies above it in shared memory.
 __device__ __forceinline__ void select_bin(SampleShared& sh, int buf, bool by_mass, unsigned long long limit) {
   const int lane = threadIdx.x;
+  const SampleHistogram& all = sh.total(buf);
   unsigned long long w[8], sum = 0ull;
   unsigned int c[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int b = 255 - 8 * lane - i;
-    c[i] = sh.total_count[buf][b];
-    w[i] = by_mass ? (unsigned long long)sh.total_limb[buf][0][b] + ((unsigned long long)sh.total_limb[buf][1][b] << 20) +
-                         ((unsigned long long)sh.total_limb[buf][2][b] << 40)
+    c[i] = all.count[b];
+    w[i] = by_mass ? (unsigned long long)all.limb[0][b] + ((unsigned long long)all.limb[1][b] << 20) +
+                         ((unsigned long long)all.limb[2][b] << 40)
                    : (unsigned long long)c[i];
     sum += w[i];
   }
@@ -244,26 +274,6 @@ __device__ __forceinline__ void select_bin(SampleShared& sh, int buf, bool by_ma
   }
 }
 
-// What the whole row's draw comes down to once the top_k bound of the cluster has left few candidates:
-// each block sends its own to block 0, which finishes alone, a candidate a thread.
-#define SAMPLE_SENT 128
-struct SampleSent {
-  float s[SAMPLE_CLUSTER][SAMPLE_SENT];
-  int i[SAMPLE_CLUSTER][SAMPLE_SENT];
-};
-struct SampleFew {  // of each candidate, to be compared with every other
-  unsigned int key[SAMPLE_THREADS];
-  unsigned long long mass[SAMPLE_THREADS];
-};
-union SampleWork {  // used one after the other
-  struct {
-    unsigned int largest[SAMPLE_THREADS / 2];   // of each group
-    unsigned int above[2][SAMPLE_THREADS / 2];  // how many groups of each half are larger
-  } groups;
-  SampleFew few;
-  unsigned short list[SAMPLE_LIST];
-};
-
 // Bounds: the logits are read once (0.6 MB a row); what costs time is everything that walks the row again, and
 // shared-memory atomics on the few bins that most of a row's logits share. So what cannot be chosen is cut away
 // first, by bounds that hold whatever the values:
@@ -277,7 +287,7 @@ union SampleWork {  // used one after the other
 // over all logits stands. 64 rows of 151,936 logits, top_k 50, top_p 0.95: 146 us with the selection over all logits,
 // 44 so (a cluster of eight blocks a row is 512 blocks, two to an SM: 1.7 rounds of them).
 __global__ void __cluster_dims__(SAMPLE_CLUSTER, 1, 1) __launch_bounds__(SAMPLE_THREADS, 2)
-sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice, int cached,
+sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice, int cached, unsigned int list_most,
               const float* __restrict__ temperature, const int* __restrict__ top_k,
               const float* __restrict__ top_p, const float* __restrict__ min_p,
               const float* __restrict__ penalty, const int* __restrict__ history, int history_len,
@@ -292,10 +302,7 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
   const int row = blockIdx.x / SAMPLE_CLUSTER, rank = (int)cluster.block_rank();
   float* z = logits + (size_t)row * stride;
   const int begin = min(vocab, rank * slice), n = min(vocab, begin + slice) - begin;
-  // Behind the slice: the candidates sent to block 0 by the whole cluster, then this block's own working space.
-  SampleSent& sent = *reinterpret_cast<SampleSent*>(sv + (cached ? slice : 0));
-  SampleWork& work = *reinterpret_cast<SampleWork*>(&sent + 1);
-  unsigned short* list = work.list;
+  unsigned short* list = reinterpret_cast<unsigned short*>(sv + (cached ? slice : 0));  // [list_most], behind the slice
 
   // Repetition penalty: once per distinct recent id, on the raw logit, by the block whose slice holds it.
   const float pen = penalty ? penalty[row] : 1.f;
@@ -349,21 +356,21 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
   const bool bounded = ranked && m <= SAMPLE_THREADS / 2;
   if (bounded) {
     top = max(top, __shfl_xor_sync(0xffffffffu, top, 1));
-    if (!(threadIdx.x & 1)) work.groups.largest[threadIdx.x >> 1] = top;
+    if (!(threadIdx.x & 1)) sh.groups.largest[threadIdx.x >> 1] = top;
     if (threadIdx.x == 0) sh.bound = 0xffffffffu;
     __syncthreads();
     constexpr int GROUPS = SAMPLE_THREADS / 2;
     const int g = threadIdx.x % GROUPS, half = threadIdx.x / GROUPS;
-    const unsigned int mine = work.groups.largest[g];
+    const unsigned int mine = sh.groups.largest[g];
     unsigned int larger = 0u;
 #pragma unroll 8
     for (int q = 0; q < GROUPS / 8; ++q) {
-      const uint4 o = reinterpret_cast<const uint4*>(work.groups.largest)[half * (GROUPS / 8) + q];
+      const uint4 o = reinterpret_cast<const uint4*>(sh.groups.largest)[half * (GROUPS / 8) + q];
       larger += (o.x > mine) + (o.y > mine) + (o.z > mine) + (o.w > mine);
     }
-    work.groups.above[half][g] = larger;
+    sh.groups.above[half][g] = larger;
     __syncthreads();
-    const unsigned int all = work.groups.above[0][g] + work.groups.above[1][g];
+    const unsigned int all = sh.groups.above[0][g] + sh.groups.above[1][g];
     const unsigned int low = __reduce_min_sync(0xffffffffu, all < (unsigned int)m ? mine : 0xffffffffu);
     if ((threadIdx.x & 31) == 0) atomicMin(&sh.bound, low);
   }
@@ -372,8 +379,8 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
     sh.listed = 0u;
   }
   for (int b = threadIdx.x; b < 256; b += blockDim.x) {  // the first pass's totals start at zero
-    sh.total_count[0][b] = 0u;
-    sh.total_limb[0][0][b] = sh.total_limb[0][1][b] = sh.total_limb[0][2][b] = 0u;
+    sh.even.count[b] = 0u;
+    sh.even.limb[0][b] = sh.even.limb[1][b] = sh.even.limb[2][b] = 0u;
   }
   cluster.sync();
   unsigned int bound = bounded ? 0xffffffffu : 0u;  // keys below it are not among the k largest
@@ -405,7 +412,7 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
 
   if (bounded && isfinite(smax)) {
     // What reaches the bound goes to block 0.
-    SampleSent* at0 = cluster.map_shared_rank(&sent, 0);
+    SampleSent* at0 = &cluster.map_shared_rank(&sh, 0)->sent;
     for (int j = threadIdx.x; j < n; j += SAMPLE_THREADS) {
       const float s = s_of(j);
       if (order_key(s) < bound) continue;
@@ -416,13 +423,13 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
       }
     }
     __syncthreads();
-    if (threadIdx.x < SAMPLE_CLUSTER) cluster.map_shared_rank(&sh, threadIdx.x)->sent[rank] = sh.listed;
+    if (threadIdx.x < SAMPLE_CLUSTER) cluster.map_shared_rank(&sh, threadIdx.x)->sent_count[rank] = sh.listed;
     cluster.sync();
     int total = 0, from = 0, before = 0;  // candidates, and where this thread's is: which block's, how many ahead of that
     bool fits = true;
 #pragma unroll
     for (int r = 0; r < SAMPLE_CLUSTER; ++r) {
-      const int c = (int)sh.sent[r];
+      const int c = (int)sh.sent_count[r];
       fits = fits && c <= SAMPLE_SENT;
       if ((int)threadIdx.x >= total) from = r, before = total;
       total += c;
@@ -431,29 +438,30 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
       if (rank != 0) return;  // (every access to another block's memory lies before the barrier above)
       const int i = threadIdx.x;
       const bool mine = i < total;
-      const float s = mine ? sent.s[from][i - before] : 0.f;
-      const int id = mine ? sent.i[from][i - before] : 0;
+      const float s = mine ? sh.sent.s[from][i - before] : 0.f;
+      const int id = mine ? sh.sent.i[from][i - before] : 0;
       const unsigned int key = order_key(s);
-      if (mine) work.few.key[i] = key;
+      __syncthreads();  // what was sent has been read; its place is used for the keys
+      if (mine) sh.few.key[i] = key;
       if (i == 0) sh.mass = 0ull;
       __syncthreads();
       int larger = 0;
-      for (int o = 0; o < total; ++o) larger += work.few.key[o] > key;
+      for (int o = 0; o < total; ++o) larger += sh.few.key[o] > key;
       bool kept = mine && larger < k;  // a tie at the k-th largest is kept whole
       const float e = expf(s - smax);
       if (p < 1.f) {
         const unsigned long long mass = kept ? fixed_mass(e) : 0ull;
         __syncthreads();  // the keys of s have been read
         if (mine) {
-          work.few.key[i] = kept ? __float_as_uint(e) : 0u;  // e >= 0: its bits order it
-          work.few.mass[i] = mass;
+          sh.few.key[i] = kept ? __float_as_uint(e) : 0u;  // e >= 0: its bits order it
+          sh.few.mass[i] = mass;
         }
         if (mass) atomicAdd(&sh.mass, mass);
         __syncthreads();
         const unsigned long long limit = mass_limit(p, sh.mass);
         if (kept && limit != 0ull) {
           unsigned long long greater = 0ull;
-          for (int o = 0; o < total; ++o) greater += work.few.key[o] > __float_as_uint(e) ? work.few.mass[o] : 0ull;
+          for (int o = 0; o < total; ++o) greater += sh.few.key[o] > __float_as_uint(e) ? sh.few.mass[o] : 0ull;
           kept = greater < limit;
         }
       }
@@ -534,10 +542,10 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
           unsigned int at = 0u;
           if ((threadIdx.x & 31) == 0) at = atomicAdd(&sh.listed, (unsigned int)__popc(who));
           at = __shfl_sync(0xffffffffu, at, 0) + (unsigned int)__popc(who & ((1u << (threadIdx.x & 31)) - 1u));
-          if (in && at < SAMPLE_LIST) list[at] = (unsigned short)j;
+          if (in && at < list_most) list[at] = (unsigned short)j;
         }
         __syncthreads();
-        if (sh.listed <= SAMPLE_LIST) listed = (int)sh.listed;
+        if (sh.listed <= list_most) listed = (int)sh.listed;
       }
       __syncthreads();
     }
@@ -626,7 +634,19 @@ extern "C" int omnia_sample(float* logits, long long stride, int rows, int vocab
   // A slice starts on 16 bytes wherever its row does.
   const int slice = ((vocab + SAMPLE_CLUSTER - 1) / SAMPLE_CLUSTER + 3) & ~3;
   const int cached = slice <= 49152 ? 1 : 0;
-  const size_t smem = (cached ? (size_t)slice * sizeof(float) : 0) + sizeof(SampleSent) + sizeof(SampleWork);
+  const size_t held = cached ? (size_t)slice * sizeof(float) : 0;
+  // The list takes what is left of half an SM: with 64 rows of 201,088 logits a block without its neighbour on the SM
+  // took half as long again (temperature alone 147 us against 115).
+  static size_t half = 0;
+  if (half == 0) {
+    cudaFuncAttributes attributes;
+    const cudaError_t e = cudaFuncGetAttributes(&attributes, sample_kernel);
+    if (e != cudaSuccess) return (int)e;
+    half = (114 - 1) * 1024 - ((attributes.sharedSizeBytes + 127) & ~(size_t)127);  // a block's own KB, and what it holds anyway
+  }
+  size_t room = SAMPLE_LIST * sizeof(unsigned short);
+  if (held <= half && held + room > half) room = (half - held) & ~(size_t)127;
+  const size_t smem = held + room;
   static size_t configured = 0;
   if (smem > configured) {
     cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -634,6 +654,6 @@ extern "C" int omnia_sample(float* logits, long long stride, int rows, int vocab
     configured = smem;
   }
   launch_pdl(sample_kernel, rows * SAMPLE_CLUSTER, SAMPLE_THREADS, smem, stream, logits, stride, vocab, slice, cached,
-             temperature, top_k, top_p, min_p, penalty, history, history_len, seeds, draws, out);
+             (unsigned int)(room / sizeof(unsigned short)), temperature, top_k, top_p, min_p, penalty, history, history_len, seeds, draws, out);
   return OMNIA_LAUNCH_RESULT();
 }

@@ -619,6 +619,25 @@ def test_sampling_by_every_route(ops, vocab, levels):
     assert ops.sample(strided, *args).tolist() == got.tolist()
 
 
+@pytest.mark.parametrize("vocab", [201088, 206144, 393216, 393220])
+def test_sampling_where_shared_memory_is_short(ops, vocab):
+    """Rows whose slices leave the list of candidates part of its room, none of it, all of it in a block that has an SM
+    to itself (the largest row kept in shared memory), and rows that are read from memory every time."""
+    cases = [(50, 0.95), (400, 1.0), (700, 0.9), (2048, 1.0), (0, 0.9), (0, 0.3)]
+    rows = len(cases)
+    logits = rand(rows, vocab, scale=4.0, seed=vocab)
+    logits[-1, 5:] -= 40.0  # next to nothing left but five
+    dev = lambda v, dt: torch.tensor(v, dtype=dt, device="cuda")
+    args = (dev([0.9] * rows, torch.float32), dev([k for k, _ in cases], torch.int32), dev([p for _, p in cases], torch.float32),
+            dev([0.0, 0.02] * (rows // 2), torch.float32), dev(list(range(rows)), torch.int64), dev([5] * rows, torch.int64))
+    assert ops.sample(logits.clone(), *args).tolist() == kernel_refs.sample(logits, *args).tolist()
+    # A flat row inside a wide one whose other logits weigh nothing: one block has nearly all that can be chosen.
+    flat = rand(rows, 20011, scale=0.5, seed=3)
+    wide = torch.full((rows, vocab), -1e4, device="cuda")
+    wide[:, : flat.shape[1]] = flat
+    assert ops.sample(wide, *args).tolist() == ops.sample(flat, *args).tolist()
+
+
 def test_sampling_keeps_exactly_the_filtered_set(ops):
     """Many draws never leave the set that top_k/top_p/min_p keep, and reach all of it."""
     vocab = 300
