@@ -120,9 +120,11 @@ struct SampleShared {
   ArgMax ascratch[33];
   unsigned int digit;                // the bin a pass settled on
   unsigned long long above;          // count or mass of the bins above it
-  unsigned long long mass;           // this block's whole mass; where block 0 finishes alone, the kept mass
+  unsigned long long limit;          // what the count or mass above an element must stay below
+  unsigned long long mass;           // where block 0 finishes alone, the kept mass
   unsigned int bound;                // this block's bound on the keys that top_k can keep
   unsigned int listed;               // elements listed or sent
+  unsigned int here;                 // this block's elements in the bin a pass settled on or above it
   unsigned int sent_count[SAMPLE_CLUSTER];  // how many each block sent
   __device__ SampleHistogram& total(int buf) { return buf ? odd : even; }
 };
@@ -233,8 +235,10 @@ __device__ __forceinline__ void cluster_totals(cooperative_groups::cluster_group
 
 // Warp 0 walks the cluster's histogram from the top, lane l taking bins 255 - 8 l down to 248 - 8 l:
 // the lowest bin that holds an element with less than `limit` (counts, or mass) in the bins above
-// it. Leaves the bin and what lies above it in shared memory.
-__device__ __forceinline__ void select_bin(SampleShared& sh, int buf, bool by_mass, unsigned long long limit) {
+// it. With `fraction` >= 0 the limit is first set to that fraction of the histogram's whole mass. Leaves the bin, what lies
+// above it, the limit, and how many of this block's own elements were counted in that bin or above it in shared memory.
+__device__ __forceinline__ void select_bin(SampleShared& sh, int buf, bool by_mass, unsigned long long limit,
+                                           float fraction) {
   const int lane = threadIdx.x;
   const SampleHistogram& all = sh.total(buf);
   unsigned long long w[8], sum = 0ull;
@@ -254,6 +258,7 @@ __device__ __forceinline__ void select_bin(SampleShared& sh, int buf, bool by_ma
     const unsigned long long up = __shfl_up_sync(0xffffffffu, inclusive, o);
     if (lane >= o) inclusive += up;
   }
+  if (fraction >= 0.f) limit = mass_limit(fraction, __shfl_sync(0xffffffffu, inclusive, 31));
   unsigned long long above = inclusive - sum, chosen_above = 0ull;
   int chosen = -1;
 #pragma unroll
@@ -268,9 +273,17 @@ __device__ __forceinline__ void select_bin(SampleShared& sh, int buf, bool by_ma
   const int from = has ? 31 - __clz(has) : 0;  // the lane with the lowest such bin
   chosen = __shfl_sync(0xffffffffu, chosen, from);
   chosen_above = __shfl_sync(0xffffffffu, chosen_above, from);
+  if (!has) chosen = 0;
+  unsigned int here = 0u;
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+    if (255 - 8 * lane - i >= chosen) here += sh.own.count[255 - 8 * lane - i];
+  here = __reduce_add_sync(0xffffffffu, here);
   if (lane == 0) {
-    sh.digit = has ? (unsigned int)chosen : 0u;
+    sh.digit = (unsigned int)chosen;
     sh.above = has ? chosen_above : 0ull;
+    sh.limit = limit;
+    sh.here = here;
   }
 }
 
@@ -281,8 +294,10 @@ __device__ __forceinline__ void select_bin(SampleShared& sh, int buf, bool by_ma
 //    largest of its 256 groups' maxima is a value that m of its logits reach, so k logits of the row reach the
 //    smallest of the eight. What reaches that bound (some 80 logits for k = 50) goes to block 0, which finds the
 //    threshold, the kept mass and the draw by comparing each with each, and the other blocks leave.
-//  * top_p: with Z the whole mass, a token whose mass is below (1 - p) Z / vocab has at most (1 - p) Z at or below
-//    it, so it is out. The histograms count what is left, and after the first digit only a list of it.
+//  * top_p: what lies below the bin that the first digit settles on is out; where a block has at most half of its
+//    logits left (and room to list them), the other digits walk that list. (A bound on a token's mass, to spare the
+//    first histogram its atomics, cost a pass and more than it saved: top_p 0.95 alone over 64 rows of 151,936 normal
+//    logits 291 us, 200 so, 209 without a list; of 32,768: 108, 60, 71.)
 // Where a bound leaves too much (k above 2,048, ties by the thousand, an infinite maximum) the radix selection
 // over all logits stands. 64 rows of 151,936 logits, top_k 50, top_p 0.95: 146 us with the selection over all logits,
 // 44 so (a cluster of eight blocks a row is 512 blocks, two to an SM: 1.7 rounds of them).
@@ -397,11 +412,8 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
   const float smax = best.v / temp;
   auto s_of = [&](int j) { return cached ? sv[j] : z[begin + j] / temp; };
   const float p = top_p ? top_p[row] : 1.f;
-  const float mp = min_p ? min_p[row] : 0.f;
-  const unsigned long long seed = (unsigned long long)seeds[row];
-  const unsigned long long draw = (unsigned long long)draws[row];
   // Gumbel-max: a token's scaled logit and its own noise.
-  auto noisy = [&](float s, int id) {
+  auto noisy = [](float s, int id, unsigned long long seed, unsigned long long draw) {
     unsigned int r[4];
     philox4x32_10((unsigned int)id, 0u, (unsigned int)draw, (unsigned int)(draw >> 32), (unsigned int)seed,
                   (unsigned int)(seed >> 32), r);
@@ -465,7 +477,7 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
           kept = greater < limit;
         }
       }
-      if (kept && !(e < mp)) pick = noisy(s, id);
+      if (kept && !(e < (min_p ? min_p[row] : 0.f))) pick = noisy(s, id, (unsigned long long)seeds[row], (unsigned long long)draws[row]);
       pick = block_argmax(pick, sh.ascratch);
       if (i == 0) out[row] = pick.i;
       return;
@@ -484,7 +496,7 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
         return key >= bound;
       });
       cluster_totals(cluster, sh, buf, false);
-      if (threadIdx.x < 32) select_bin(sh, buf, false, want);  // the k-th largest has fewer than k above it
+      if (threadIdx.x < 32) select_bin(sh, buf, false, want, -1.f);  // the k-th largest has fewer than k above it
       __syncthreads();
       kkey |= sh.digit << shift;
       want -= sh.above;
@@ -497,69 +509,54 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
   float ecut = 0.f;
   int listed = -1;  // entries of the list of what can still be chosen (-1: no list)
   if (p < 1.f) {
-    unsigned long long sum = 0ull;
-    for (int j = threadIdx.x; j < n; j += SAMPLE_THREADS) {
-      const float s = s_of(j);
-      if (order_key(s) >= kkey) sum += fixed_mass(expf(s - smax));
-    }
-    if (threadIdx.x == 0) sh.mass = 0ull;
-    __syncthreads();
-    if (sum) atomicAdd(&sh.mass, sum);
-    cluster.sync();
-    sum = 0ull;
-    for (unsigned int r = 0; r < cluster.num_blocks(); ++r) sum += cluster.map_shared_rank(&sh, r)->mass;
-    unsigned long long limit = mass_limit(p, sum);
-    const unsigned long long least = limit < sum ? (sum - limit) / (unsigned long long)vocab : 0ull;
     unsigned int ckey = 0u;
+    unsigned long long limit = 0ull;
     for (int shift = 24; shift >= 0; shift -= 8, buf ^= 1) {
-      histogram_pass<true>(sh, buf, listed < 0 ? n : listed, ckey, shift,
-                           [&](int at, unsigned int& key, unsigned long long& weight) {
-        const float s = s_of(listed < 0 ? at : (int)list[at]);
+      auto item = [&](int j, unsigned int& key, unsigned long long& weight) {
+        const float s = s_of(j);
         if (order_key(s) < kkey) return false;  // not kept by top_k
         const float e = expf(s - smax);
         key = __float_as_uint(e);  // e >= 0: its bits order it
         weight = fixed_mass(e);
-        return weight >= least;
-      });
+        return true;
+      };
+      if (listed < 0)
+        histogram_pass<true>(sh, buf, n, ckey, shift, item);
+      else
+        histogram_pass<true>(sh, buf, listed, ckey, shift, [&](int at, unsigned int& key, unsigned long long& weight) {
+          return item((int)list[at], key, weight);
+        });
       cluster_totals(cluster, sh, buf, true);
       // The lowest bin that holds an element whose strictly greater mass is below p * Z: a bin's
       // largest element has exactly the mass of the bins above it.
-      if (threadIdx.x < 32) select_bin(sh, buf, true, limit);
+      if (threadIdx.x < 32) select_bin(sh, buf, true, limit, shift == 24 ? p : -1.f);
       __syncthreads();
       ckey |= sh.digit << shift;
-      limit -= sh.above;
-      if (shift == 24) {
-        // From here on only what lies in that bin or above it counts: a list of it, where it fits.
-        for (int j0 = 0; j0 < n; j0 += SAMPLE_THREADS) {
-          const int j = j0 + (int)threadIdx.x;
-          bool in = false;
-          if (j < n) {
-            const float s = s_of(j);
-            in = order_key(s) >= kkey && __float_as_uint(expf(s - smax)) >= ckey;
-          }
-          const unsigned int who = __ballot_sync(0xffffffffu, in);
-          if (who == 0u) continue;
-          unsigned int at = 0u;
-          if ((threadIdx.x & 31) == 0) at = atomicAdd(&sh.listed, (unsigned int)__popc(who));
-          at = __shfl_sync(0xffffffffu, at, 0) + (unsigned int)__popc(who & ((1u << (threadIdx.x & 31)) - 1u));
-          if (in && at < list_most) list[at] = (unsigned short)j;
+      limit = sh.limit - sh.above;
+      if (shift == 24 && 2 * (int)sh.here <= n && sh.here <= list_most) {
+        // From here on only what lies in that bin or above it counts: a list of it, where that is the smaller part.
+        for (int j = threadIdx.x; j < n; j += SAMPLE_THREADS) {
+          const float s = s_of(j);
+          if (order_key(s) < kkey || __float_as_uint(expf(s - smax)) < ckey) continue;
+          list[atomicAdd(&sh.listed, 1u)] = (unsigned short)j;
         }
-        __syncthreads();
-        if (sh.listed <= list_most) listed = (int)sh.listed;
+        listed = (int)sh.here;
       }
       __syncthreads();
     }
     ecut = __uint_as_float(ckey);
   }
+  const float mp = min_p ? min_p[row] : 0.f;
   if (mp > ecut) ecut = mp;
 
   // The draw over the kept tokens.
+  const unsigned long long seed = (unsigned long long)seeds[row], draw = (unsigned long long)draws[row];
   for (int at = threadIdx.x; at < (listed < 0 ? n : listed); at += SAMPLE_THREADS) {
     const int j = listed < 0 ? at : (int)list[at];
     const float s = s_of(j);
     if (order_key(s) < kkey) continue;
     if (expf(s - smax) < ecut) continue;
-    pick = better(pick, noisy(s, begin + j));
+    pick = better(pick, noisy(s, begin + j, seed, draw));
   }
   pick = block_argmax(pick, sh.ascratch);
   if (threadIdx.x == 0) sh.draw_best = pick;
