@@ -293,13 +293,15 @@ __device__ __forceinline__ void select_bin(SampleShared& sh, int buf, bool by_ma
 //  * top_k: a thread's logits are a group, two lanes' groups make one; with m = ceil(k / 8), every block's m-th
 //    largest of its 256 groups' maxima is a value that m of its logits reach, so k logits of the row reach the
 //    smallest of the eight. What reaches that bound (some 80 logits for k = 50) goes to block 0, which finds the
-//    threshold, the kept mass and the draw by comparing each with each, and the other blocks leave.
+//    threshold, the kept mass and the draw by comparing each with each, and the other blocks leave. Where that is
+//    more than the 512 that one block finishes (always, for k above 512: nothing is sent then), every block walks
+//    the list of its own. top_k 400 over 64 rows of 151,936: 97 us with the whole row walked again, 56 so; 2,000: 128, 65.
 //  * top_p: what lies below the bin that the first digit settles on is out; where a block has at most half of its
 //    logits left (and room to list them), the other digits walk that list. (A bound on a token's mass, to spare the
 //    first histogram its atomics, cost a pass and more than it saved: top_p 0.95 alone over 64 rows of 151,936 normal
 //    logits 291 us, 200 so, 209 without a list; of 32,768: 108, 60, 71.)
-// Where a bound leaves too much (k above 2,048, ties by the thousand, an infinite maximum) the radix selection
-// over all logits stands. 64 rows of 151,936 logits, top_k 50, top_p 0.95: 146 us with the selection over all logits,
+// Where there is no bound or no room for a list (k above 2,048, ties by the thousand, an infinite maximum) the radix
+// selection over all logits stands. 64 rows of 151,936 logits, top_k 50, top_p 0.95: 146 us with the selection over all logits,
 // 44 so (a cluster of eight blocks a row is 512 blocks, two to an SM: 1.7 rounds of them).
 __global__ void __cluster_dims__(SAMPLE_CLUSTER, 1, 1) __launch_bounds__(SAMPLE_THREADS, 2)
 sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice, int cached, unsigned int list_most,
@@ -422,67 +424,73 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
   };
   ArgMax pick{-INFINITY, 0x7fffffff};
 
+  int listed = -1;  // entries of the list of what can still be chosen (-1: no list)
   if (bounded && isfinite(smax)) {
-    // What reaches the bound goes to block 0.
+    // What reaches the bound is listed, and goes to block 0 where k may leave few enough for one block.
+    const bool sends = k <= SAMPLE_THREADS;
     SampleSent* at0 = &cluster.map_shared_rank(&sh, 0)->sent;
     for (int j = threadIdx.x; j < n; j += SAMPLE_THREADS) {
       const float s = s_of(j);
       if (order_key(s) < bound) continue;
       const unsigned int at = atomicAdd(&sh.listed, 1u);
-      if (at < SAMPLE_SENT) {
+      if (at < list_most) list[at] = (unsigned short)j;
+      if (sends && at < SAMPLE_SENT) {
         at0->s[rank][at] = s;
         at0->i[rank][at] = begin + j;
       }
     }
     __syncthreads();
-    if (threadIdx.x < SAMPLE_CLUSTER) cluster.map_shared_rank(&sh, threadIdx.x)->sent_count[rank] = sh.listed;
-    cluster.sync();
-    int total = 0, from = 0, before = 0;  // candidates, and where this thread's is: which block's, how many ahead of that
-    bool fits = true;
+    if (sh.listed <= list_most) listed = (int)sh.listed;
+    if (sends) {
+      if (threadIdx.x < SAMPLE_CLUSTER) cluster.map_shared_rank(&sh, threadIdx.x)->sent_count[rank] = sh.listed;
+      cluster.sync();
+      int total = 0, from = 0, before = 0;  // candidates, and where this thread's is: which block's, how many ahead of that
+      bool fits = true;
 #pragma unroll
-    for (int r = 0; r < SAMPLE_CLUSTER; ++r) {
-      const int c = (int)sh.sent_count[r];
-      fits = fits && c <= SAMPLE_SENT;
-      if ((int)threadIdx.x >= total) from = r, before = total;
-      total += c;
-    }
-    if (fits && total <= SAMPLE_THREADS) {
-      if (rank != 0) return;  // (every access to another block's memory lies before the barrier above)
-      const int i = threadIdx.x;
-      const bool mine = i < total;
-      const float s = mine ? sh.sent.s[from][i - before] : 0.f;
-      const int id = mine ? sh.sent.i[from][i - before] : 0;
-      const unsigned int key = order_key(s);
-      __syncthreads();  // what was sent has been read; its place is used for the keys
-      if (mine) sh.few.key[i] = key;
-      if (i == 0) sh.mass = 0ull;
-      __syncthreads();
-      int larger = 0;
-      for (int o = 0; o < total; ++o) larger += sh.few.key[o] > key;
-      bool kept = mine && larger < k;  // a tie at the k-th largest is kept whole
-      const float e = expf(s - smax);
-      if (p < 1.f) {
-        const unsigned long long mass = kept ? fixed_mass(e) : 0ull;
-        __syncthreads();  // the keys of s have been read
-        if (mine) {
-          sh.few.key[i] = kept ? __float_as_uint(e) : 0u;  // e >= 0: its bits order it
-          sh.few.mass[i] = mass;
-        }
-        if (mass) atomicAdd(&sh.mass, mass);
-        __syncthreads();
-        const unsigned long long limit = mass_limit(p, sh.mass);
-        if (kept && limit != 0ull) {
-          unsigned long long greater = 0ull;
-          for (int o = 0; o < total; ++o) greater += sh.few.key[o] > __float_as_uint(e) ? sh.few.mass[o] : 0ull;
-          kept = greater < limit;
-        }
+      for (int r = 0; r < SAMPLE_CLUSTER; ++r) {
+        const int c = (int)sh.sent_count[r];
+        fits = fits && c <= SAMPLE_SENT;
+        if ((int)threadIdx.x >= total) from = r, before = total;
+        total += c;
       }
-      if (kept && !(e < (min_p ? min_p[row] : 0.f))) pick = noisy(s, id, (unsigned long long)seeds[row], (unsigned long long)draws[row]);
-      pick = block_argmax(pick, sh.ascratch);
-      if (i == 0) out[row] = pick.i;
-      return;
+      if (fits && total <= SAMPLE_THREADS) {
+        if (rank != 0) return;  // (every access to another block's memory lies before the barrier above)
+        const int i = threadIdx.x;
+        const bool mine = i < total;
+        const float s = mine ? sh.sent.s[from][i - before] : 0.f;
+        const int id = mine ? sh.sent.i[from][i - before] : 0;
+        const unsigned int key = order_key(s);
+        __syncthreads();  // what was sent has been read; its place is used for the keys
+        if (mine) sh.few.key[i] = key;
+        if (i == 0) sh.mass = 0ull;
+        __syncthreads();
+        int larger = 0;
+        for (int o = 0; o < total; ++o) larger += sh.few.key[o] > key;
+        bool kept = mine && larger < k;  // a tie at the k-th largest is kept whole
+        const float e = expf(s - smax);
+        if (p < 1.f) {
+          const unsigned long long mass = kept ? fixed_mass(e) : 0ull;
+          __syncthreads();  // the keys of s have been read
+          if (mine) {
+            sh.few.key[i] = kept ? __float_as_uint(e) : 0u;  // e >= 0: its bits order it
+            sh.few.mass[i] = mass;
+          }
+          if (mass) atomicAdd(&sh.mass, mass);
+          __syncthreads();
+          const unsigned long long limit = mass_limit(p, sh.mass);
+          if (kept && limit != 0ull) {
+            unsigned long long greater = 0ull;
+            for (int o = 0; o < total; ++o) greater += sh.few.key[o] > __float_as_uint(e) ? sh.few.mass[o] : 0ull;
+            kept = greater < limit;
+          }
+        }
+        if (kept && !(e < (min_p ? min_p[row] : 0.f)))
+          pick = noisy(s, id, (unsigned long long)seeds[row], (unsigned long long)draws[row]);
+        pick = block_argmax(pick, sh.ascratch);
+        if (i == 0) out[row] = pick.i;
+        return;
+      }
     }
-    if (threadIdx.x == 0) sh.listed = 0u;  // (read by nobody until the list is made, several barriers on)
   }
 
   int buf = 0;
@@ -491,10 +499,16 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
   if (ranked) {
     unsigned long long want = (unsigned long long)k;  // the rank looked for among the elements that match the prefix
     for (int shift = 24; shift >= 0; shift -= 8, buf ^= 1) {
-      histogram_pass<false>(sh, buf, n, kkey, shift, [&](int j, unsigned int& key, unsigned long long&) {
-        key = order_key(s_of(j));
-        return key >= bound;
-      });
+      if (listed < 0)
+        histogram_pass<false>(sh, buf, n, kkey, shift, [&](int j, unsigned int& key, unsigned long long&) {
+          key = order_key(s_of(j));
+          return key >= bound;
+        });
+      else
+        histogram_pass<false>(sh, buf, listed, kkey, shift, [&](int at, unsigned int& key, unsigned long long&) {
+          key = order_key(s_of((int)list[at]));
+          return true;
+        });
       cluster_totals(cluster, sh, buf, false);
       if (threadIdx.x < 32) select_bin(sh, buf, false, want, -1.f);  // the k-th largest has fewer than k above it
       __syncthreads();
@@ -507,7 +521,6 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
   // top_p over what top_k kept: with e = exp(s - max) and Z its sum, the smallest e whose
   // strictly greater mass is below p * Z. min_p: e >= p (the most probable token has e == 1).
   float ecut = 0.f;
-  int listed = -1;  // entries of the list of what can still be chosen (-1: no list)
   if (p < 1.f) {
     unsigned int ckey = 0u;
     unsigned long long limit = 0ull;
@@ -533,7 +546,9 @@ sample_kernel(float* __restrict__ logits, long long stride, int vocab, int slice
       __syncthreads();
       ckey |= sh.digit << shift;
       limit = sh.limit - sh.above;
-      if (shift == 24 && 2 * (int)sh.here <= n && sh.here <= list_most) {
+      if (shift == 24 && listed < 0 && 2 * (int)sh.here <= n && sh.here <= list_most) {
+        if (threadIdx.x == 0) sh.listed = 0u;
+        __syncthreads();
         // From here on only what lies in that bin or above it counts: a list of it, where that is the smaller part.
         for (int j = threadIdx.x; j < n; j += SAMPLE_THREADS) {
           const float s = s_of(j);
@@ -632,7 +647,7 @@ extern "C" int omnia_sample(float* logits, long long stride, int rows, int vocab
   const int slice = ((vocab + SAMPLE_CLUSTER - 1) / SAMPLE_CLUSTER + 3) & ~3;
   const int cached = slice <= 49152 ? 1 : 0;
   const size_t held = cached ? (size_t)slice * sizeof(float) : 0;
-  // The list takes what is left of half an SM: with 64 rows of 201,088 logits a block without its neighbour on the SM
+  // Where the blocks are more than the SMs, the list takes what is left of half an SM: with 64 rows of 201,088 logits a block without its neighbour on the SM
   // took half as long again (temperature alone 147 us against 115).
   static size_t half = 0;
   if (half == 0) {
@@ -642,7 +657,7 @@ extern "C" int omnia_sample(float* logits, long long stride, int rows, int vocab
     half = (114 - 1) * 1024 - ((attributes.sharedSizeBytes + 127) & ~(size_t)127);  // a block's own KB, and what it holds anyway
   }
   size_t room = SAMPLE_LIST * sizeof(unsigned short);
-  if (held <= half && held + room > half) room = (half - held) & ~(size_t)127;
+  if (rows * SAMPLE_CLUSTER > omnia_sm_count() && held <= half && held + room > half) room = (half - held) & ~(size_t)127;
   const size_t smem = held + room;
   static size_t configured = 0;
   if (smem > configured) {
