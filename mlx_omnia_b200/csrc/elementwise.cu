@@ -632,11 +632,13 @@ extern "C" int omnia_rope_angles(const int* positions, const float* inv_freq, in
 
 // ---------------------------------------------------------------------------------
 // act[t, i] = unit(gu[t, i], gu[t, inner + i]) in float32, rounded once, `limit` naming the unit (gated_unit in
-// common.cuh; 0: silu(gate) * up). Sixteen bytes a thread where rows and halves start on sixteen: an element a thread
+// common.cuh; 0: silu(gate) * up). Sixteen bytes a thread (`wide`) where rows and halves start on sixteen: an element a thread
 // with a 64-bit division for its row took 8.3 us for 264 rows of 6,144 bfloat16 (9.7 MB, from L2) and 15.2 for 300 of 12,288; so 4.0 and 6.0.
+// Where an element a thread gives an SM no more than three blocks, the launch is the latency of one thread, and eight
+// elements are one exponential after another: 1 row of 2,048 2.0 us by sixteen bytes, 1.65 so, 17 rows 2.0 and 1.85, 48 rows even.
 template <typename T>
 __global__ void __launch_bounds__(256)
-gated_rows_kernel(const T* __restrict__ gu, T* __restrict__ act, int inner, float alpha, float limit) {
+gated_rows_kernel(const T* __restrict__ gu, T* __restrict__ act, int inner, float alpha, float limit, int wide) {
   pdl_wait();
   pdl_launch_dependents();
   const T* gate = gu + (size_t)blockIdx.x * 2 * inner;
@@ -644,7 +646,7 @@ gated_rows_kernel(const T* __restrict__ gu, T* __restrict__ act, int inner, floa
   T* out = act + (size_t)blockIdx.x * inner;
   constexpr int VEC = 16 / (int)sizeof(T);
   const int first = blockIdx.y * blockDim.x + threadIdx.x, step = gridDim.y * blockDim.x;
-  if (inner % VEC == 0 && (((uintptr_t)gu | (uintptr_t)act) & 15) == 0) {
+  if (wide && inner % VEC == 0 && (((uintptr_t)gu | (uintptr_t)act) & 15) == 0) {
     for (int c = first * VEC; c < inner; c += step * VEC) {
       const uint4 pg = *reinterpret_cast<const uint4*>(gate + c), pu = *reinterpret_cast<const uint4*>(up + c);
       const T *g = reinterpret_cast<const T*>(&pg), *u = reinterpret_cast<const T*>(&pu);
@@ -659,10 +661,14 @@ gated_rows_kernel(const T* __restrict__ gu, T* __restrict__ act, int inner, floa
   for (int c = first; c < inner; c += step) out[c] = from_f32<T>(gated_unit(to_f32(gate[c]), to_f32(up[c]), alpha, limit));
 }
 
+// Up to this many elements a pass over them takes one a thread: three blocks an SM.
+long long small_elements() { return 3LL * 256 * omnia_sm_count(); }
+
 template <typename T>
 void launch_gated_rows(const T* gu, T* act, int rows, int inner, float alpha, float limit, cudaStream_t stream) {
-  const int vec = inner % (16 / (int)sizeof(T)) == 0 ? 16 / (int)sizeof(T) : 1, pieces = (inner / vec + 255) / 256;
-  launch_pdl(gated_rows_kernel<T>, dim3(rows, pieces < 64 ? pieces : 64), 256, 0, stream, gu, act, inner, alpha, limit);
+  const bool wide = (long long)rows * inner > small_elements();
+  const int vec = wide && inner % (16 / (int)sizeof(T)) == 0 ? 16 / (int)sizeof(T) : 1, pieces = (inner / vec + 255) / 256;
+  launch_pdl(gated_rows_kernel<T>, dim3(rows, pieces < 64 ? pieces : 64), 256, 0, stream, gu, act, inner, alpha, limit, (int)wide);
 }
 
 extern "C" int omnia_swiglu(const void* gu, void* act, int rows, int inner, int dtype,
@@ -800,10 +806,11 @@ extern "C" int omnia_scaled_sum(const void* a, float sa, const void* b, float sb
 
 // ---------------------------------------------------------------------------------
 // logits = cap * tanh(z * multiplier / cap)  (cap <= 0: logits = z * multiplier), float32 out.
-// Sixteen bytes of z a thread where both start on sixteen (64 rows of 151,936: 21 us an element a thread, 15 so).
+// Sixteen bytes of z a thread (`wide`) where both start on sixteen (64 rows of 151,936: 21 us an element a thread, 15 so);
+// an element a thread where there are few, as for the gated units (4 rows of 512: 2.0 and 1.6 us, a row of 32,000 2.05 and 1.65).
 template <typename T>
 __global__ void __launch_bounds__(256)
-softcap_kernel(const T* __restrict__ z, float* __restrict__ out, long long total, float multiplier, float cap) {
+softcap_kernel(const T* __restrict__ z, float* __restrict__ out, long long total, float multiplier, float cap, int wide) {
   pdl_wait();
   pdl_launch_dependents();
   constexpr int VEC = 16 / (int)sizeof(T);
@@ -812,7 +819,7 @@ softcap_kernel(const T* __restrict__ z, float* __restrict__ out, long long total
     const float v = to_f32(a) * multiplier;
     return cap > 0.f ? cap * tanhf(v / cap) : v;
   };
-  const long long whole = (((uintptr_t)z | (uintptr_t)out) & 15) == 0 ? total / VEC : 0;
+  const long long whole = wide && (((uintptr_t)z | (uintptr_t)out) & 15) == 0 ? total / VEC : 0;
   for (long long i = at; i < whole; i += stride) {
     const uint4 piece = reinterpret_cast<const uint4*>(z)[i];
     const T* a = reinterpret_cast<const T*>(&piece);
@@ -831,7 +838,7 @@ extern "C" int omnia_softcap(const void* z, float* out, long long total, float m
   if (total == 0) return 0;
   const long long pieces = (total + 255) / 256, most = 16LL * omnia_sm_count();
   OMNIA_DISPATCH_DTYPE(dtype, (launch_pdl(softcap_kernel<T>, (int)(pieces < most ? pieces : most), 256, 0, stream, (const T*)z, out,
-                                          total, multiplier, cap)));
+                                          total, multiplier, cap, total > small_elements())));
   return OMNIA_LAUNCH_RESULT();
 }
 
