@@ -215,10 +215,13 @@ struct Vec4<__nv_bfloat16> {
 // LATE: the norms' weights are read where they are needed instead of up front. With many rows they come from L1,
 // where the rows before left them, and what counts is how many rows an SM has in flight: 32 registers a thread instead
 // of 48, and eight values a thread at every width (sixteen took 84). 2,048 rows of 4,096: 30.4 -> 17.3 us (100 MB: 15.4 at
-// the copy rate), of 2,048: 11.3 -> 10.5, 600 rows of 4,096: 10.5 -> 7.1; under four rows to an SM the weights come
-// up front, since there a row is one chain of trips to memory.
+// the copy rate), 600 rows of 4,096: 10.5 -> 7.1. With few rows a row is one chain of trips to memory, and the weights come
+// up front: up to two rows an SM, and up to twelve where 256 threads or fewer make a row, since an SM holds a good part of
+// those at once either way. Launch after launch (x and branch in L2), 600 / 1,200 / 2,048 rows of 2,048: late 4.5 / 5.9 /
+// 7.8 us, up front 3.8 / 5.8 / 8.4; of 1,024: 3.1 / 4.5 / 4.8 and 2.7 / 3.7 / 5.3; 260 / 300 rows of 4,096 late 3.6 / 4.5 and
+// up front 3.5 / 4.9. Few wide rows of float32 take sixteen values a thread (8 rows of 5,120: 3.2 us, 3.4 with eight).
 template <typename T, int ITERS, bool LATE>
-__global__ void __launch_bounds__(1024, LATE ? 2 : 1) add_rmsnorm_reg_kernel(float* __restrict__ x, const T* __restrict__ branch,
+__global__ void __launch_bounds__(ITERS > 2 ? 512 : 1024, LATE ? 2 : 1) add_rmsnorm_reg_kernel(float* __restrict__ x, const T* __restrict__ branch,
                                        const float* __restrict__ wb, float eps_b, int norm_branch,
                                        const float* __restrict__ wo, float eps_o, int norm_out,
                                        T* __restrict__ h, int hidden) {
@@ -289,11 +292,17 @@ extern "C" int omnia_add_rmsnorm(float* x, const void* branch, const float* wb, 
                                  void* h, int rows, int hidden, int dtype, cudaStream_t stream) {
   if (rows == 0) return 0;
   if (hidden % 4 == 0 && hidden <= 8192) {
+    const bool wide = hidden > 2048, late = rows > (wide ? 2 : 12) * omnia_sm_count();
     const int threads = hidden <= 1024 ? 128 : hidden <= 2048 ? 256 : hidden <= 4096 ? 512 : 1024;  // eight values each
-    const bool late = rows >= 4 * omnia_sm_count();
-    OMNIA_DISPATCH_DTYPE(dtype, (launch_pdl(late ? add_rmsnorm_reg_kernel<T, 2, true> : add_rmsnorm_reg_kernel<T, 2, false>, rows,
-                                            threads, 0, stream, x, (const T*)branch, wb, eps_b, norm_branch, wo, eps_o, norm_out,
-                                            (T*)h, hidden)));
+    OMNIA_DISPATCH_DTYPE(dtype, {
+      auto launch = [&](auto* kernel, int threads) {
+        launch_pdl(kernel, rows, threads, 0, stream, x, (const T*)branch, wb, eps_b, norm_branch, wo, eps_o, norm_out, (T*)h, hidden);
+      };
+      constexpr int FEW = sizeof(T) == 4 ? 4 : 2;
+      if (late) launch(add_rmsnorm_reg_kernel<T, 2, true>, threads);
+      else if (wide) launch(add_rmsnorm_reg_kernel<T, FEW, false>, threads * 2 / FEW);
+      else launch(add_rmsnorm_reg_kernel<T, 2, false>, threads);
+    });
     return OMNIA_LAUNCH_RESULT();
   }
   const size_t smem = (size_t)hidden * sizeof(float);
@@ -635,7 +644,7 @@ extern "C" int omnia_rope_angles(const int* positions, const float* inv_freq, in
 // common.cuh; 0: silu(gate) * up). Sixteen bytes a thread (`wide`) where rows and halves start on sixteen: an element a thread
 // with a 64-bit division for its row took 8.3 us for 264 rows of 6,144 bfloat16 (9.7 MB, from L2) and 15.2 for 300 of 12,288; so 4.0 and 6.0.
 // Where an element a thread gives an SM no more than three blocks, the launch is the latency of one thread, and eight
-// elements are one exponential after another: 1 row of 2,048 2.0 us by sixteen bytes, 1.65 so, 17 rows 2.0 and 1.85, 48 rows even.
+// elements are one exponential after another: a row of 2,048 2.0 us by sixteen bytes, 1.6 so, 17 rows 2.0 and 1.65.
 template <typename T>
 __global__ void __launch_bounds__(256)
 gated_rows_kernel(const T* __restrict__ gu, T* __restrict__ act, int inner, float alpha, float limit, int wide) {

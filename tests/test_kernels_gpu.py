@@ -86,6 +86,14 @@ def test_residual_step_of_many_rows(ops, dtype, rows, hidden):
             close(h1, h2, dtype)
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("rows,hidden", [(1776, 72), (1777, 72), (1780, 1028), (1777, 2048), (296, 2052), (297, 2052),
+                                         (296, 8192), (297, 5000), (3, 4100)])
+def test_residual_steps_around_the_lines_of_their_rule(ops, dtype, rows, hidden):
+    """On both sides of the lines from which narrow and wide rows' weights are read late."""
+    test_residual_step_of_many_rows(ops, dtype, rows, hidden)
+
+
 def make_kv(tokens, nkv, d, page_size, dtype, num_pages, seed=0):
     """A cache view with one request per row of `tokens` (a list of lengths): random page
     placement, every other page poisoned with huge values."""
