@@ -2003,10 +2003,20 @@ MOE_TCGEN05_PAIRS = 1024
 grouped products run on the tcgen05 kernel (tiles of 128 rows of one expert each; fewer rows an expert
 would leave most of every tile empty); below, on the mma.sync kernel with tiles of 64 rows."""
 
-MOE_PAIR_ROWS = 112
-"""From this many pairs an expert on average the grouped products take tiles of 256 rows, two SMs to a tile: such a tile
-brings in a third less than two of 128 rows, which are bound by what they pull out of L2 (19 us a wave of tiles 2,048
-deep against 10.5), and an expert of 113 to 256 rows fills one. With fewer rows most experts need one tile of either."""
+def _moe_pair_pays(pairs: int, experts: int, columns: int, sms: int) -> bool:
+    """Whether the experts' grouped tcgen05 products take tiles of 256 rows, two SMs to a tile, rather than of 128
+    (`columns`: 128 of the first product's per tile). A wave of them brings in a third less, but an expert's last tile
+    is twice as empty. Experts of 137 to 256 rows fill one such tile or two of the others: 0.86 to 0.98 of the time with
+    8 to 128 experts of 512 to 1,536; at 112 to 128 rows, one tile of either, 1.00 to 1.08, at 280 to 350 rows, two
+    against three, 1.0 to 1.07. Further up (0.81 to 0.98) what is left is the waves, as for a dense product: with 8
+    experts of 512 rows three of these against two of the others, 84 us and 78."""
+    rows = pairs / experts
+    if rows < 384:
+        return 136 <= rows <= 256
+    tiles = experts * -(-columns // 128)
+    one, two = -int(-tiles * (rows / 128 + 0.5) // sms), -int(-tiles * (rows / 256 + 0.5) // (sms // 2))
+    return 9 + 11 * two < 10 + 14 * one
+
 
 MOE_STREAM_PAIRS = 8
 """Up to this many pairs an expert on average (or 16 rows, which give no expert more than 16 pairs) the bfloat16 grouped
@@ -2065,7 +2075,7 @@ def moe_experts(h: torch.Tensor, router: torch.Tensor | None, correction: torch.
     if tcgen05 is None:
         tcgen05 = tensor_cores and pairs >= MOE_TCGEN05_PAIRS and pairs >= 64 * experts
     streamed = tensor_cores and not tcgen05 and (rows <= 16 or pairs <= MOE_STREAM_PAIRS * experts)
-    pair = tcgen05 and pairs >= MOE_PAIR_ROWS * experts
+    pair = tcgen05 and _moe_pair_pays(pairs, experts, inner if dual else -(-inner // 2), sm_count(device))
     tile_rows = (256 if pair else 128) if tcgen05 else (8 if rows <= 8 else 16) if streamed else MOE_TILE_ROWS
     max_tiles = min(pairs, -(-pairs // tile_rows) + experts)
     def chosen() -> tuple:

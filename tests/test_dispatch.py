@@ -272,6 +272,7 @@ def test_a_replayed_mixed_step_refuses_an_entry_without_tokens():
 @pytest.mark.parametrize("rows", [1, 16, 17, 600])
 def test_experts_on_the_tensor_cores_take_bfloat16_only(monkeypatch, rows):
     """Every kernel that a step of so many rows would choose reads its operands as bfloat16."""
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
     monkeypatch.setattr(ops, "_function", lambda *a: lambda *args: 0)
     monkeypatch.setattr(ops, "_stream", lambda: 0)
     monkeypatch.setattr(ops, "error_word", lambda device: torch.zeros(1, dtype=torch.int32))
@@ -310,3 +311,12 @@ def test_chunked_recurrence_takes_the_requests_that_bring_a_chunk(monkeypatch, q
         entries, count = calls[name][at: at + 2]
         assert count == (len(q_lens) if want == "all" else len(want))
         assert entries is None if want == "all" else held[entries] == want
+
+
+def test_which_tcgen05_kernel_takes_the_experts():
+    """Tiles of 256 rows where an expert's rows fill one, and from 384 rows on by the waves either kernel runs."""
+    pair = lambda rows, experts=32, columns=768: ops._moe_pair_pays(rows * experts, experts, columns, 148)
+    assert [rows for rows in range(64, 384) if pair(rows)] == list(range(136, 257))
+    assert all(pair(rows) for rows in (400, 512, 700, 1024)) and pair(512, 128) and pair(400, 64, 512) and pair(512, 16, 1536)
+    assert not pair(512, 8, 1024) and pair(400, 8, 1024) and pair(1024, 8, 1024)
+    assert pair(1, 1, 8) is False and ops._moe_pair_pays(200, 1, 136, 148)

@@ -290,6 +290,14 @@ def test_routed_experts(dtype, tensor_cores, rows, hidden, inner, experts, ident
     assert counts.cpu().tolist() == [int((chosen == e).sum()) for e in range(experts)]
 
 
+@pytest.mark.parametrize("rows,hidden,inner,experts,identity,top", [(1500, 72, 40, 9, 0, 1), (1020, 64, 24, 12, 1, 2),
+                                                                  (1300, 72, 136, 3, 0, 1), (1050, 64, 264, 2, 1, 2)])
+def test_routed_experts_on_tiles_of_256_rows(rows, hidden, inner, experts, identity, top):
+    """Experts whose rows fill a tile of two SMs about once and several times, the last one never whole."""
+    assert ops._moe_pair_pays(rows * top, experts, inner, ops.sm_count(CUDA))
+    test_routed_experts("bfloat16", True, rows, hidden, inner, experts, identity, top)
+
+
 # ---- the engine ------------------------------------------------------------------------------
 
 
