@@ -214,6 +214,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   const bool leader = rank == 0;
   const int cluster_id = blockIdx.x >> 1, clusters = gridDim.x >> 1;
   const int k_blocks = (k + BLOCK_K - 1) / BLOCK_K;
+  const bool on_sixteen = ((uintptr_t)out & 15) == 0;  // whole rows of the result may be stored 16 bytes at a time
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
   const uint32_t acc_full0 = smem_u32(bars + 2 * STAGES), acc_empty0 = smem_u32(bars + 2 * STAGES + 2);
 
@@ -350,7 +351,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             unit[j / 2] = __floats2bfloat162_rn(v[0], v[1]);
           }
           // 16 bytes a store: every lane has a row of its own, so a store is 32 requests whatever it carries.
-          if (n0 + c + 32 <= pair_offset && (pair_offset & 7) == 0) {
+          if (n0 + c + 32 <= pair_offset && (pair_offset & 7) == 0 && on_sixteen) {
 #pragma unroll
             for (int j = 0; j < 16; j += 4)
               *reinterpret_cast<uint4*>(dst + c + 2 * j) =
@@ -459,7 +460,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
             float* dst = reinterpret_cast<float*>(out) + (size_t)row * n + n0 + c;
             // 16 bytes a store, as above: with four bytes eight epilogue warps were slower than four (2,048 x 151,936 x
             // 2,048: 2.63 ms against 2.31), so 1.34.
-            const bool whole = n0 + c + 32 <= n && (n & 3) == 0 && ((uintptr_t)out & 15) == 0;
+            const bool whole = n0 + c + 32 <= n && (n & 3) == 0 && on_sixteen;
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
               float v[4];
@@ -484,7 +485,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
               for (int j = 0; j < 32; ++j)
                 acc[j] = __float_as_uint(gelu_erf(__bfloat162float(__float2bfloat16_rn(__uint_as_float(acc[j])))));
             }
-            if (n0 + c + 32 <= n && (n & 7) == 0) {
+            if (n0 + c + 32 <= n && (n & 7) == 0 && on_sixteen) {
 #pragma unroll
               for (int j = 0; j < 32; j += 8) {
                 uint4 packed;

@@ -567,6 +567,20 @@ def test_tcgen05_products(ops, kernel, m, n, k):
     ops.raise_on_error(a.device)
 
 
+@pytest.mark.parametrize("offset", [2, 4])
+def test_two_sm_products_into_a_result_off_sixteen_bytes(ops, offset):
+    """A result that starts anywhere its elements may start: every epilogue gives the bits of an aligned one."""
+    m, n, k = 260, 512, 128
+    a, w = rand(m, k, dtype=torch.bfloat16, seed=1), rand(n, k, dtype=torch.bfloat16, scale=0.05, seed=2)
+    for epilogue, columns, dtype in ((0, n, torch.bfloat16), (1, n // 2, torch.bfloat16), (2, n, torch.float32)):
+        want = ops._gemm_tcgen05(a, w, torch.empty(m, columns, dtype=dtype, device="cuda"), epilogue, 3.0, 7.0 * (epilogue == 2), pair=True)
+        room = torch.zeros(m * columns + 16, dtype=dtype, device="cuda")
+        got = room[offset // 2: offset // 2 + m * columns].view(m, columns)
+        ops._gemm_tcgen05(a, w, got, epilogue, 3.0, 7.0 * (epilogue == 2), pair=True)
+        assert torch.equal(got, want) and float(room[: offset // 2].abs().sum() + room[offset // 2 + m * columns:].abs().sum()) == 0
+    ops.raise_on_error(a.device)
+
+
 def test_sampling(ops):
     vocab, rows = 1531, 6
     logits = rand(rows, vocab, scale=2.0, seed=9)
