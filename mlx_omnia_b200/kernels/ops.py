@@ -2018,10 +2018,20 @@ def _moe_pair_pays(pairs: int, experts: int, columns: int, sms: int) -> bool:
     return 9 + 11 * two < 10 + 14 * one
 
 
-MOE_STREAM_PAIRS = 8
-"""Up to this many pairs an expert on average (or 16 rows, which give no expert more than 16 pairs) the bfloat16 grouped
-products stream the weights as a decode step's dense products do, in entries of 8 or 16 rows: an expert with more rows
-than that has its matrix read again for the next entry, which above this average happens often."""
+def _moe_stream_rows(rows: int, pairs: int, experts: int, hidden: int, inner: int) -> int:
+    """Rows of an entry (8 or 16) where the experts' bfloat16 products stream the weights as a decode step's dense
+    products do, 0 where they take mma.sync tiles. An expert with more rows than an entry has its matrix read again for
+    the next one; entries of 16 multiply twice as much for every weight and take 1.1 to 1.2 times as long, until second
+    entries come often: from 7 pairs an expert on (8 of 32 experts of 2,048 x 768: 78 us with eight, 73 with sixteen, 81
+    on mma.sync tiles; 6: 65, 71, 78), and not at all above 8, unless 16 rows in all leave no expert more than an entry.
+    Small matrices pay for an entry's start: above 6 pairs they stay with the tiles (64 experts of 512 x 512 at 8: 51
+    and 47 us), and inner widths under 512, which fill less than half of the second product's stages, stream only
+    few pairs (256 of 1,024 x 256, 64 pairs: 49 against 51, 128: 67 against 60; 64 of 4,096 x 256, 256 pairs: 124, 110)."""
+    if inner < 512 and pairs > inner // 4:
+        return 0
+    if rows <= 8 or pairs <= 6 * experts:
+        return 8
+    return 16 if rows <= 16 or (pairs <= 8 * experts and min(hidden, inner) >= 768) else 0
 
 
 def moe_experts(h: torch.Tensor, router: torch.Tensor | None, correction: torch.Tensor | None, gate_up: torch.Tensor,
@@ -2074,9 +2084,9 @@ def moe_experts(h: torch.Tensor, router: torch.Tensor | None, correction: torch.
         tensor_cores = h.dtype == torch.bfloat16 and hidden % 8 == 0 and inner % 8 == 0
     if tcgen05 is None:
         tcgen05 = tensor_cores and pairs >= MOE_TCGEN05_PAIRS and pairs >= 64 * experts
-    streamed = tensor_cores and not tcgen05 and (rows <= 16 or pairs <= MOE_STREAM_PAIRS * experts)
+    entry_rows = _moe_stream_rows(rows, pairs, experts, hidden, inner) if tensor_cores and not tcgen05 else 0
     pair = tcgen05 and _moe_pair_pays(pairs, experts, inner if dual else -(-inner // 2), sm_count(device))
-    tile_rows = (256 if pair else 128) if tcgen05 else (8 if rows <= 8 else 16) if streamed else MOE_TILE_ROWS
+    tile_rows = (256 if pair else 128) if tcgen05 else entry_rows or MOE_TILE_ROWS
     max_tiles = min(pairs, -(-pairs // tile_rows) + experts)
     def chosen() -> tuple:
         """The choices, and every chosen expert's output."""
@@ -2124,7 +2134,7 @@ def moe_experts(h: torch.Tensor, router: torch.Tensor | None, correction: torch.
                            _ptr(tile_count), max_tiles, alpha, limit, err, _stream()), "gemm_tcgen05_grouped")
             _check(grouped(_ptr(act), _ptr(down), _ptr(out), pairs, hidden, inner, experts, 0, _ptr(tiles),
                            _ptr(tile_count), max_tiles, 1.0, 0.0, err, _stream()), "gemm_tcgen05_grouped")
-        elif streamed:
+        elif entry_rows:
             stream = _function("gemv_stream", "omnia_gemv_stream_grouped",
                                [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int,
                                 c_float, c_float, c_int, c_void_p, c_void_p])

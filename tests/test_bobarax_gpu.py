@@ -492,6 +492,16 @@ def test_streamed_experts(rows, hidden, inner, experts, top, gated, skewed):
     ops.raise_on_error(CUDA)
 
 
+@pytest.mark.parametrize("rows,hidden,inner,experts,top,entry", [(12, 264, 520, 5, 3, 16), (16, 1032, 1048, 3, 2, 16), (70, 776, 792, 40, 4, 16),
+                                                                 (9, 1048, 520, 9, 4, 8), (40, 136, 1032, 33, 4, 8), (1, 264, 24, 2, 1, 8)])
+@pytest.mark.parametrize("gated", [True, False])
+@pytest.mark.parametrize("skewed", [False, True])
+def test_streamed_experts_in_entries_of_eight_and_sixteen(rows, hidden, inner, experts, top, entry, gated, skewed):
+    """Steps whose experts stream, in entries of the size that the rule names."""
+    assert ops._moe_stream_rows(rows, rows * top, experts, hidden, inner) == entry
+    test_streamed_experts(rows, hidden, inner, experts, top, gated, skewed)
+
+
 # ---- the engine -----------------------------------------------------------------------------
 
 

@@ -320,3 +320,14 @@ def test_which_tcgen05_kernel_takes_the_experts():
     assert all(pair(rows) for rows in (400, 512, 700, 1024)) and pair(512, 128) and pair(400, 64, 512) and pair(512, 16, 1536)
     assert not pair(512, 8, 1024) and pair(400, 8, 1024) and pair(1024, 8, 1024)
     assert pair(1, 1, 8) is False and ops._moe_pair_pays(200, 1, 136, 148)
+
+
+def test_which_experts_stream_their_weights():
+    """Entries of eight rows up to six pairs an expert, of sixteen just above, tiles beyond, and for small matrices sooner."""
+    entry = lambda rows, top, experts, hidden, inner: ops._moe_stream_rows(rows, rows * top, experts, hidden, inner)
+    assert [entry(rows, 4, 32, 2048, 768) for rows in (1, 8, 9, 48, 49, 64, 65)] == [8, 8, 8, 8, 16, 16, 0]
+    assert [entry(rows, 6, 64, 512, 512) for rows in (8, 16, 64, 65, 85)] == [8, 8, 8, 0, 0]
+    assert [entry(rows, 8, 256, 1024, 256) for rows in (1, 8, 9, 64)] == [8, 8, 0, 0]
+    assert [entry(rows, 6, 64, 2048, 384) for rows in (8, 16, 17)] == [8, 8, 0]
+    assert [entry(rows, 8, 8, 2048, 1024) for rows in (8, 9, 16, 17)] == [8, 16, 16, 0]
+    assert [entry(rows, 1, 2, 264, 24) for rows in (6, 7, 16)] == [8, 0, 0]
