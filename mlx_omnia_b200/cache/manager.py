@@ -159,7 +159,8 @@ class CacheManager:
             elif need.state is not None:
                 self.state[entry] = slots_of(need.state)
                 if need.initial_state is not None:
-                    self.initial_state[entry] = need.initial_state.to(need.state.dtype).to(device).expand(need.state.shape).contiguous()
+                    start = need.initial_state.to(need.state.dtype).to(device)  # whatever can be written to a slot
+                    self.initial_state[entry] = start.expand(1, *need.state.shape)[0].contiguous()
             if getattr(need, "block_state", None):
                 self.block_state[entry] = {name: slots_of(spec) for name, spec in need.block_state.items()}
         # State that belongs to the model and to no schedule entry (an embedding that looks at the token before).

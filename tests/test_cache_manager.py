@@ -6,6 +6,7 @@ from __future__ import annotations
 import random
 
 import pytest
+import torch
 
 from mlx_omnia_b200.cache import CacheError, CacheManager, PagePool
 from mlx_omnia_b200.parts.base import KVSpec, StateSpec
@@ -144,3 +145,14 @@ def test_rows_of_any_shape_and_a_stride_size_their_own_pages():
     assert all(g.pool.free == 10 for g in m.groups)
     with pytest.raises(ValueError, match="positive"):
         KVSpec(())
+
+
+@pytest.mark.parametrize("shape", [(3, 4), (1, 3, 4), (3, 1), (4,), (1,), ()])
+def test_a_state_starts_as_whatever_can_be_written_to_its_slot(shape):
+    start = torch.arange(1, 13, dtype=torch.float32)[: max(torch.Size(shape).numel(), 1)].reshape(shape)
+    m = CacheManager([CacheNeed(None, StateSpec((3, 4)), None, start)], page_size=4, pages_per_group=1, max_requests=4)
+    m.state[0].fill_(9.0)
+    m.reset_slots([2, 0])
+    expect = torch.full((5, 3, 4), 9.0)
+    expect[[2, 0]] = start
+    assert torch.equal(m.state[0], expect)
