@@ -258,6 +258,46 @@ def test_single_tokens_beside_prompts(ops, nq, nkv, d, page, window, q_lens, seq
     ops.raise_on_error(q.device)
 
 
+@pytest.mark.parametrize("nq,nkv,d,page,q_lens,seq_lens", [
+    (16, 8, 128, 16, [1, 256, 1, 1], [4000, 900, 9, 700]), (16, 8, 128, 16, [1, 512, 1], [3000, 512, 77]),  # two prompt blocks to an SM, one
+    (4, 2, 16, 4, [1, 40, 1], [600, 40, 33]), (4, 2, 64, 16, [1] * 9 + [3], [5 + 300 * i for i in range(9)] + [4000])])
+def test_single_tokens_beside_prompts_in_a_chain_of_launches(ops, nq, nkv, d, page, q_lens, seq_lens):
+    """What the two kernels read is written right in front of them and what they wrote is read right behind them, all by
+    kernels that may begin early, with new values every time: a captured chain gives the bits of launches that each
+    have the GPU to themselves."""
+    step = step_of(q_lens, seq_lens)
+    step.workspace = {"private": True}
+    pages, table = make_kv(seq_lens, nkv, d, page, torch.bfloat16, 4 + sum(-(-n // page) for n in seq_lens), seed=3)
+    pages.normal_(generator=torch.Generator(device="cuda").manual_seed(4))
+    slots = [int(table[s, pos // page]) * page + pos % page for s, (q, n) in enumerate(zip(q_lens, seq_lens)) for pos in range(n - q, n)]
+    view = KVView(pages, table, torch.tensor(slots, device="cuda"), page, None)
+    inv_freq = (10000.0 ** (-torch.arange(d // 2, dtype=torch.float64) * 2 / d)).float().cuda()
+    projs = [rand(step.num_tokens, (nq + 2 * nkv) * d, dtype=torch.bfloat16, seed=50 + i) for i in range(12)]
+    before = pages.clone()
+
+    def chain(settle):
+        outs = []
+        for proj in projs:
+            q = ops.qk_norm_rope_store(proj, 0, nq * d, (nq + nkv) * d, nq, nkv, d, 1e-6, inv_freq, step.positions, view)
+            settle()
+            out = ops.paged_attention(q, view, step, d ** -0.5)
+            settle()
+            outs.append((out, ops.swiglu(out)))
+            settle()
+        return outs
+
+    want = [(a.clone(), b.clone()) for a, b in chain(torch.cuda.synchronize)]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = chain(lambda: None)
+    for _ in range(3):
+        pages.copy_(before)
+        graph.replay()
+        for (a, b), (c, e) in zip(got, want):
+            assert torch.equal(a, c) and torch.equal(b, e)
+    ops.raise_on_error(pages.device)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("nq,nkv,d,page,window", [(6, 3, 128, 16, 33), (16, 8, 64, 16, 20), (6, 3, 128, 16, None),
                                                    (4, 2, 128, 32, 100), (8, 1, 24, 8, 16), (5, 5, 40, 4, 70)])
