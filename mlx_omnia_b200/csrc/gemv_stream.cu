@@ -475,8 +475,9 @@ gemv_stream_kernel(const bf16* __restrict__ a, const __grid_constant__ CUtensorM
           for (int s2 = 0; s2 < CONSUMER_WARPS; ++s2) up += partial[s2][i * TILE_ROWS + 8 + r][token];
           const int col = tile * 8 + r;
           if (col >= inner) continue;
-          // The two halves are rounded to bfloat16 first, as a separate product would round them (the experts' other
-          // kernels round the unit's result only, and so does the grouped form).
+          // The two halves are rounded to bfloat16 first, as a separate product would round them. The grouped form rounds
+          // the unit's result only, as the experts' mma.sync product does (moe.cu), which takes the steps of a few more
+          // rows; their tcgen05 products, for many rows, round the halves first.
           const float gate = GROUPED ? v : __bfloat162float(__float2bfloat16_rn(v));
           if (!GROUPED) up = __bfloat162float(__float2bfloat16_rn(up));
           // `cap` says which unit (gated_unit in common.cuh), `multiplier` is the clamped one's slope.

@@ -10,7 +10,7 @@
 // -> 97, 600 + 300 + 5 tokens 165 -> 44, 32 tokens 13.2 -> 8.8, 16 tokens 9.4 -> 9.1. The activated q, k and v are
 // bfloat16 as lightning.cu rounds them, so they are exact operands; everything else that enters a product (the weighted
 // triangle, the weighted v, the state) is float32 and goes in as the sum of three bfloat16 numbers, 24 bits of mantissa
-// over the whole range of exponents. Sums and the carried state are float32, sixteen products at a time from zero and
+// for numbers from 2^-109 up. Sums and the carried state are float32, sixteen products at a time from zero and
 // then added on the ordinary cores: the tensor cores' own running sum cuts off what does not fit instead of rounding
 // it. From the result in 64 bits, after 2,048 tokens: outputs 1.1e-7 and state 1.4e-7 (token by token 1.2e-7 and
 // 5.8e-7; with running sums 2e-6 both), after 128: 7.6e-8 and 6.5e-8 (6.0e-8 and 1.8e-7). The powers of the decay are
@@ -20,7 +20,7 @@
 // product, or as a bfloat16), a chunk's products would carry it to tokens that come before it, since a weight of zero
 // times it is NaN, and would make NaN of an infinity taken apart. Whatever went in, an output or the last state that is
 // not finite comes of it; the block then walks its tokens once more, one by one as lightning.cu does, from the state in
-// memory, which it writes only at its end. (The parts of a number below 2^-109 lose bits to bfloat16's smallest exponent.)
+// memory, which it writes only at its end.
 //
 // A block owns LIGHTNING_COLS value columns of one head of one request and walks its chunks in order; a column of S
 // needs no other column. Warp w has 16 of the chunk's tokens for the first three products (the tokens dealt so that the

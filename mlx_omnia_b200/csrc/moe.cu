@@ -624,7 +624,8 @@ extern "C" int omnia_moe_route_table(const int* ids, const int* table, int token
 extern "C" int omnia_moe_tile_rows() { return TILE_ROWS; }
 
 // After `route`: the sorted order (offsets, place, source) and the list of row tiles (of at most `tile_rows`
-// rows: omnia_moe_tile_rows() for this file's products, 128 for the tcgen05 kernel's grouped form).
+// rows: omnia_moe_tile_rows() for this file's products, 8 or 16 for the streamed ones (gemv_stream.cu), 128 or 256 for the
+// tcgen05 kernels' grouped forms, one SM or two to a tile).
 extern "C" int omnia_moe_plan(const int* choice, int* counts, int* cursors, int* offsets, int* tiles, int* tile_count,
                               int* place, int* source, int tokens, int top, int experts, int max_tiles,
                               int tile_rows, cudaStream_t stream) {

@@ -889,8 +889,10 @@ def _pair_pays(rows: int, n: int, k: int, epilogue: int, sms: int) -> bool:
         # gate|up with SwiGLU: tiles of 128 output columns, 128 rows to an SM or 256 to a pair. What
         # decides is how many waves of tiles each kernel runs (measured, 12,288 weight rows of 2,048:
         # some 10 us and 14 a wave for one SM, 9 and 11 a wave for a pair; 512 / 1,082 rows: 38 / 53 us
-        # against 29.6 / 52). A pair's wave counts as 12: where pairs run one wave more than a few, what they gain
-        # depends on the depth (1,082 rows of 4,096: 90 us against 93), and one SM keeps those.
+        # against 29.6 / 52). A pair's wave counts as 12, and the depth is not asked: where pairs run one wave more than
+        # a few, shallow products would gain by them and deep ones lose, and one SM keeps them all (one SM / a pair, us,
+        # 1,024, 2,048, 4,096 and 8,192 deep: 1,082 x 12,288 39 / 32, 53 / 52, 93 / 99, 194 / 209; 896 x 24,576 63 / 44,
+        # 93 / 80, 167 / 163, 342 / 335).
         tiles = -(-(n // 2) // 128)
         one = -(-(-(-rows // 128) * tiles) // sms)
         two = -(-(-(-rows // 256) * tiles) // (sms // 2))
@@ -1996,12 +1998,12 @@ def moe_route_table(token_ids: torch.Tensor, table: torch.Tensor, experts: int,
 
 
 MOE_TILE_ROWS = 64
-"""Rows of a tile of the grouped products of csrc/moe.cu (the tcgen05 kernel's grouped form takes 128)."""
+"""Rows of a tile of the grouped products of csrc/moe.cu."""
 
 MOE_TCGEN05_PAIRS = 1024
 """From this many (row, choice) pairs on, and at least 64 of them an expert on average, the bfloat16
 grouped products run on the tcgen05 kernel (tiles of 128 rows of one expert each; fewer rows an expert
-would leave most of every tile empty); below, on the mma.sync kernel with tiles of 64 rows."""
+would leave most of every tile empty); below, on the mma.sync kernel with tiles of 64 rows, or streamed."""
 
 def _moe_pair_pays(pairs: int, experts: int, columns: int, sms: int) -> bool:
     """Whether the experts' grouped tcgen05 products take tiles of 256 rows, two SMs to a tile, rather than of 128
@@ -2048,8 +2050,9 @@ def moe_experts(h: torch.Tensor, router: torch.Tensor | None, correction: torch.
     rows) and down [experts, hidden, inner]; router outputs beyond the experts with tensors are
     identity experts (their output is h). Nothing is asked of the host: rows are sorted by expert on
     the device, and the grouped products walk a tile list made there. bfloat16 runs on the tensor
-    cores: the tcgen05 kernel's grouped form for many rows (`tcgen05` names the choice), mma.sync for
-    few (`tensor_cores` False keeps both off); float32 on the ordinary cores.
+    cores: the tcgen05 kernels' grouped forms for many rows (`tcgen05` names the choice; one SM to a tile or two:
+    `_moe_pair_pays`), streamed weights for few (`_moe_stream_rows`), mma.sync between them (`tensor_cores` False
+    keeps all off); float32 on the ordinary cores.
 
     With `table` (int32 [vocab, top]) and the rows' `token_ids` there is no router: a token's experts are
     its id's row of the table, each weighing 1 / top. `limit` > 0 makes every expert the clamped unit
