@@ -133,7 +133,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   volatile uint32_t* group_mask = reinterpret_cast<volatile uint32_t*>(tmem_holder + 2);  // [V_STAGES]
   volatile int* drawn = reinterpret_cast<volatile int*>(tmem_holder + 2 + V_STAGES);  // the ticket this part drew
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = omnia_warp_index(), lane = threadIdx.x & 31;
   const int* item = work + WORK_INTS * blockIdx.x;
   const int seq = item[0], tok0 = item[1], kvh = item[2], parts = item[5] & 255, part = item[5] >> 8, slot0 = item[6],
             unit = item[7];
@@ -196,15 +196,15 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     // a warp busy for about 70 ns: one warp for both rings spent more than half a tile's time on it
     // (2,048 tokens: 61 us with one warp, 52 us with one per ring; two per ring: no faster). ------
     const int which = warp == 0 ? 0 : 1;  // 0 keys, 1 values
-    if (warp == 0 && lane == 0) {
+    if (warp == 0 && omnia_elect_one()) {
       mbar_expect_tx(q_full, DH * ROWS * 128);
       for (int h = 0; h < DH; ++h)
         tma_load_3d(smem_u32(q_s) + h * HALF_BYTES, &map_q, q_full, h * 64, kvh * GROUP, q_begin + tok0);
     }
-    // Lane = group * DH + half: each of the tile's boxes (16 keys x 64 dims) is issued by its own lane.
+    // Lane = group * DH: the tile's page groups are looked up side by side, their boxes (16 keys x 64 dims) issued by one lane.
     const int* table = block_table + (size_t)seq * max_pages;
     if (lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_kv) : "memory");
-    const int g = lane / DH, h = lane % DH;
+    const int g = lane / DH;
     const bool active = lane < (BN / 16) * DH;
     // The page of this lane's group in tile t (-2: the group lies outside what the block reads).
     // Page numbers are fetched a whole tile before they are used, so the table's latency is hidden.
@@ -232,7 +232,11 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         load = false;
       }
       const uint32_t loaded = __ballot_sync(0xffffffffu, load);
-      if (lane == 0) {
+      const int mine = load ? (((page * 2 + which) * nkv + kvh) * page_size) + pos % page_size : 0;
+      int y[BN / 16];
+#pragma unroll
+      for (int x = 0; x < BN / 16; ++x) y[x] = __shfl_sync(0xffffffffu, mine, x * DH);
+      if (omnia_elect_one()) {
         if (which) {
           uint32_t mask = 0;
 #pragma unroll
@@ -240,13 +244,15 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
           group_mask[s] = mask;
         }
         mbar_expect_tx(full, __popc(loaded) * GROUP_BYTES);
+        const uint32_t dst = smem_u32(which ? v_s + s * V_BYTES : k_s + s * K_BYTES);
+#pragma unroll
+        for (int x = 0; x < BN / 16; ++x)
+          if ((loaded >> (x * DH)) & 1u)
+#pragma unroll
+            for (int half = 0; half < DH; ++half)
+              tma_load_2d(dst + half * TILE_HALF + x * GROUP_BYTES, &map_kv, full, half * 64, y[x]);
       }
       __syncwarp();
-      if (load) {
-        const int y = (((page * 2 + which) * nkv + kvh) * page_size) + pos % page_size;
-        const uint32_t dst = smem_u32(which ? v_s + s * V_BYTES : k_s + s * K_BYTES) + h * TILE_HALF + g * GROUP_BYTES;
-        tma_load_2d(dst, &map_kv, full, h * 64, y);
-      }
       if (lane == 0) STAMP(0, j, which * 2 + 1);
       issued = j + 1;
     };
@@ -275,7 +281,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     // 1.27 us, two threads keep the scores' chain and the values' chain going side by side (1.06 us).
     // What one thread's products must wait for of the other's goes through barriers: a score buffer
     // is written again only when the P V product that read P from it is done (v_done, two tiles back).
-    if (lane == 0) {
+    if (omnia_elect_one()) {
       constexpr uint32_t instr_s = idesc(BM, BN, false);
       // Descriptors differ only in their address field (the low 14 bits, in units of 16 bytes).
       const uint64_t q_desc = desc_k_major(smem_u32(q_s));
@@ -299,7 +305,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     }
   } else if (warp == 7) {
     // ---- issuer of the value products: O += P_j V_j ---------------------------------------------------
-    if (lane == 0) {
+    if (omnia_elect_one()) {
       constexpr uint32_t instr_o = idesc(BM, D, true);
       uint64_t v_desc[V_STAGES];
       for (int s = 0; s < V_STAGES; ++s) v_desc[s] = desc_mn_major(smem_u32(v_s + s * V_BYTES), TILE_HALF);

@@ -111,7 +111,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   float* row_state = reinterpret_cast<float*>(tmem_holder + 4 + V_STAGES);  // [2][128]: the offset each team last chose
   float* row_sum = row_state + 2 * BM;                                       // [2][128] sums, then [2][128] their offsets
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = omnia_warp_index(), lane = threadIdx.x & 31;
   const int* item = work + WORK_INTS * blockIdx.x;
   const int seq = item[0], tok0 = item[1], kvh = item[2];
   if (item[4] >= 0 || (item[5] & 255) > 1) {  // a part of a block: not this kernel's
@@ -162,18 +162,18 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     // 70 ns whatever its size, so each ring has two warps that take turns with its stages. ----------
     const int which = warp >= WARP_V ? 1 : 0;          // 0 keys, 1 values
     const int turn = warp - (which ? WARP_V : WARP_K);  // this warp's stages: turn, turn + 2, ...
-    if (warp == WARP_K && lane == 0) {
+    if (warp == WARP_K && omnia_elect_one()) {
       mbar_expect_tx(q_full, DH * ROWS * 128);
       for (int h = 0; h < DH; ++h)
         tma_load_3d(smem_u32(q_s) + h * HALF_BYTES, &map_q, q_full, h * 64, kvh * GROUP, q_begin + tok0);
     }
-    // Lane = group * DH + half: each of the stage's boxes is issued by its own lane.
+    // Lane = group * DH: the stage's page groups are looked up side by side, their boxes issued by one lane.
     const int* table = block_table + (size_t)seq * max_pages;
     if (lane == 0) asm volatile("prefetch.tensormap [%0];" ::"l"(&map_kv) : "memory");
     const int keys = which ? BN : SN;              // keys per stage of this ring
     const int count = which ? n_tiles : n_super;   // stages the ring's warps fill
     const int stages = which ? V_STAGES : K_STAGES;
-    const int g = lane / DH, h = lane % DH;
+    const int g = lane / DH;
     const bool active = lane < (keys / 16) * DH;
     // The page of this lane's group in stage t (-2: the group lies outside what the block reads).
     // Page numbers are fetched a turn before they are used, so the table's latency is hidden.
@@ -200,7 +200,11 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
         load = false;
       }
       const uint32_t loaded = __ballot_sync(0xffffffffu, load);
-      if (lane == 0) {
+      const int mine = load ? (((page * 2 + which) * nkv + kvh) * page_size) + pos % page_size : 0;
+      int y[SN / 16];
+#pragma unroll
+      for (int x = 0; x < SN / 16; ++x) y[x] = __shfl_sync(0xffffffffu, mine, x * DH);
+      if (omnia_elect_one()) {
         if (which) {
           uint32_t mask = 0;
 #pragma unroll
@@ -208,14 +212,15 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
           group_mask[s] = mask;
         }
         mbar_expect_tx(full, __popc(loaded) * GROUP_BYTES);
+        const uint32_t dst = smem_u32(which ? v_s + s * V_BYTES : k_s + s * K_BYTES);
+#pragma unroll
+        for (int x = 0; x < SN / 16; ++x)
+          if ((loaded >> (x * DH)) & 1u)
+#pragma unroll
+            for (int half = 0; half < DH; ++half)
+              tma_load_2d(dst + half * (which ? TILE_HALF : K_TILE_HALF) + x * GROUP_BYTES, &map_kv, full, half * 64, y[x]);
       }
       __syncwarp();
-      if (load) {
-        const int y = (((page * 2 + which) * nkv + kvh) * page_size) + pos % page_size;
-        const uint32_t dst = smem_u32(which ? v_s + s * V_BYTES : k_s + s * K_BYTES) + h * (which ? TILE_HALF : K_TILE_HALF) +
-                             g * GROUP_BYTES;
-        tma_load_2d(dst, &map_kv, full, h * 64, y);
-      }
       if (lane == 0) STAMP(0, j, which * 2 + 1);
       issued = j;
     };
@@ -242,7 +247,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     // chain and the values' chain run side by side. What one thread's products must wait for of the
     // other's goes through barriers: a score buffer is written again only when the products that read
     // P from it are done (v_done of its last V stage, two tiles back).
-    if (lane == 0) {
+    if (omnia_elect_one()) {
       constexpr uint32_t instr_s = idesc(BM, SN, false);
       // Descriptors differ only in their address field (the low 14 bits, in units of 16 bytes).
       const uint64_t q_desc = desc_k_major(smem_u32(q_s));
@@ -268,7 +273,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     }
   } else if (warp == WARP_PV) {
     // ---- issuer of the value products: O += P V, a V stage (64 keys) at a time ------------------------
-    if (lane == 0) {
+    if (omnia_elect_one()) {
       constexpr uint32_t instr_o = idesc(BM, D, true);
       uint64_t v_desc[V_STAGES];
       for (int s = 0; s < V_STAGES; ++s) v_desc[s] = desc_mn_major(smem_u32(v_s + s * V_BYTES), TILE_HALF);

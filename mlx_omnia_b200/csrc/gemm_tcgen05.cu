@@ -143,7 +143,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = omnia_warp_index(), lane = threadIdx.x & 31;
   const int k_blocks = (k + BLOCK_K - 1) / BLOCK_K;
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + STAGES);
   const uint32_t acc_full0 = smem_u32(bars + 2 * STAGES), acc_empty0 = smem_u32(bars + 2 * STAGES + 2);
@@ -189,7 +189,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   // same rows of w), so blocks running side by side read the same weight tile out of L2.
   if (warp == 0) {
     // ---- producer ----------------------------------------------------------------------
-    if (lane == 0) {
+    if (omnia_elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
@@ -222,7 +222,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     }
   } else if (warp == 1) {
     // ---- MMA issuer ----------------------------------------------------------------------
-    if (lane == 0) {
+    if (omnia_elect_one()) {
       constexpr uint32_t idesc = umma_idesc(BLOCK_M, BLOCK_N);
       uint32_t it = 0, local = 0;
       bool ok = true;

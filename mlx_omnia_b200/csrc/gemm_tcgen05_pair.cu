@@ -209,7 +209,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = omnia_warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
   const bool leader = rank == 0;
   const int cluster_id = blockIdx.x >> 1, clusters = gridDim.x >> 1;
@@ -257,7 +257,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
 
   if (warp == 0) {
     // ---- producer (both blocks) -------------------------------------------------------------
-    if (lane == 0) {
+    if (omnia_elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (int tile = cluster_id; tile < total_tiles && ok; tile += clusters) {
@@ -280,7 +280,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid
     }
   } else if (warp == 1) {
     // ---- MMA issuer (the leader) --------------------------------------------------------------
-    if (lane == 0 && leader) {
+    if (leader && omnia_elect_one()) {
       constexpr uint32_t idesc = umma_idesc(2 * BLOCK_M, TILE_N);
       uint32_t it = 0, local = 0;
       bool ok = true;
