@@ -75,6 +75,12 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool va
   const int bytes = valid ? 16 : 0;  // 0 source bytes: the 16 destination bytes are zero-filled
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(s), "l"(gmem), "r"(bytes));
 }
+// The same with a cache policy.
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool valid, uint64_t policy) {
+  const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+  const int bytes = valid ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global.L2::cache_hint [%0], [%1], 16, %2, %3;\n" ::"r"(s), "l"(gmem), "r"(bytes), "l"(policy));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
@@ -132,7 +138,7 @@ __device__ __forceinline__ const bf16* cache_row(const CacheRef& c, int pos, int
 //   keep:    keys below it are visible whatever row_lo says (up to row_hi) ...
 //   floor:   ... unless they lie below this (they were attended to in a tile of their own)
 //   cap, pre: cap > 0: a raw score s becomes cap * tanh(s * pre) (pre = scale / cap; sl2 = log2(e))
-template <int NKEYS>
+template <int NKEYS, bool CAPPED = true>
 __device__ __forceinline__ void attend_tile(const unsigned (*qf)[4], const bf16* ks, const bf16* vs,
                                             int key0, const int* row_lo, const int* row_hi,
                                             float sl2, float* m, float* l, float (*o)[4], int keep = 0,
@@ -156,7 +162,7 @@ __device__ __forceinline__ void attend_tile(const unsigned (*qf)[4], const bf16*
     }
   }
   // Capped scores: s <- cap * tanh(s * pre) with pre = scale / cap; the caller's sl2 is then log2(e) alone.
-  if (cap > 0.f) {
+  if (CAPPED && cap > 0.f) {
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
@@ -538,7 +544,7 @@ struct FusedQK {
   long long num_slots;
 };
 
-template <int WARPS, int RING>
+template <int WARPS, int RING, bool CAPPED>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pages,
                         const int* __restrict__ block_table, const int* __restrict__ cu_seqlens,
@@ -604,6 +610,7 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
     const int listed = warp + tile * WARPS;
     return listed < kept_tiles ? listed : lo / DECODE_BN + listed - kept_tiles;
   };
+  const uint64_t policy = omnia_read_once_policy();
   // A tile's loads: lane l looks up the row of key l once; then the warp copies the tile in
   // flat order (consecutive lanes take consecutive 16-byte chunks of a row, so every
   // request covers whole 128-byte lines), fetching each row's address by shuffle.
@@ -620,8 +627,8 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
       const int key = flat / CH, c = flat % CH;
       const bf16* kp = reinterpret_cast<const bf16*>(
           __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(mine), key));
-      cp_async16(kt + key * ROW + c * 8, kp ? kp + c * 8 : pages, kp != nullptr);
-      cp_async16(vt + key * ROW + c * 8, kp ? kp + v_offset + c * 8 : pages, kp != nullptr);
+      cp_async16(kt + key * ROW + c * 8, kp ? kp + c * 8 : pages, kp != nullptr, policy);
+      cp_async16(vt + key * ROW + c * 8, kp ? kp + v_offset + c * 8 : pages, kp != nullptr, policy);
     }
   };
   // In flight before the loop: all stages but one of a lone warp's ring (the last is asked for at the
@@ -759,8 +766,8 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
     row_lo[r] = lo;
     row_hi[r] = row < GROUP ? hi : -1;
   }
-  const float sl2 = softcap > 0.f ? LOG2E : scale * LOG2E;
-  const float pre = softcap > 0.f ? scale / softcap : 0.f;
+  const float sl2 = CAPPED && softcap > 0.f ? LOG2E : scale * LOG2E;
+  const float pre = CAPPED && softcap > 0.f ? scale / softcap : 0.f;
 
   for (int tile = 0; tile < tiles; ++tile) {
     if (FILLED) {
@@ -784,14 +791,12 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
       }
       __syncwarp();
     }
-    if (warp + tile * WARPS < kept_tiles) {
-      const int all[2] = {0, 0}, below[2] = {min(row_hi[0], kept - 1), min(row_hi[1], kept - 1)};
-      attend_tile<DECODE_BN>(qf, kt, kt + DECODE_BN * ROW, tile_of(tile) * DECODE_BN, all, below, sl2, m, l, o, 0, 0,
-                             softcap, pre);
-    } else {
-      attend_tile<DECODE_BN>(qf, kt, kt + DECODE_BN * ROW, tile_of(tile) * DECODE_BN, row_lo, row_hi, sl2, m, l, o, 0, 0,
-                             softcap, pre);
-    }
+    // A tile of kept positions sees those alone, whatever the window says.
+    const bool of_kept = warp + tile * WARPS < kept_tiles;
+    const int see_lo[2] = {of_kept ? 0 : row_lo[0], of_kept ? 0 : row_lo[1]};
+    const int see_hi[2] = {of_kept ? min(row_hi[0], kept - 1) : row_hi[0], of_kept ? min(row_hi[1], kept - 1) : row_hi[1]};
+    attend_tile<DECODE_BN, CAPPED>(qf, kt, kt + DECODE_BN * ROW, tile_of(tile) * DECODE_BN, see_lo, see_hi, sl2, m, l, o, 0, 0,
+                                   softcap, pre);
     __syncwarp();
     if (STAGES == 1) {  // the one stage is free again
       if (tile + 1 < tiles) load_tile(tile + 1, 0);
@@ -938,6 +943,10 @@ extern "C" int omnia_attention_prefill_tc(const void* q, const void* pages, cons
   return OMNIA_LAUNCH_RESULT();
 }
 
+typedef void (*DecodeKernel)(const bf16*, const bf16*, const int*, const int*, const int*, const int*, float*, float*, int*, const bf16*,
+                             int, bf16*, int, int, int, int, int, int, int, int, float, const FusedQK, int, const float*, int, float,
+                             const MapDifference, int, int*);
+
 // Shared memory of an SM, the most a block may ask for, and what a block costs beside its dynamic
 // part (the system's kilobyte and the kernel's static arrays). Both decode entry points allow the
 // kernels the same dynamic size, so neither undoes the other's setting.
@@ -983,15 +992,13 @@ extern "C" int omnia_attention_decode_tc(const void* q, const void* pages, const
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess || device < 0 || device >= 64) return (int)cudaErrorInvalidDevice;
   if (!configured[device]) {
-    cudaError_t e = cudaFuncSetAttribute(attention_decode_kernel<1, DECODE_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(BLOCK_MOST - BLOCK_OVERHEAD));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attention_decode_kernel<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(BLOCK_MOST - BLOCK_OVERHEAD));
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attention_decode_kernel<4, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(BLOCK_MOST - BLOCK_OVERHEAD));
-    if (e != cudaSuccess) return (int)e;
+    const DecodeKernel all[] = {attention_decode_kernel<1, DECODE_STAGES, false>, attention_decode_kernel<1, DECODE_STAGES, true>,
+                                attention_decode_kernel<4, 1, false>, attention_decode_kernel<4, 1, true>,
+                                attention_decode_kernel<4, 2, false>, attention_decode_kernel<4, 2, true>};
+    for (DecodeKernel kernel : all) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(BLOCK_MOST - BLOCK_OVERHEAD));
+      if (e != cudaSuccess) return (int)e;
+    }
     configured[device] = true;
   }
   if (spread) {
@@ -1004,21 +1011,17 @@ extern "C" int omnia_attention_decode_tc(const void* q, const void* pages, const
     const size_t room = SM_SHARED / (size_t)share;
     if (room > smem + BLOCK_OVERHEAD) smem = (room > BLOCK_MOST ? BLOCK_MOST : room) - BLOCK_OVERHEAD;
   }
-  if (warps == 1)
-    launch_pdl(attention_decode_kernel<1, DECODE_STAGES>, dim3(max_chunks, nkv, requests), 32, smem, stream,
-        (const bf16*)q, (const bf16*)pages, block_table, cu_seqlens, seq_lens, seq_ids, part_o, part_ml,
-        tickets, (const bf16*)gate, gate_stride, (bf16*)out, chunk_keys, max_chunks, max_pages,
-        num_pages, nq, nkv, page_size, window, scale, fused, keep_first, sink, run, softcap, difference, beside, err);
-  else if (deep)
-    launch_pdl(attention_decode_kernel<4, 2>, dim3(max_chunks, nkv, requests), 128, smem, stream,
-        (const bf16*)q, (const bf16*)pages, block_table, cu_seqlens, seq_lens, seq_ids, part_o, part_ml,
-        tickets, (const bf16*)gate, gate_stride, (bf16*)out, chunk_keys, max_chunks, max_pages,
-        num_pages, nq, nkv, page_size, window, scale, fused, keep_first, sink, run, softcap, difference, beside, err);
-  else
-    launch_pdl(attention_decode_kernel<4, 1>, dim3(max_chunks, nkv, requests), 128, smem, stream,
-        (const bf16*)q, (const bf16*)pages, block_table, cu_seqlens, seq_lens, seq_ids, part_o, part_ml,
-        tickets, (const bf16*)gate, gate_stride, (bf16*)out, chunk_keys, max_chunks, max_pages,
-        num_pages, nq, nkv, page_size, window, scale, fused, keep_first, sink, run, softcap, difference, beside, err);
+  // Scores without a cap take kernels without its tanh: 16 of them stand in a tile's straight line of code, and a decode
+  // step fetches every kernel's code anew (a layer's weights have pushed it out of the caches).
+  const DecodeKernel kernel =
+      softcap > 0.f ? (warps == 1 ? attention_decode_kernel<1, DECODE_STAGES, true>
+                                  : deep ? attention_decode_kernel<4, 2, true> : attention_decode_kernel<4, 1, true>)
+                    : (warps == 1 ? attention_decode_kernel<1, DECODE_STAGES, false>
+                                  : deep ? attention_decode_kernel<4, 2, false> : attention_decode_kernel<4, 1, false>);
+  launch_pdl(kernel, dim3(max_chunks, nkv, requests), warps * 32, smem, stream,
+      (const bf16*)q, (const bf16*)pages, block_table, cu_seqlens, seq_lens, seq_ids, part_o, part_ml,
+      tickets, (const bf16*)gate, gate_stride, (bf16*)out, chunk_keys, max_chunks, max_pages,
+      num_pages, nq, nkv, page_size, window, scale, fused, keep_first, sink, run, softcap, difference, beside, err);
   return OMNIA_LAUNCH_RESULT();
 }
 
@@ -1090,7 +1093,7 @@ extern "C" int omnia_attention_decode_tc_static(const void* q, const void* pages
       snprintf(static_error, sizeof static_error, "cudaGetSymbolAddress: %s", cudaGetErrorString(e));
       return (int)e;
     }
-    e = cudaFuncSetAttribute(attention_decode_kernel<1, DECODE_STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(attention_decode_kernel<1, DECODE_STAGES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)(BLOCK_MOST - BLOCK_OVERHEAD));
     if (e != cudaSuccess) {
       snprintf(static_error, sizeof static_error, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
@@ -1109,7 +1112,7 @@ extern "C" int omnia_attention_decode_tc_static(const void* q, const void* pages
     return (int)e;
   }
   const size_t smem = (size_t)(DECODE_STAGES * 2 * DECODE_BN) * ROW * sizeof(bf16);
-  launch_pdl(attention_decode_kernel<1, DECODE_STAGES>, dim3(max_chunks, nkv, requests), 32, smem, stream,
+  launch_pdl(attention_decode_kernel<1, DECODE_STAGES, false>, dim3(max_chunks, nkv, requests), 32, smem, stream,
       (const bf16*)q, (const bf16*)pages, block_table, cu_seqlens, seq_lens, seq_ids, part_o, part_ml,
       ticket_area, (const bf16*)gate, gate_stride, (bf16*)out, chunk_keys, max_chunks, max_pages,
       num_pages, nq, nkv, page_size, window, scale, FusedQK{}, 0, nullptr, 0, 0.f, MapDifference{}, 0, err);

@@ -134,6 +134,14 @@ __device__ __forceinline__ bool omnia_elect_one() {
 // The number of this thread's warp, as a value the compiler knows to be the same in all of its lanes.
 __device__ __forceinline__ int omnia_warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 
+// The cache policy of what is read once a step, a product's weights and the cache's keys and values: such lines leave L2
+// first, so that a step's stream of gigabytes does not push out what the next layer needs again.
+__device__ __forceinline__ uint64_t omnia_read_once_policy() {
+  uint64_t policy;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
+  return policy;
+}
+
 // Programmatic dependent launch. A kernel launched through launch_pdl may begin while the kernel
 // before it in the stream is still running; it must call pdl_wait() before it touches anything an
 // earlier kernel wrote (reading weights before that is fine and hides their latency), and calls

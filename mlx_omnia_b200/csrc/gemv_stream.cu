@@ -116,10 +116,10 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
   *abort_flag = 1;
   return false;
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
+__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y, uint64_t policy) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y)
+      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(y), "l"(policy)
       : "memory");
 }
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
@@ -217,6 +217,7 @@ gemv_stream_kernel(const bf16* __restrict__ a, const __grid_constant__ CUtensorM
     // ---- producer: needs nothing from the kernel before, so it does not wait for it ----
     int s = 0, phase = 1, in_flight = 0;
     bool ok = true;
+    const uint64_t policy = omnia_read_once_policy();
     for (int first = 0, count; first < my_tiles && ok; first += count) {
       count = together(first);
       int matrix0 = 0, in_matrix = tile0 + first;  // the matrix's first row, and the tile's place in it
@@ -239,7 +240,7 @@ gemv_stream_kernel(const bf16* __restrict__ a, const __grid_constant__ CUtensorM
           const unsigned live = __ballot_sync(0xffffffffu, copies);
           if (lane == 0) mbar_expect_tx(full0 + 8 * s, (uint32_t)__popc(live) * BOX_BYTES);
           __syncwarp();
-          if (copies) tma_load_2d(smem_u32(ring + s * STAGE_BYTES + lane * BOX_BYTES), &map_w, full0 + 8 * s, x, matrix0 + y);
+          if (copies) tma_load_2d(smem_u32(ring + s * STAGE_BYTES + lane * BOX_BYTES), &map_w, full0 + 8 * s, x, matrix0 + y, policy);
           in_flight = min(in_flight + 1, STAGES);
           if (++s == STAGES) s = 0, phase ^= 1;
         }
