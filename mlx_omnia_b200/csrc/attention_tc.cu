@@ -30,6 +30,8 @@
 // attention, and what is written is their difference (see MapDifference), [tokens, nq / 2, dv].
 #include "common.cuh"
 
+#include <type_traits>
+
 #ifndef HEAD_DIM
 #define HEAD_DIM 128
 #endif
@@ -421,104 +423,132 @@ attention_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pa
   }
 }
 
-// Merge chunks c0..c1 of H heads of one token (heads head0 .., whose partials lie max_chunks apart),
-// ascending, then gate and round; run by one warp. The merge is the tail of the whole kernel and
-// nothing but memory round trips (the partials were written to L2 a moment ago by other blocks), so
-// everything a round needs is asked for before anything is used: the gates at once, then per
-// round of eight chunks the chunks' (max, sum) pairs, one chunk per lane, and the H x 8 partial
-// rows, every lane its own dims. Eight chunks or fewer are one round trip for all H heads.
-// The merge of a head's (H heads') chunks by one warp. The chunks' unnormalised accumulators lie one
-// after the other in part_o, so a batch of them is brought into shared memory (`stage`, room for
-// `stage_floats` floats: the block's ring, idle by now) with one round of 16-byte asynchronous
-// copies, all in flight together: one trip to L2 for up to 32 chunks, where reading them eight at
-// a time into registers took one trip per eight. Lane u holds chunk u's maximum and sum.
-template <int H>
-__device__ __forceinline__ void combine_heads(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                              size_t base, int max_chunks, int c0, int c1, const bf16* gate_row,
-                                              bf16* out_row, float* stage, int stage_floats,
-                                              const float* sink = nullptr, const MapDifference difference = {}) {
-  const int lane = threadIdx.x & 31;
-  constexpr int PER_LANE = (D + 31) / 32;
-  float gate_v[H][PER_LANE];
+// The merge of `chunks` chunks of H neighbouring heads of one token by a block of THREADS threads, in ascending order: weigh, add
+// up, gate, round. `base` is the first head's first partial; the heads' lie max_chunks apart. It is the tail of the whole
+// kernel and nothing but latency, so a round's loads (sixteen chunks' maxima and sums, lane u those of chunk u, the
+// thread's own dims of their accumulators, the gates) all leave together, straight into registers: one trip to L2. One warp
+// that brought them through shared memory by asynchronous copies took 5.5 us behind the last ticket of eight requests.
+template <int H, int THREADS>
+__device__ __forceinline__ void merge_chunks(const float* __restrict__ part_o, const float* __restrict__ part_ml, size_t base,
+                                             int max_chunks, int chunks, const bf16* __restrict__ gate_row, bf16* __restrict__ out_row,
+                                             float* stage, const float* __restrict__ sink, const MapDifference difference) {
+  const int lane = threadIdx.x & 31, tid = threadIdx.x;
+  constexpr int VEC = H * D >= 4 * THREADS ? 4 : 2, PIECES = H * D / VEC, V = (PIECES + THREADS - 1) / THREADS, ROUND = 16;
+  using Piece = std::conditional_t<VEC == 4, float4, float2>;
+  float acc[V][VEC], gates[V][VEC], mx[H], total[H];
 #pragma unroll
-  for (int h = 0; h < H; ++h)
+  for (int h = 0; h < H; ++h) mx[h] = -INFINITY, total[h] = 0.f;
 #pragma unroll
-    for (int k = 0; k < PER_LANE; ++k) {
-      const int dim = lane + 32 * k;
-      gate_v[h][k] = gate_row && dim < D ? __bfloat162float(gate_row[(size_t)h * D + dim]) : 0.f;
-    }
-  float acc[H][PER_LANE], mx[H], total[H];
+  for (int v = 0; v < V; ++v)
 #pragma unroll
-  for (int h = 0; h < H; ++h) {
-    mx[h] = -INFINITY, total[h] = 0.f;
-#pragma unroll
-    for (int k = 0; k < PER_LANE; ++k) acc[h][k] = 0.f;
-  }
-  const int batch = min(32, stage_floats / (H * D));  // chunks a round (at least one: a stage holds far more than H rows)
-  for (int r0 = c0; r0 <= c1; r0 += batch) {
-    const int count = min(batch, c1 - r0 + 1);
-    float mc[H], lc[H];
+    for (int e = 0; e < VEC; ++e) acc[v][e] = gates[v][e] = 0.f;
+  for (int done = 0; done < chunks; done += ROUND) {
+    const int count = min(ROUND, chunks - done);
+    float mc[H], lc[H], w[H], rescale[H];
 #pragma unroll
     for (int h = 0; h < H; ++h) {
-      const size_t slot = base + (size_t)h * max_chunks + r0;
-      const float* src = part_o + slot * D;  // `count` chunks of D floats, one after the other
-      for (int i = lane; i < count * (D / 4); i += 32) cp_async16(stage + (size_t)h * batch * D + 4 * i, src + 4 * i, true);
-      mc[h] = lane < count ? __ldcg(part_ml + (slot + lane) * 2) : -INFINITY;
-      lc[h] = lane < count ? __ldcg(part_ml + (slot + lane) * 2 + 1) : 0.f;
+      const float* ml = part_ml + (base + (size_t)h * max_chunks + done + lane) * 2;
+      mc[h] = lane < count ? __ldcg(ml) : -INFINITY;
+      lc[h] = lane < count ? __ldcg(ml + 1) : 0.f;
     }
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncwarp();
+    Piece x[V][ROUND];
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      const int at = (tid + v * THREADS) * VEC, h = H == 1 ? 0 : at / D;
+      const float* src = part_o + (base + (size_t)h * max_chunks + done) * D + (at - h * D);
+#pragma unroll
+      for (int u = 0; u < ROUND; ++u)
+        if (u < count && at < H * D) x[v][u] = __ldcg(reinterpret_cast<const Piece*>(src + (size_t)u * D));
+    }
+    if (done == 0 && gate_row != nullptr)
+#pragma unroll
+      for (int v = 0; v < V; ++v)
+#pragma unroll
+        for (int e = 0; e < VEC; ++e)
+          if ((tid + v * THREADS) * VEC < H * D) gates[v][e] = __bfloat162float(gate_row[(tid + v * THREADS) * VEC + e]);
 #pragma unroll
     for (int h = 0; h < H; ++h) {
       const float mx_new = fmaxf(mx[h], warp_max(mc[h]));
-      const float rescale = mx[h] == -INFINITY ? 0.f : exp2f(mx[h] - mx_new);
-      const float w = lane < count && mc[h] != -INFINITY ? exp2f(mc[h] - mx_new) : 0.f;
-      total[h] = total[h] * rescale + warp_sum(lc[h] * w);
+      rescale[h] = mx[h] == -INFINITY ? 0.f : exp2f(mx[h] - mx_new);
+      w[h] = lane < count && mc[h] != -INFINITY ? exp2f(mc[h] - mx_new) : 0.f;
+      total[h] = total[h] * rescale[h] + warp_sum(lc[h] * w[h]);
       mx[h] = mx_new;
+    }
 #pragma unroll
-      for (int k = 0; k < PER_LANE; ++k) acc[h][k] *= rescale;
-      const float* rows = stage + (size_t)h * batch * D;
-      for (int u = 0; u < count; ++u) {
-        const float wj = __shfl_sync(0xffffffffu, w, u);
+    for (int v = 0; v < V; ++v) {
+      const bool upper = H == 2 && (tid + v * THREADS) * VEC >= D;
+      const float r = upper ? rescale[H - 1] : rescale[0];
 #pragma unroll
-        for (int k = 0; k < PER_LANE; ++k) {
-          const int dim = lane + 32 * k;
-          if (dim < D) acc[h][k] += rows[u * D + dim] * wj;
-        }
+      for (int e = 0; e < VEC; ++e) acc[v][e] *= r;
+    }
+#pragma unroll
+    for (int u = 0; u < ROUND; ++u) {
+      const float w0 = __shfl_sync(0xffffffffu, w[0], u), w1 = H == 1 ? w0 : __shfl_sync(0xffffffffu, w[H - 1], u);
+      if (u >= count) continue;
+#pragma unroll
+      for (int v = 0; v < V; ++v) {
+        const bool upper = H == 2 && (tid + v * THREADS) * VEC >= D;
+        const float* xv = reinterpret_cast<const float*>(&x[v][u]);
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) acc[v][e] += xv[e] * (upper ? w1 : w0);
       }
     }
-    __syncwarp();  // the stage is read before the next round overwrites it
   }
+  if (sink != nullptr) {
+#pragma unroll
+    for (int h = 0; h < H; ++h)
+      if (mx[h] != -INFINITY) total[h] += exp2f(sink[h] * LOG2E - mx[h]);  // mx is in log2 units
+  }
+  const float inv0 = total[0] > 0.f ? 1.f / total[0] : 0.f, inv1 = total[H - 1] > 0.f ? 1.f / total[H - 1] : 0.f;
   if constexpr (MAPS == 2) {
+    // The two maps of a dim are different threads': both go through shared memory, the first warp takes it from there.
     static_assert(H == 2, "a head's two maps are merged together");
-    const float inv0 = total[0] > 0.f ? 1.f / total[0] : 0.f, inv1 = total[H - 1] > 0.f ? 1.f / total[H - 1] : 0.f;
-    float ss = 0.f;
+    if (THREADS > 32) __syncthreads(); else __syncwarp();  // the stage may still be read by an earlier pair's merge
 #pragma unroll
-    for (int k = 0; k < PER_LANE; ++k) {
-      acc[0][k] = acc[0][k] * inv0 - difference.lambda * (acc[H - 1][k] * inv1);
-      if (lane + 32 * k < D) ss += acc[0][k] * acc[0][k];
-    }
-    const float f = rsqrtf(warp_sum(ss) / (float)difference.dv + difference.eps) * difference.factor;
+    for (int v = 0; v < V; ++v)
 #pragma unroll
-    for (int k = 0; k < PER_LANE; ++k) {
-      const int dim = lane + 32 * k;
-      if (dim < difference.dv) out_row[dim] = __float2bfloat16_rn(acc[0][k] * f);
+      for (int e = 0; e < VEC; ++e) {
+        const int at = (tid + v * THREADS) * VEC + e;
+        if (at < H * D) stage[at] = acc[v][e] * (at < D ? inv0 : inv1);
+      }
+    if (THREADS > 32) __syncthreads(); else __syncwarp();
+    if (tid < 32) {
+      constexpr int PER_LANE = (D + 31) / 32;
+      float d[PER_LANE], ss = 0.f;
+#pragma unroll
+      for (int k = 0; k < PER_LANE; ++k) {
+        const int dim = lane + 32 * k;
+        d[k] = dim < D ? stage[dim] - difference.lambda * stage[D + dim] : 0.f;
+        ss += d[k] * d[k];
+      }
+      const float f = rsqrtf(warp_sum(ss) / (float)difference.dv + difference.eps) * difference.factor;
+#pragma unroll
+      for (int k = 0; k < PER_LANE; ++k)
+        if (lane + 32 * k < difference.dv) out_row[lane + 32 * k] = __float2bfloat16_rn(d[k] * f);
     }
   } else {
+    const bool whole = (reinterpret_cast<uintptr_t>(out_row) & (2 * VEC - 1)) == 0;
 #pragma unroll
-  for (int h = 0; h < H; ++h) {
-    if (sink != nullptr && mx[h] != -INFINITY) total[h] += exp2f(sink[h] * LOG2E - mx[h]);  // mx is in log2 units
-    const float inv = total[h] > 0.f ? 1.f / total[h] : 0.f;
+    for (int v = 0; v < V; ++v) {
+      const int at = (tid + v * THREADS) * VEC;
+      if (at >= H * D) break;
+      const float inv = at < D ? inv0 : inv1;
+      float y[VEC];
 #pragma unroll
-    for (int k = 0; k < PER_LANE; ++k) {
-      const int dim = lane + 32 * k;
-      if (dim >= D) continue;
-      float v = acc[h][k] * inv;
-      if (gate_row) v *= 1.f / (1.f + expf(-gate_v[h][k]));
-      out_row[(size_t)h * D + dim] = __float2bfloat16_rn(v);
+      for (int e = 0; e < VEC; ++e) {
+        y[e] = acc[v][e] * inv;
+        if (gate_row != nullptr) y[e] *= 1.f / (1.f + expf(-gates[v][e]));
+      }
+      if (whole) {
+        if constexpr (VEC == 4)
+          *reinterpret_cast<uint2*>(out_row + at) = make_uint2(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]));
+        else
+          *reinterpret_cast<unsigned*>(out_row + at) = pack_bf16(y[0], y[1]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) out_row[at + e] = __float2bfloat16_rn(y[e]);
+      }
     }
-  }
   }
 }
 
@@ -845,63 +875,76 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
   }
   if (WARPS > 1) {
     __syncthreads();
-    if (warp != 0) return;
-    for (int row = 0; row < GROUP; ++row) {
-      const size_t slot = (((size_t)blockIdx.z * nq + kvh * GROUP + row) * max_chunks + chunk);
-      float top = -INFINITY;
 #pragma unroll
-      for (int w = 0; w < WARPS; ++w) top = fmaxf(top, merge[((size_t)w * GROUP + row) * (D + 2) + D]);
-      float weight[WARPS], sum = 0.f;
+    for (int i0 = 0; i0 < GROUP * D; i0 += WARPS * 32) {
+      const int i = i0 + threadIdx.x;
+      if (i >= GROUP * D) break;
+      const int row = i / D, dim = i - row * D;
+      const float* src = merge + (size_t)row * (D + 2);  // the first warp's; the others' lie GROUP rows apart
+      constexpr int APART = GROUP * (D + 2);
+      float top = -INFINITY, sum = 0.f, acc = 0.f;
+#pragma unroll
+      for (int w = 0; w < WARPS; ++w) top = fmaxf(top, src[w * APART + D]);
 #pragma unroll
       for (int w = 0; w < WARPS; ++w) {
-        const float* src = merge + ((size_t)w * GROUP + row) * (D + 2);
-        weight[w] = src[D] == -INFINITY ? 0.f : exp2f(src[D] - top);
-        sum += src[D + 1] * weight[w];
+        const float weight = src[w * APART + D] == -INFINITY ? 0.f : exp2f(src[w * APART + D] - top);
+        sum += src[w * APART + D + 1] * weight;
+        acc += src[w * APART + dim] * weight;
       }
-      for (int dim = lane; dim < D; dim += 32) {
-        float acc = 0.f;
-#pragma unroll
-        for (int w = 0; w < WARPS; ++w) acc += merge[((size_t)w * GROUP + row) * (D + 2) + dim] * weight[w];
-        part_o[slot * D + dim] = acc;
-      }
-      if (lane == 0) {
+      const size_t slot = (((size_t)blockIdx.z * nq + kvh * GROUP + row) * max_chunks + chunk);
+      part_o[slot * D + dim] = acc;
+      if (dim == 0) {
         part_ml[slot * 2] = top;
         part_ml[slot * 2 + 1] = sum;
       }
     }
   }
   // Whoever finishes last merges: publish the partial, take a ticket, and if it is the last
-  // one of this (request, head group), read all partials back and write the output.
-  __threadfence();
-  __syncwarp();
+  // one of this (request, head group), read all partials back and write the output. The fences are the ticket thread's: its
+  // own and, through the barrier, the block's writes are released by the first, the other blocks' acquired by the second.
   const int c0 = first / chunk_keys, c1 = pos / chunk_keys;
-  int ticket = 0;
   int* counter = tickets + (size_t)blockIdx.z * nkv + kvh;
-  if (lane == 0) ticket = atomicAdd(counter, 1);
-  ticket = __shfl_sync(0xffffffffu, ticket, 0);
+  int ticket = 0;
+  if (WARPS == 1) {
+    __syncwarp();
+    if (lane == 0) {
+      __threadfence();
+      ticket = atomicAdd(counter, 1);
+      __threadfence();
+    }
+    ticket = __shfl_sync(0xffffffffu, ticket, 0);
+    __syncwarp();
+  } else {
+    __shared__ int drawn;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      __threadfence();
+      drawn = atomicAdd(counter, 1);
+      __threadfence();
+    }
+    __syncthreads();
+    ticket = drawn;
+  }
   OMNIA_TRACE_BLOCK(6);
   if (ticket != c1 - c0) return;
-  if (lane == 0) *counter = 0;
-  __threadfence();
   // Two heads at a time (their loads travel together; one at a time where a head's rows would not
   // fit in registers twice), then the odd one.
-  constexpr int TOGETHER = MAPS == 2 || D <= 128 ? 2 : 1;
-  // The block's rings are idle by now: the least they hold, in floats, stages the chunks' accumulators.
-  constexpr int STAGE_FLOATS = WARPS * STAGES * 2 * DECODE_BN * ROW * (int)sizeof(bf16) / (int)sizeof(float);
+  constexpr int TOGETHER = MAPS == 2 || (D <= 128 && GROUP > 1) ? 2 : 1;
 #pragma unroll 1
   for (int r = 0; r + TOGETHER <= GROUP; r += TOGETHER) {
     const int head = kvh * GROUP + r;
-    combine_heads<TOGETHER>(part_o, part_ml, ((size_t)blockIdx.z * nq + head) * max_chunks, max_chunks, c0, c1,
-                     gate ? gate + token * gate_stride + (size_t)head * D : nullptr,
-                     MAPS == 2 ? out + (token * (nq / 2) + head / 2) * difference.dv : out + (token * nq + head) * D,
-                     reinterpret_cast<float*>(smem_raw), STAGE_FLOATS, sink ? sink + head : nullptr, difference);
+    merge_chunks<TOGETHER, WARPS * 32>(part_o, part_ml, ((size_t)blockIdx.z * nq + head) * max_chunks + c0, max_chunks, c1 - c0 + 1,
+                                       gate ? gate + token * gate_stride + (size_t)head * D : nullptr,
+                                       MAPS == 2 ? out + (token * (nq / 2) + head / 2) * difference.dv : out + (token * nq + head) * D,
+                                       reinterpret_cast<float*>(smem_raw), sink ? sink + head : nullptr, difference);
   }
   if constexpr (GROUP % TOGETHER != 0) {
     const int head = kvh * GROUP + GROUP - 1;
-    combine_heads<1>(part_o, part_ml, ((size_t)blockIdx.z * nq + head) * max_chunks, max_chunks, c0, c1,
-                     gate ? gate + token * gate_stride + (size_t)head * D : nullptr, out + (token * nq + head) * D,
-                     reinterpret_cast<float*>(smem_raw), STAGE_FLOATS, sink ? sink + head : nullptr);
+    merge_chunks<1, WARPS * 32>(part_o, part_ml, ((size_t)blockIdx.z * nq + head) * max_chunks + c0, max_chunks, c1 - c0 + 1,
+                                gate ? gate + token * gate_stride + (size_t)head * D : nullptr, out + (token * nq + head) * D,
+                                reinterpret_cast<float*>(smem_raw), sink ? sink + head : nullptr, difference);
   }
+  if (threadIdx.x == 0) *counter = 0;  // for the next launch
   OMNIA_TRACE_BLOCK(7);
   if (beside) pdl_wait();
 }
