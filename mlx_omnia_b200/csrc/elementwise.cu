@@ -2,6 +2,8 @@
 // One row (token) per block unless said otherwise; float32 arithmetic throughout.
 #include "common.cuh"
 
+#include <type_traits>
+
 // ---------------------------------------------------------------------------------
 // Embedding lookup with an optional weightless RMS norm: x[t] = rms0(table[ids[t]]).
 // The residual stream x is float32 in both precisions.
@@ -594,6 +596,188 @@ qkv_prepare_kernel(const T* __restrict__ proj, int row_stride, int q_col, int k_
   }
 }
 
+// N consecutive elements as float32, by the widest loads there are for their bytes; and back, rounded once.
+template <int BYTES>
+using piece_t = std::conditional_t<BYTES == 4, unsigned, std::conditional_t<BYTES == 8, uint2, uint4>>;
+template <typename T, int N>
+__device__ __forceinline__ void load_row_piece(const T* src, float (&dst)[N]) {
+  using V = piece_t<N * (int)sizeof(T)>;
+  constexpr int EACH = (int)(sizeof(V) / sizeof(T));
+#pragma unroll
+  for (int at = 0; at < N; at += EACH) {
+    const V v = *reinterpret_cast<const V*>(src + at);
+    const T* e = reinterpret_cast<const T*>(&v);
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) dst[at + i] = to_f32(e[i]);
+  }
+}
+template <typename T, int N>
+__device__ __forceinline__ void store_row_piece(T* dst, const float (&src)[N]) {
+  using V = piece_t<N * (int)sizeof(T)>;
+  constexpr int EACH = (int)(sizeof(V) / sizeof(T));
+#pragma unroll
+  for (int at = 0; at < N; at += EACH) {
+    V v;
+    T* e = reinterpret_cast<T*>(&v);
+#pragma unroll
+    for (int i = 0; i < EACH; ++i) e[i] = from_f32<T>(src[at + i]);
+    *reinterpret_cast<V*>(dst + at) = v;
+  }
+}
+
+// The same step for keys and values of one width, 32 * PL dims, and at most 8 * HPW heads (32): a warp has up to HPW heads, a
+// lane PL neighbouring dims of each. Blocks stay and take every gridDim.x-th token: the norms' weights are read once, ahead of
+// the wait for the kernel before, and a token's rows, position and slot are asked for while the token before it is worked
+// on. The kernel above walks a warp's heads one after another, twice where the norm is over all of them, each a trip to L2
+// by 2-byte loads: that, not its bytes, is what it takes its time for.
+// A rotation's pairs are a lane's own (interleaved), or its and those of the lane rot / 2 dims further, which have to be a
+// power of two of lanes.
+template <typename T, int PL, int HPW>
+__global__ void __launch_bounds__(256, PL == 8 ? 2 : 3)
+qkv_prepare_vec_kernel(const T* __restrict__ proj, int row_stride, int q_col, int k_col, int v_col, int tokens, int nq, int nkv,
+                       const T* __restrict__ bias, const float* __restrict__ q_weight, const float* __restrict__ k_weight,
+                       float eps, const float* __restrict__ inv_freq, int rot, const int* __restrict__ positions,
+                       const long long* __restrict__ slot_mapping, T* __restrict__ q_out, T* __restrict__ k_pages,
+                       T* __restrict__ v_pages, long long page_stride, int page_size, long long num_slots, int whole,
+                       int interleaved, const T* __restrict__ other, int other_stride, float lam, int* err) {
+  constexpr int d = 32 * PL;
+  using V = piece_t<PL * (int)sizeof(T)>;
+  constexpr int PARTS = PL * (int)sizeof(T) / (int)sizeof(V);
+  __shared__ float cos_s[2][d / 2], sin_s[2][d / 2], head_ss[2][32];  // two tokens' in turn: one barrier a token
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rhalf = inv_freq != nullptr ? rot / 2 : 0, normed = nq + nkv, heads = normed + nkv;
+  auto column = [&](int hs) { return (hs < nq ? q_col + hs * d : hs < normed ? k_col + (hs - nq) * d : v_col + (hs - normed) * d) + lane * PL; };
+  float w[HPW][PL];
+#pragma unroll
+  for (int j = 0; j < HPW; ++j) {
+    const int hs = warp + 8 * j;
+    const float* weight = hs < nq ? q_weight : k_weight;
+#pragma unroll
+    for (int e = 0; e < PL; ++e) w[j][e] = 1.f;
+    if (hs < normed && eps >= 0.f && weight != nullptr)
+      load_row_piece<float, PL>(weight + (whole ? (hs < nq ? hs : hs - nq) * d : 0) + lane * PL, w[j]);
+  }
+  const float freq = (int)threadIdx.x < rhalf ? inv_freq[threadIdx.x] : 0.f;
+  pdl_wait();
+  pdl_launch_dependents();
+  V next[HPW][PARTS];
+  int next_pos = 0;
+  long long next_slot = -1;
+  auto ask = [&](int t) {
+    if (t >= tokens) return;
+#pragma unroll
+    for (int j = 0; j < HPW; ++j)
+      if (warp + 8 * j < heads) {
+        const V* src = reinterpret_cast<const V*>(proj + (size_t)t * row_stride + column(warp + 8 * j));
+#pragma unroll
+        for (int part = 0; part < PARTS; ++part) next[j][part] = src[part];
+      }
+    if ((int)threadIdx.x < rhalf) next_pos = positions[t];
+    if (slot_mapping != nullptr) next_slot = slot_mapping[t];
+  };
+  ask(blockIdx.x);
+  int turn = 0;
+  for (int t = blockIdx.x; t < tokens; t += gridDim.x, turn ^= 1) {
+    float a[HPW][PL];
+#pragma unroll
+    for (int j = 0; j < HPW; ++j)
+#pragma unroll
+      for (int e = 0; e < PL; ++e)
+        a[j][e] = warp + 8 * j < heads ? to_f32(reinterpret_cast<const T*>(&next[j][e * sizeof(T) / sizeof(V)])[e % (sizeof(V) / sizeof(T))]) : 0.f;
+    const int pos = next_pos;
+    const long long slot = next_slot;
+    ask(t + gridDim.x);
+    if ((int)threadIdx.x < rhalf) sincosf((float)pos * freq, &sin_s[turn][threadIdx.x], &cos_s[turn][threadIdx.x]);
+    if (nkv > 0 && slot >= num_slots && threadIdx.x == 0) atomicOr(err, OMNIA_ERR_SLOT);
+    float scale[HPW];
+#pragma unroll
+    for (int j = 0; j < HPW; ++j) {
+      const int hs = warp + 8 * j;
+      if (bias != nullptr && hs < heads) {
+        float b[PL];
+        load_row_piece<T, PL>(bias + column(hs), b);
+#pragma unroll
+        for (int e = 0; e < PL; ++e) a[j][e] += b[e];
+      }
+      float ss = 0.f;
+#pragma unroll
+      for (int e = 0; e < PL; ++e) ss += a[j][e] * a[j][e];
+      ss = warp_sum(ss);
+      scale[j] = eps < 0.f ? 1.f : rsqrtf(ss / (float)d + eps);
+      if (whole && lane == 0 && hs < normed) head_ss[turn][hs] = ss;
+    }
+    __syncthreads();
+    if (whole && eps >= 0.f) {  // one root mean square over all heads of q, one over all heads of k
+      const float ss = lane < normed ? head_ss[turn][lane] : 0.f;
+      const float sq = warp_sum(lane < nq ? ss : 0.f), sk = warp_sum(lane < nq ? 0.f : ss);
+      const float scale_q = rsqrtf(sq / (float)(nq * d) + eps), scale_k = nkv > 0 ? rsqrtf(sk / (float)(nkv * d) + eps) : 1.f;
+#pragma unroll
+      for (int j = 0; j < HPW; ++j) scale[j] = warp + 8 * j < nq ? scale_q : scale_k;
+    }
+    const bool stored = slot >= 0 && slot < num_slots;
+    const long long page = stored ? slot / page_size : 0, off = stored ? slot - page * page_size : 0;
+    const int apart = rhalf / PL;  // lanes to a rotation's other half
+#pragma unroll
+    for (int j = 0; j < HPW; ++j) {
+      const int hs = warp + 8 * j;
+      if (hs >= heads || (hs >= nq && !stored)) break;
+      T* dst = hs < nq ? q_out + ((size_t)t * nq + hs) * d
+                       : (hs < normed ? k_pages : v_pages) + page * page_stride + ((long long)(hs < normed ? hs - nq : hs - normed) * page_size + off) * d;
+      if (hs >= normed) {
+        if (other != nullptr) {  // the token's values of another layer mixed in
+          float o[PL];
+          load_row_piece<T, PL>(other + (size_t)t * other_stride + (hs - normed) * d + lane * PL, o);
+#pragma unroll
+          for (int e = 0; e < PL; ++e) a[j][e] = (1.f - lam) * a[j][e] + lam * o[e];
+        }
+        store_row_piece<T, PL>(dst + lane * PL, a[j]);
+        continue;
+      }
+      if (eps >= 0.f) {
+#pragma unroll
+        for (int e = 0; e < PL; ++e) a[j][e] = a[j][e] * scale[j] * w[j][e];
+      }
+      if (rhalf > 0) {
+        if (interleaved) {
+#pragma unroll
+          for (int e = 0; e < PL; e += 2) {
+            const int i = (lane * PL + e) / 2;
+            if (i >= rhalf) break;
+            const float c = cos_s[turn][i], sn = sin_s[turn][i], a0 = a[j][e], a1 = a[j][e + 1];
+            a[j][e] = a0 * c - a1 * sn;
+            a[j][e + 1] = a1 * c + a0 * sn;
+          }
+        } else {
+          const bool lower = lane < apart, turns = lane < 2 * apart;
+#pragma unroll
+          for (int e = 0; e < PL; ++e) {
+            const float partner = __shfl_xor_sync(0xffffffffu, a[j][e], apart);
+            if (!turns) continue;
+            const int i = (lower ? lane : lane - apart) * PL + e;
+            const float c = cos_s[turn][i], sn = sin_s[turn][i];
+            a[j][e] = lower ? a[j][e] * c - partner * sn : a[j][e] * c + partner * sn;
+          }
+        }
+      }
+      store_row_piece<T, PL>(dst + lane * PL, a[j]);
+    }
+  }
+}
+
+template <typename T, int PL>
+void launch_qkv_prepare_vec(int heads, int tokens, cudaStream_t stream, const T* proj, int row_stride, int q_col, int k_col,
+                            int v_col, int nq, int nkv, const T* bias, const float* q_weight, const float* k_weight, float eps,
+                            const float* inv_freq, int rot, const int* positions, const long long* slot_mapping, T* q_out,
+                            T* k_pages, T* v_pages, long long page_stride, int page_size, long long num_slots, int whole,
+                            int interleaved, const T* other, int other_stride, float lam, int* err) {
+  const auto kernel = heads <= 8 ? qkv_prepare_vec_kernel<T, PL, 1> : heads <= 16 ? qkv_prepare_vec_kernel<T, PL, 2>
+                    : heads <= 24 ? qkv_prepare_vec_kernel<T, PL, 3> : qkv_prepare_vec_kernel<T, PL, 4>;
+  const int places = (PL == 8 ? 2 : 3) * omnia_sm_count();  // as many blocks an SM as the kernel's registers are bounded for
+  launch_pdl(kernel, tokens < places ? tokens : places, 256, 0, stream, proj, row_stride, q_col, k_col, v_col, tokens, nq, nkv, bias, q_weight,
+             k_weight, eps, inv_freq, rot, positions, slot_mapping, q_out, k_pages, v_pages, page_stride, page_size, num_slots, whole,
+             interleaved, other, other_stride, lam, err);
+}
+
 extern "C" int omnia_qkv_prepare(const void* proj, int row_stride, int q_col, int k_col, int v_col, int nq, int nkv,
                                  int dk, int dv, const void* bias, const float* q_weight, const float* k_weight,
                                  float eps, const float* inv_freq, int rot, const int* positions,
@@ -605,6 +789,22 @@ extern "C" int omnia_qkv_prepare(const void* proj, int row_stride, int q_col, in
   if (dk > 256 || dv > 256 || rot > dk || (rot & 1) || (whole && nq + nkv > QKV_PREPARE_MAX_NORMED))
     return (int)cudaErrorInvalidValue;
   const int heads = nq + 2 * nkv;
+  // Keys and values of 64, 128 or 256 dims, at most 32 heads, everything on 16 bytes, and a half-split rotation whose halves
+  // are a power of two of a lane's dims: a lane's piece of a head then is one load, and its partner one exchange away.
+  const int piece = dk / 32, apart = rot / 2 / (piece > 0 ? piece : 1);
+  const uintptr_t starts = (uintptr_t)proj | (uintptr_t)bias | (uintptr_t)q_weight | (uintptr_t)k_weight | (uintptr_t)q_out |
+                           (uintptr_t)k_pages | (uintptr_t)v_pages | (uintptr_t)other;
+  const bool turns = inv_freq == nullptr || rot == 0 || interleaved || (piece > 0 && rot / 2 % piece == 0 && (apart & (apart - 1)) == 0);
+  if (dk == dv && (dk == 64 || dk == 128 || dk == 256) && heads <= 32 && turns && (starts & 15) == 0 &&
+      ((row_stride | q_col | k_col | v_col | other_stride) & 7) == 0 && (page_stride & 7) == 0) {
+    OMNIA_DISPATCH_DTYPE(dtype, {
+      const auto launch = dk == 64 ? launch_qkv_prepare_vec<T, 2> : dk == 128 ? launch_qkv_prepare_vec<T, 4> : launch_qkv_prepare_vec<T, 8>;
+      launch(heads, tokens, stream, (const T*)proj, row_stride, q_col, k_col, v_col, nq, nkv, (const T*)bias, q_weight, k_weight, eps,
+             inv_freq, rot, positions, slot_mapping, (T*)q_out, (T*)k_pages, (T*)v_pages, page_stride, page_size, num_slots, whole,
+             interleaved, (const T*)other, other_stride, lam, err);
+    });
+    return OMNIA_LAUNCH_RESULT();
+  }
   const int threads = heads >= 8 ? 256 : heads >= 4 ? 128 : 64;
   OMNIA_DISPATCH_DTYPE(dtype, (launch_pdl(qkv_prepare_kernel<T>, tokens, threads, 0, stream, (const T*)proj, row_stride, q_col,
                                           k_col, v_col, nq, nkv, dk, dv, (const T*)bias, q_weight, k_weight, eps,
