@@ -574,6 +574,13 @@ struct FusedQK {
   long long num_slots;
 };
 
+// A piece of a request's keys, as the list that omnia_decode_pieces (elementwise.cu) makes of a step holds it: request of
+// the call (-1: none), its position, the piece's first and last key, its number among the request's pieces and how many
+// these are, and the pieces listed ahead of the request's first.
+struct __align__(16) Piece {
+  int request, pos, lo, hi, index, count, before, unused;
+};
+
 template <int WARPS, int RING, bool CAPPED>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pages,
@@ -581,7 +588,7 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
                         const int* __restrict__ seq_lens, const int* __restrict__ seq_ids,
                         float* __restrict__ part_o, float* __restrict__ part_ml,
                         int* __restrict__ tickets, const bf16* __restrict__ gate, int gate_stride,
-                        bf16* __restrict__ out, int chunk_keys, int max_chunks, int max_pages,
+                        bf16* __restrict__ out, int chunk_keys, int max_chunks, const Piece* __restrict__ list, int pieces, int listed_before, int max_pages,
                         int num_pages, int nq, int nkv, int page_size, int window, float scale,
                         const FusedQK fused, int keep_first, const float* __restrict__ sink, int run, float softcap,
                         const MapDifference difference, int beside, int* err) {
@@ -603,19 +610,42 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   bf16* kv = reinterpret_cast<bf16*>(smem_raw) + warp * STAGES * 2 * DECODE_BN * ROW;  // STAGES x (K [32][ROW], V [32][ROW])
-  const int seq = seq_ids ? seq_ids[blockIdx.z] : blockIdx.z;
-  const int kvh = blockIdx.y, chunk = blockIdx.x;
-  const int pos = seq_lens[seq] - 1;
-  int first = window > 0 ? max(0, pos - window + 1) : 0;
-  if (run > 0 && pos >= 0) first = max(first, pos - pos % run);
-  const int lo = max(first, chunk * chunk_keys), hi = min(pos, (chunk + 1) * chunk_keys - 1);
-  if (pos < 0 || lo > hi) {
-    if (early || (beside && pos < 0)) pdl_wait();
-    return;
+  auto first_key = [&](int pos) {  // the first key that the query at `pos` sees (kept first positions aside)
+    int first = window > 0 ? max(0, pos - window + 1) : 0;
+    if (run > 0 && pos >= 0) first = max(first, pos - pos % run);
+    return first;
+  };
+  // What this block does: request `request` of the call, which is request `seq` of the step; keys lo..hi, the `chunk`th of
+  // the request's `chunks` runs of keys, whose partials lie one after the other.
+  int request = blockIdx.z, kvh = blockIdx.y, chunk = blockIdx.x, chunks = 0, seq = 0, pos = -1, first = 0, lo = 0, hi = -1;
+  if (WARPS == 1 && pieces > 0) {
+    if (listed_before) pdl_wait();  // the list comes from the kernel right before this one
+    const Piece mine = list[blockIdx.y];
+    if (mine.request < 0) {
+      if (early) pdl_wait();
+      return;
+    }
+    request = seq = mine.request, kvh = blockIdx.x, chunk = mine.index, chunks = mine.count;
+    pos = mine.pos, lo = mine.lo, hi = mine.hi;
+    first = first_key(pos);
+    max_chunks = pieces;
+    part_o += (size_t)mine.before * D, part_ml += (size_t)mine.before * 2;  // the heads' partials lie `pieces` apart
+  } else {
+    seq = seq_ids ? seq_ids[request] : request;
+    pos = seq_lens[seq] - 1;
+    first = first_key(pos);
+    lo = max(first, chunk * chunk_keys), hi = min(pos, (chunk + 1) * chunk_keys - 1);
+    if (pos < 0 || lo > hi) {
+      if (early || (beside && pos < 0)) pdl_wait();
+      return;
+    }
+    const int c0 = first / chunk_keys;
+    chunk -= c0, chunks = pos / chunk_keys - c0 + 1;
+    part_o += (size_t)request * nq * max_chunks * D, part_ml += (size_t)request * nq * max_chunks * 2;
   }
   // The chunk that holds the window's first key also takes the kept first positions below the
   // window: their tiles come ahead of the chunk's own in the list the warps share out.
-  const int kept = chunk == first / chunk_keys ? min(keep_first, first) : 0;
+  const int kept = chunk == 0 ? min(keep_first, first) : 0;
   const int kept_tiles = (kept + DECODE_BN - 1) / DECODE_BN;
   const size_t token = (size_t)cu_seqlens[seq];
   // The chunk's block-table entries are read once, up front: a tile's loads then never wait
@@ -854,7 +884,7 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
   for (int r = 0; r < 2; ++r) {
     const int row = (lane >> 2) + 8 * r;
     if (row >= GROUP) continue;
-    const size_t slot = (((size_t)blockIdx.z * nq + kvh * GROUP + row) * max_chunks + chunk);
+    const size_t slot = (size_t)(kvh * GROUP + row) * max_chunks + chunk;
     float* dst = WARPS == 1 ? part_o + slot * D : merge + ((size_t)warp * GROUP + row) * (D + 2);
 #pragma unroll
     for (int j = 0; j < NT_O; ++j) {
@@ -891,7 +921,7 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
         sum += src[w * APART + D + 1] * weight;
         acc += src[w * APART + dim] * weight;
       }
-      const size_t slot = (((size_t)blockIdx.z * nq + kvh * GROUP + row) * max_chunks + chunk);
+      const size_t slot = (size_t)(kvh * GROUP + row) * max_chunks + chunk;
       part_o[slot * D + dim] = acc;
       if (dim == 0) {
         part_ml[slot * 2] = top;
@@ -902,8 +932,7 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
   // Whoever finishes last merges: publish the partial, take a ticket, and if it is the last
   // one of this (request, head group), read all partials back and write the output. The fences are the ticket thread's: its
   // own and, through the barrier, the block's writes are released by the first, the other blocks' acquired by the second.
-  const int c0 = first / chunk_keys, c1 = pos / chunk_keys;
-  int* counter = tickets + (size_t)blockIdx.z * nkv + kvh;
+  int* counter = tickets + (size_t)request * nkv + kvh;
   int ticket = 0;
   if (WARPS == 1) {
     __syncwarp();
@@ -926,21 +955,21 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
     ticket = drawn;
   }
   OMNIA_TRACE_BLOCK(6);
-  if (ticket != c1 - c0) return;
+  if (ticket != chunks - 1) return;
   // Two heads at a time (their loads travel together; one at a time where a head's rows would not
   // fit in registers twice), then the odd one.
   constexpr int TOGETHER = MAPS == 2 || (D <= 128 && GROUP > 1) ? 2 : 1;
 #pragma unroll 1
   for (int r = 0; r + TOGETHER <= GROUP; r += TOGETHER) {
     const int head = kvh * GROUP + r;
-    merge_chunks<TOGETHER, WARPS * 32>(part_o, part_ml, ((size_t)blockIdx.z * nq + head) * max_chunks + c0, max_chunks, c1 - c0 + 1,
+    merge_chunks<TOGETHER, WARPS * 32>(part_o, part_ml, (size_t)head * max_chunks, max_chunks, chunks,
                                        gate ? gate + token * gate_stride + (size_t)head * D : nullptr,
                                        MAPS == 2 ? out + (token * (nq / 2) + head / 2) * difference.dv : out + (token * nq + head) * D,
                                        reinterpret_cast<float*>(smem_raw), sink ? sink + head : nullptr, difference);
   }
   if constexpr (GROUP % TOGETHER != 0) {
     const int head = kvh * GROUP + GROUP - 1;
-    merge_chunks<1, WARPS * 32>(part_o, part_ml, ((size_t)blockIdx.z * nq + head) * max_chunks + c0, max_chunks, c1 - c0 + 1,
+    merge_chunks<1, WARPS * 32>(part_o, part_ml, (size_t)head * max_chunks, max_chunks, chunks,
                                 gate ? gate + token * gate_stride + (size_t)head * D : nullptr, out + (token * nq + head) * D,
                                 reinterpret_cast<float*>(smem_raw), sink ? sink + head : nullptr, difference);
   }
@@ -987,7 +1016,7 @@ extern "C" int omnia_attention_prefill_tc(const void* q, const void* pages, cons
 }
 
 typedef void (*DecodeKernel)(const bf16*, const bf16*, const int*, const int*, const int*, const int*, float*, float*, int*, const bf16*,
-                             int, bf16*, int, int, int, int, int, int, int, int, float, const FusedQK, int, const float*, int, float,
+                             int, bf16*, int, int, const Piece*, int, int, int, int, int, int, int, int, float, const FusedQK, int, const float*, int, float,
                              const MapDifference, int, int*);
 
 // Shared memory of an SM, the most a block may ask for, and what a block costs beside its dynamic
@@ -998,7 +1027,10 @@ constexpr size_t SM_SHARED = 228 * 1024, BLOCK_MOST = 227 * 1024, BLOCK_OVERHEAD
 // proj non-null selects the fused mode: the kernel first does the step's QK-norm (eps < 0: none),
 // rotation (inv_freq: head_dim / 2 inverse frequencies, or null) and cache write from the
 // projected rows [tokens, stride] with q, k, v heads at q_col, k_col, v_col, and q is not read.
-// It needs a head size that is a multiple of 32. beside != 0: the launch before this one on the stream is the
+// It needs a head size that is a multiple of 32. pieces > 0: instead of chunks of chunk_keys at fixed positions the
+// pieces of `list` (omnia_decode_pieces), a place of the list a block and head; scratch is then that of one request of `pieces`
+// chunks, tickets are as ever; one warp a block, all of a step's requests. listed_before: the launch before this one made
+// the list. beside != 0: the launch before this one on the stream is the
 // attention of the same step's other entries (a prefill kernel of this package); not in the fused mode.
 extern "C" int omnia_attention_decode_tc(const void* q, const void* pages, const int* block_table,
                                          const int* cu_seqlens, const int* seq_lens,
@@ -1009,7 +1041,7 @@ extern "C" int omnia_attention_decode_tc(const void* q, const void* pages, const
                                          int page_size, int window, float scale, int warps,
                                          const void* proj, int proj_stride, int q_col, int k_col, int v_col,
                                          float eps, const float* inv_freq, const long long* slot_mapping,
-                                         int spread, int keep_first, const float* sink, int run, float softcap,
+                                         int spread, const void* list, int pieces, int listed_before, int keep_first, const float* sink, int run, float softcap,
                                          float lambda, float diff_eps, float diff_factor, int out_dv,
                                          int beside, int* err, cudaStream_t stream) {
   if (requests == 0) return 0;
@@ -1019,6 +1051,8 @@ extern "C" int omnia_attention_decode_tc(const void* q, const void* pages, const
   if (run < 0 || softcap < 0.f || (run > 0 && keep_first > 0)) return (int)cudaErrorInvalidValue;
   if (requests < 0 || nkv < 1 || nq != nkv * GROUP || chunk_keys <= 0 || chunk_keys % DECODE_BN != 0 ||
       max_chunks < 1 || max_pages < 1 || num_pages < 1 || page_size < 1 || (warps != 1 && warps != 4))
+    return (int)cudaErrorInvalidValue;
+  if (pieces != 0 && (pieces < 0 || pieces > 65535 || warps != 1 || list == nullptr || seq_ids != nullptr || beside))
     return (int)cudaErrorInvalidValue;
   if (proj != nullptr && (beside || D % 32 != 0 || slot_mapping == nullptr || proj_stride % 2 || q_col % 2 || k_col % 2 || v_col % 2))
     return (int)cudaErrorInvalidValue;
@@ -1049,7 +1083,7 @@ extern "C" int omnia_attention_decode_tc(const void* q, const void* pages, const
     // before this one frees its SMs one after the other: left alone, six blocks each go to the first
     // SMs (seen: 512 blocks on 86 of 148 SMs) and the rest of the GPU idles. So every block asks
     // for so much shared memory that an SM holds no more than its share of the grid.
-    const long long blocks = (long long)max_chunks * nkv * requests;
+    const long long blocks = pieces > 0 ? (long long)pieces * nkv : (long long)max_chunks * nkv * requests;
     const long long share = (blocks + sms - 1) / sms;
     const size_t room = SM_SHARED / (size_t)share;
     if (room > smem + BLOCK_OVERHEAD) smem = (room > BLOCK_MOST ? BLOCK_MOST : room) - BLOCK_OVERHEAD;
@@ -1061,9 +1095,9 @@ extern "C" int omnia_attention_decode_tc(const void* q, const void* pages, const
                                   : deep ? attention_decode_kernel<4, 2, true> : attention_decode_kernel<4, 1, true>)
                     : (warps == 1 ? attention_decode_kernel<1, DECODE_STAGES, false>
                                   : deep ? attention_decode_kernel<4, 2, false> : attention_decode_kernel<4, 1, false>);
-  launch_pdl(kernel, dim3(max_chunks, nkv, requests), warps * 32, smem, stream,
+  launch_pdl(kernel, pieces > 0 ? dim3(nkv, pieces) : dim3(max_chunks, nkv, requests), warps * 32, smem, stream,
       (const bf16*)q, (const bf16*)pages, block_table, cu_seqlens, seq_lens, seq_ids, part_o, part_ml,
-      tickets, (const bf16*)gate, gate_stride, (bf16*)out, chunk_keys, max_chunks, max_pages,
+      tickets, (const bf16*)gate, gate_stride, (bf16*)out, chunk_keys, max_chunks, (const Piece*)list, pieces, listed_before, max_pages,
       num_pages, nq, nkv, page_size, window, scale, fused, keep_first, sink, run, softcap, difference, beside, err);
   return OMNIA_LAUNCH_RESULT();
 }
@@ -1157,7 +1191,7 @@ extern "C" int omnia_attention_decode_tc_static(const void* q, const void* pages
   const size_t smem = (size_t)(DECODE_STAGES * 2 * DECODE_BN) * ROW * sizeof(bf16);
   launch_pdl(attention_decode_kernel<1, DECODE_STAGES, false>, dim3(max_chunks, nkv, requests), 32, smem, stream,
       (const bf16*)q, (const bf16*)pages, block_table, cu_seqlens, seq_lens, seq_ids, part_o, part_ml,
-      ticket_area, (const bf16*)gate, gate_stride, (bf16*)out, chunk_keys, max_chunks, max_pages,
+      ticket_area, (const bf16*)gate, gate_stride, (bf16*)out, chunk_keys, max_chunks, nullptr, 0, 0, max_pages,
       num_pages, nq, nkv, page_size, window, scale, FusedQK{}, 0, nullptr, 0, 0.f, MapDifference{}, 0, err);
   e = cudaGetLastError();
   if (e != cudaSuccess) snprintf(static_error, sizeof static_error, "launch: %s", cudaGetErrorString(e));

@@ -715,7 +715,9 @@ qkv_prepare_vec_kernel(const T* __restrict__ proj, int row_stride, int q_col, in
       for (int j = 0; j < HPW; ++j) scale[j] = warp + 8 * j < nq ? scale_q : scale_k;
     }
     const bool stored = slot >= 0 && slot < num_slots;
-    const long long page = stored ? slot / page_size : 0, off = stored ? slot - page * page_size : 0;
+    // (A 64-bit division is a hundred instructions a warp, and these set this kernel's pace: there are 24 heads of them.)
+    const long long page = !stored ? 0 : slot <= 0xffffffffLL ? (unsigned)slot / (unsigned)page_size : slot / page_size;
+    const long long off = stored ? slot - page * page_size : 0;
     const int apart = rhalf / PL;  // lanes to a rotation's other half
 #pragma unroll
     for (int j = 0; j < HPW; ++j) {
@@ -1114,5 +1116,85 @@ extern "C" int omnia_fill_slots(const void* const* to, const void* const* from, 
   for (int s = 0; s < count; ++s) fill.slots[s] = slots[s];
   const long long pieces = (most / 16 + 255) / 256;
   launch_pdl(fill_slots_kernel, dim3((unsigned)(pieces < 1 ? 1 : pieces > 64 ? 64 : pieces), tensors, count), 256, 0, stream, fill);
+  return OMNIA_LAUNCH_RESULT();
+}
+
+// ---------------------------------------------------------------------------------
+// A decode step's requests cut into pieces for the decode attention kernel, a block a piece and key/value head. Chunks at
+// fixed positions give a short request's only chunk as much of the GPU as a long one's, and the last blocks run alone. Here a
+// request is cut into equal parts of at most `size` tiles of 32 keys, `size` the least with which the parts of all
+// requests fit into one, two or three times `places` (the blocks a head that the GPU holds at a time), and the parts are
+// listed largest first: SMs are given blocks in turn, so each gets its share of every size. Which of the three is estimated
+// from blocks an SM times their mean size, and WAVE tiles of an SM's time for each further round of blocks (their starts).
+// Lengths are on the device alone in a replayed step, hence a kernel, once for all layers that see as far: one block, a warp
+// for each of the three to find its size, a thread for each request to list its parts.
+constexpr int PIECE_LEAST = 4, PIECE_ROUNDS = 3, PIECE_WAVE = 13, PIECE_THREADS = 256;
+struct __align__(16) Piece {  // (as attention_tc.cu reads it)
+  int request, pos, lo, hi, index, count, before, unused;
+};
+__global__ void __launch_bounds__(PIECE_THREADS)
+decode_pieces_kernel(const int* __restrict__ seq_lens, int requests, int window, int run, int nkv, int places, int rounds, int sms,
+                     Piece* __restrict__ list) {
+  __shared__ int tiles[PIECE_THREADS], parts[PIECE_THREADS], sizes[PIECE_THREADS];
+  __shared__ int found[PIECE_ROUNDS], cost[PIECE_ROUNDS];
+  pdl_wait();
+  pdl_launch_dependents();
+  const int r = threadIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int pos = r < requests ? seq_lens[r] - 1 : -1;
+  int first = window > 0 ? max(0, pos - window + 1) : 0;
+  if (run > 0 && pos >= 0) first = max(first, pos - pos % run);
+  const int mine = pos < 0 ? 0 : pos / 32 - first / 32 + 1;
+  tiles[r] = mine;
+  __syncthreads();
+  if (warp < rounds) {
+    const int room = places * (warp + 1);
+    int total = 0, most = 0, live = 0;
+    for (int i = lane; i < PIECE_THREADS; i += 32) total += tiles[i], most = max(most, tiles[i]), live += tiles[i] > 0;
+    total = __reduce_add_sync(0xffffffffu, total), most = __reduce_max_sync(0xffffffffu, most), live = __reduce_add_sync(0xffffffffu, live);
+    auto needed = [&](int size) {
+      int need = 0;
+      for (int i = lane; i < PIECE_THREADS; i += 32) need += (tiles[i] + size - 1) / size;
+      return (int)__reduce_add_sync(0xffffffffu, need);
+    };
+    int lo = max(PIECE_LEAST, (total + room - 1) / room), hi = max(lo, most);  // the least size that fits lies within
+    while (lo < hi) {
+      const int mid = (lo + hi) / 2;
+      if (needed(mid) <= room) hi = mid; else lo = mid + 1;
+    }
+    const int count = needed(lo);
+    if (lane == 0) {
+      found[warp] = lo;
+      const int blocks = count * nkv;
+      cost[warp] = live > room || count == 0 ? 0x7fffffff : (int)((long long)((blocks + sms - 1) / sms) * total / count) + PIECE_WAVE * warp;
+    }
+  }
+  __syncthreads();
+  int round = 0;
+  for (int i = 1; i < rounds; ++i)
+    if (cost[i] < cost[round]) round = i;
+  const int size = found[round], count = (mine + size - 1) / size, part = count > 0 ? (mine + count - 1) / count : 0;
+  parts[r] = count, sizes[r] = part;
+  __syncthreads();
+  int before = 0, all = 0;
+  for (int i = 0; i < requests; ++i) {
+    const int n = parts[i], s = sizes[i];
+    all += n;
+    if (s > part || (s == part && i < r)) before += n;
+  }
+  const int base = count > 0 ? mine / count : 0, longer = count > 0 ? mine - base * count : 0;  // the first `longer` parts have a tile more
+  for (int i = 0; i < count; ++i) {
+    const int tile = first / 32 + i * base + min(i, longer), next = tile + base + (i < longer);
+    list[before + i] = Piece{r, pos, max(first, tile * 32), min(pos, next * 32 - 1), i, count, before, 0};
+  }
+  for (int i = all + r; i < places * rounds; i += PIECE_THREADS) list[i].request = -1;
+}
+
+// list: room for rounds * places pieces of eight ints, on 16 bytes. At most 256 requests, no more than that room, and 3 rounds.
+extern "C" int omnia_decode_pieces(const int* seq_lens, int requests, int window, int run, int nkv, int places, int rounds, int sms, void* list,
+                                   cudaStream_t stream) {
+  if (requests < 1 || requests > PIECE_THREADS || places < 1 || rounds < 1 || rounds > PIECE_ROUNDS || requests > rounds * places || sms < 1 || nkv < 1 ||
+      ((uintptr_t)list & 15))
+    return (int)cudaErrorInvalidValue;
+  launch_pdl(decode_pieces_kernel, 1, PIECE_THREADS, 0, stream, seq_lens, requests, window, run, nkv, places, rounds, sms, (Piece*)list);
   return OMNIA_LAUNCH_RESULT();
 }

@@ -344,6 +344,41 @@ def decode_plan(requests: int, nkv: int, longest: int, sms: int) -> tuple[int, i
     return best
 
 
+PIECE_REQUESTS, PIECE_TILES = 256, 5
+"""The most requests a list of pieces is made for (the kernel's), and the tiles of 32 keys a block from which on decode
+attention runs by such a list."""
+
+
+def decode_places(requests: int, nkv: int, longest: int, sms: int) -> tuple[int, int]:
+    """(blocks a key/value head that the GPU holds at a time, rounds of them that there may be) where a decode step's
+    attention runs by a list of pieces (`omnia_decode_pieces`); (0, 0) where it keeps to `decode_plan`'s chunks. `requests` is
+    rounded up to a power of two, `longest` bounds the positions that a request sees."""
+    batch = 1 << max(requests - 1, 0).bit_length()
+    places = 6 * sms // max(nkv, 1)
+    rounds = 1 if 2 * batch <= places else 2
+    if batch * nkv * 8 <= sms or batch > min(PIECE_REQUESTS, rounds * places):
+        return 0, 0
+    return (places, rounds) if batch * nkv * -(-longest // 32) >= PIECE_TILES * 6 * sms else (0, 0)
+
+
+def _decode_list(step: StepContext, kv: KVView, run: int, nkv: int, places: int, rounds: int,
+                 device: torch.device) -> tuple[torch.Tensor, bool]:
+    """(the step's list of pieces, whether this call has made it: once a pass for all layers that see as far)."""
+    if step.workspace is None:
+        step.workspace = {}
+    made = step.workspace.setdefault("pass", {})
+    key = ("decode_list", kv.window or 0, run, nkv)
+    if key in made:
+        return made[key], False
+    (rows,) = _step_buffers(step, device, {f"decode_list_{kv.window or 0}_{run}_{nkv}": (rounds * places * 8, torch.int32, False)})
+    fn = _function("elementwise", "omnia_decode_pieces",
+                   [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(fn(_ptr(step.seq_lens), step.num_seqs, kv.window or 0, run, nkv, places, rounds, sm_count(device), _ptr(rows), _stream()),
+           "decode_pieces")
+    made[key] = rows
+    return rows, True
+
+
 def tiled_attention_supported(dtype: torch.dtype, nq: int, nkv: int, d: int) -> bool:
     """The tensor-core kernels take bfloat16, head sizes in steps of 8 up to 256 and up to
     16 query heads per key/value head; everything else runs on the generic kernel."""
@@ -693,15 +728,19 @@ def paged_attention(q: torch.Tensor | None, kv: KVView, step: StepContext, scale
         held = width_bucket(-(-longest // kv.page_size)) * kv.page_size
         chunk, warps = decode_plan(count, nkv, held, sm_count(q.device))
         max_chunks = -(-held // chunk)
+        sees = min(held, (kv.window or held) + 32, (run or held) + 32)
+        places, rounds = decode_places(count, nkv, sees, sm_count(q.device)) if step.decode_only and warps == 1 else (0, 0)
+        pieces, (listed, now) = rounds * places, _decode_list(step, kv, run, nkv, places, rounds, q.device) if places else (None, False)
+        places = pieces or count * max_chunks  # partial results a head
         part_o, part_ml, tickets = _step_buffers(step, q.device, {
-            "attention_part_o": (count * nq * max_chunks * d, torch.float32, False),
-            "attention_part_ml": (count * nq * max_chunks * 2, torch.float32, False),
+            "attention_part_o": (nq * places * d, torch.float32, False),
+            "attention_part_ml": (nq * places * 2, torch.float32, False),
             "attention_tickets": (count * nkv, torch.int32, True)})
         fn = _function("attention_tc", "omnia_attention_decode_tc",
                        [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p,
                         c_void_p, c_int, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_int, c_int, c_int,
                         c_float, c_int, c_void_p, c_int, c_int, c_int, c_int, c_float, c_void_p, c_void_p,
-                        c_int, c_int, c_void_p, c_int, c_float, c_float, c_float, c_float, c_int, c_int, c_void_p, c_void_p],
+                        c_int, c_void_p, c_int, c_int, c_int, c_void_p, c_int, c_float, c_float, c_float, c_float, c_int, c_int, c_void_p, c_void_p],
                        defines)
         p = projection
         fused = (None, 0, 0, 0, 0, -1.0, None, None) if p is None else (
@@ -710,7 +749,7 @@ def paged_attention(q: torch.Tensor | None, kv: KVView, step: StepContext, scale
         _check(fn(None if p is not None else _ptr(q), _ptr(kv.pages), _ptr(kv.block_table), _ptr(step.cu_seqlens),
                   _ptr(step.seq_lens), _ptr(single), count, _ptr(part_o), _ptr(part_ml), _ptr(tickets), chunk,
                   max_chunks, gate_ptr, gate_stride, _ptr(out), max_pages, num_pages, nq, nkv, kv.page_size,
-                  kv.window or 0, scale, warps, *fused, 1, keep, _ptr(sink), run, softcap, *last, int(beside), err, _stream()),
+                  kv.window or 0, scale, warps, *fused, 1, _ptr(listed), pieces, int(now), keep, _ptr(sink), run, softcap, *last, int(beside), err, _stream()),
                "attention_decode")
 
     # `beside` leaves the wait for the kernel that wrote q and the cache to the prompts' kernel in front: only where that

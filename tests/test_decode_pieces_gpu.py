@@ -1,0 +1,95 @@
+"""Decode attention by a list of even pieces, its merge of many chunks, and the head-by-head preparation of queries, keys and
+values by 16-byte loads: each against the form that it stands beside."""
+
+from __future__ import annotations
+
+import pytest
+import torch
+
+import kernel_refs
+from mlx_omnia_b200.parts.base import KVSpec, KVView
+from test_kernels_gpu import close, make_kv, ops, rand, step_of  # noqa: F401
+
+pytestmark = pytest.mark.gpu
+
+
+def _cache(seq_lens, nkv, d, page, seed):
+    pages, table = make_kv(seq_lens, nkv, d, page, torch.bfloat16, 1 + sum(-(-n // page) for n in seq_lens), seed=seed)
+    pages.copy_(rand(*pages.shape, dtype=torch.bfloat16, seed=seed + 1))
+    return pages, table
+
+
+@pytest.mark.parametrize("places,rounds", [(9, 1), (9, 2), (200, 1), (40, 3)])
+@pytest.mark.parametrize("seq_lens,window", [([1, 33, 700, 32, 0, 257, 1025, 2000, 64], None), ([900, 5, 0, 431, 128], 300),
+                                             ([160] * 7, None), ([2500] + [1] * 8, None)])
+def test_decode_attention_by_pieces(ops, monkeypatch, places, rounds, seq_lens, window):  # noqa: F811
+    """Every split that the list may make gives what the chunks at fixed positions give: both are float32 sums of the same
+    products, rounded once, so they are a rounding of the result apart (bfloat16: 2^-8, of the largest value)."""
+    nq, nkv, d, page = 6, 3, 128, 16
+    step = step_of([1] * len(seq_lens), seq_lens)
+    pages, table = _cache([max(n, 1) for n in seq_lens], nkv, d, page, 21)
+    q, gate = rand(len(seq_lens), nq, d, dtype=torch.bfloat16, seed=22), rand(len(seq_lens), nq * d, dtype=torch.bfloat16, seed=23)
+    view = KVView(pages, table, torch.zeros(len(seq_lens), dtype=torch.int64, device="cuda"), page, window)
+    monkeypatch.setattr(ops, "decode_plan", lambda *a: (128, 1))
+    want = ops.paged_attention(q, view, step, 0.9 * d ** -0.5, gate=gate)
+    assert rounds * places >= len(seq_lens)
+    monkeypatch.setattr(ops, "decode_places", lambda *a: (places, rounds))
+    for _ in range(2):  # a second layer reads the first one's list, and the tickets are back at zero
+        got = ops.paged_attention(q, view, step, 0.9 * d ** -0.5, gate=gate)
+        live = torch.tensor([n > 0 for n in seq_lens], device="cuda")
+        assert float((got[live].float() - want[live].float()).abs().max()) <= 2 ** -8 * max(1.0, float(want[live].float().abs().max()))
+    ops.begin_pass(step)
+    ops.raise_on_error(q.device)
+
+
+@pytest.mark.parametrize("warps", [1, 4])
+@pytest.mark.parametrize("nq,nkv,d", [(4, 2, 128), (3, 1, 64), (5, 1, 40), (2, 1, 256)])
+@pytest.mark.parametrize("length", [128 * 15, 128 * 16 + 1, 128 * 37 + 5])
+def test_merge_of_many_chunks(ops, monkeypatch, warps, nq, nkv, d, length):  # noqa: F811
+    """Chunks of 128 keys around the sixteen that a round of the merge takes, against the plain reference."""
+    seq_lens, page = [length, 130, 1], 16
+    step = step_of([1] * 3, seq_lens)
+    pages, table = _cache(seq_lens, nkv, d, page, 31)
+    q, gate = rand(3, nq, d, dtype=torch.bfloat16, seed=32), rand(3, nq * d, dtype=torch.bfloat16, seed=33)
+    view = KVView(pages, table, torch.zeros(3, dtype=torch.int64, device="cuda"), page, None)
+    monkeypatch.setattr(ops, "decode_plan", lambda *a: (128, warps))
+    got = ops.paged_attention(q, view, step, 0.9 * d ** -0.5, gate=gate)
+    close(got, kernel_refs.paged_attention(q, view, step, 0.9 * d ** -0.5, gate=gate), torch.bfloat16)
+    ops.raise_on_error(q.device)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nq,nkv,d,rot,whole,interleaved,biased,mixed", [
+    (16, 4, 128, 64, True, True, False, False), (4, 2, 64, 64, False, False, True, False), (30, 1, 128, 32, False, False, False, False),
+    (8, 4, 256, 256, False, False, False, True), (3, 1, 64, 0, True, False, True, False), (6, 5, 128, 8, True, False, False, True),
+    (1, 0, 256, 128, True, True, False, False), (14, 9, 128, 12, False, True, True, False)])
+def test_heads_prepared_side_by_side(ops, dtype, nq, nkv, d, rot, whole, interleaved, biased, mixed):  # noqa: F811
+    """The kernel that takes a token's heads side by side against the general one, which a projection that starts off 16 bytes
+    still takes. Both round float32 results once; their sums of squares are added in another order."""
+    tokens, page = 700, 16  # more than the blocks that stay: some take several tokens
+    heads, store = nq + 2 * max(nkv, 1), nkv > 0
+    g = max(nkv, 1)
+    cols = heads * d
+    wide = rand(tokens, cols + 8, dtype=dtype, seed=41)
+    odd = torch.empty(tokens * (cols + 8) + 1, dtype=dtype, device="cuda")[1:].view(tokens, cols + 8)
+    odd.copy_(wide)
+    assert odd.data_ptr() % 16
+    bias = rand(cols + 8, dtype=dtype, seed=42) if biased else None
+    wq, wk = (1 + rand((n if whole else 1) * d, scale=0.1, seed=43 + n) for n in (nq, g))
+    inv = (10000.0 ** (-torch.arange(rot // 2, dtype=torch.float64) * 2 / rot)).float().cuda() if rot else None
+    positions = torch.randint(0, 5000, (tokens,), device="cuda", dtype=torch.int32)
+    slots = torch.randperm(tokens + 20, device="cuda")[:tokens].to(torch.int64)
+    slots[3] = -1
+    other = (rand(tokens, g * d + 8, dtype=dtype, seed=45), 8, 0.3) if mixed and store else None
+    out = []
+    for rows in (wide, odd):
+        pages = torch.zeros(-(-(tokens + 20) // page), 2, g, page, d, dtype=dtype, device="cuda")
+        kv = KVView(pages, torch.zeros(1, 1, dtype=torch.int32, device="cuda"), slots, page, None, spec=KVSpec(((g, d), (g, d)), None))
+        q = ops.qkv_prepare(rows, 0, nq * d, (nq + g) * d, nq, d, bias if other is None else None, wq, wk, 1e-5, inv, positions, kv, store,
+                            whole=whole, interleaved=interleaved, mix=other)
+        out.append((q, pages))
+    bound = 1e-5 if dtype == torch.float32 else 2 ** -7  # bfloat16: neighbours, half a unit either side
+    for a, b in zip(*out):
+        scale = b.float().abs().clamp(min=1.0)
+        assert float(((a.float() - b.float()).abs() / scale).max()) <= bound
+    ops.raise_on_error(wide.device)

@@ -331,3 +331,12 @@ def test_which_experts_stream_their_weights():
     assert [entry(rows, 6, 64, 2048, 384) for rows in (8, 16, 17)] == [8, 8, 0]
     assert [entry(rows, 8, 8, 2048, 1024) for rows in (8, 9, 16, 17)] == [8, 16, 16, 0]
     assert [entry(rows, 1, 2, 264, 24) for rows in (6, 7, 16)] == [8, 0, 0]
+
+
+def test_decode_lists_of_pieces_where_there_is_work_for_every_block():
+    """The same answer for all batches of a bucket, one round of blocks while a head has two places a request, and chunks at fixed
+    positions for one or two requests, for short ones and for more requests than a list is made for."""
+    assert ops.decode_places(1, 8, 100000, 148) == ops.decode_places(2, 8, 4096, 148) == (0, 0)
+    assert ops.decode_places(8, 8, 4096, 148) == ops.decode_places(5, 8, 4096, 148) == (111, 1)
+    assert ops.decode_places(8, 8, 2000, 148) == (0, 0) and ops.decode_places(256, 8, 4096, 148) == (0, 0)
+    assert ops.decode_places(64, 8, 2304, 148) == (111, 2)
