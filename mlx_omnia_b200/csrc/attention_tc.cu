@@ -115,6 +115,14 @@ __device__ __forceinline__ unsigned pack_bf16(float lo, float hi) {
   return *reinterpret_cast<unsigned*>(&v);
 }
 
+// One more ticket of `counter`, with what this thread has written, or seen written behind a barrier, given out before it and
+// what earlier drawers gave out taken in behind it.
+__device__ __forceinline__ int draw_ticket(int* counter) {
+  int ticket;
+  asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;" : "=r"(ticket) : "l"(counter) : "memory");
+  return ticket;
+}
+
 struct CacheRef {
   const bf16* pages;   // [num_pages, 2, nkv, page_size, D]
   const int* table;    // block-table entries, entry 0 being logical page `first_page`
@@ -717,6 +725,23 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
   OMNIA_TRACE_BLOCK(3);
   if (early) pdl_wait();
   OMNIA_TRACE_BLOCK(4);
+  // Fused mode: the new token's key and value (this request's, this head's), for the warp whose
+  // tile holds position `pos`: lane l owns dims l * D / 32 .. of the head; a dim's rotation
+  // partner lives 16 lanes away. They go to the cache pages and, once that tile has landed,
+  // over its row of the tile (the cache had nothing there yet). They are asked for ahead of the query: the block that brings
+  // them is one its head's merge waits for, and a trip to L2 of their own made it the last by 1.1 us.
+  constexpr int VW = D / 32 > 0 ? D / 32 : 1;
+  float new_k[VW], new_v[VW];
+  const bool brings_new = fused.proj != nullptr && pos >= lo && pos <= hi &&
+                          ((pos / DECODE_BN - lo / DECODE_BN) % WARPS) == warp;
+  long long new_slot = -1;
+  if (brings_new) {
+    const bf16* k_src = fused.proj + token * fused.stride + fused.k_col + (size_t)kvh * D + lane * VW;
+    const bf16* v_src = fused.proj + token * fused.stride + fused.v_col + (size_t)kvh * D + lane * VW;
+    new_slot = fused.slot_mapping[token];
+#pragma unroll
+    for (int i = 0; i < VW; ++i) new_k[i] = __bfloat162float(k_src[i]), new_v[i] = __bfloat162float(v_src[i]);
+  }
   unsigned qf[KSTEPS][4];
   {
     const int g = lane >> 2, t = lane & 3;
@@ -772,24 +797,10 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
         }
     }
   }
-  // Fused mode: the new token's key and value (this request's, this head's), for the warp whose
-  // tile holds position `pos`: lane l owns dims l * D / 32 .. of the head; a dim's rotation
-  // partner lives 16 lanes away. They go to the cache pages and, once that tile has landed,
-  // over its row of the tile (the cache had nothing there yet).
-  constexpr int VW = D / 32 > 0 ? D / 32 : 1;
-  float new_k[VW], new_v[VW];
-  const bool brings_new = fused.proj != nullptr && pos >= lo && pos <= hi &&
-                          ((pos / DECODE_BN - lo / DECODE_BN) % WARPS) == warp;
   if (brings_new) {
-    const bf16* k_src = fused.proj + token * fused.stride + fused.k_col + (size_t)kvh * D + lane * VW;
-    const bf16* v_src = fused.proj + token * fused.stride + fused.v_col + (size_t)kvh * D + lane * VW;
     float ss = 0.f;
 #pragma unroll
-    for (int i = 0; i < VW; ++i) {
-      new_k[i] = __bfloat162float(k_src[i]);
-      new_v[i] = __bfloat162float(v_src[i]);
-      ss += new_k[i] * new_k[i];
-    }
+    for (int i = 0; i < VW; ++i) ss += new_k[i] * new_k[i];
     const float n = fused.eps >= 0.f ? rsqrtf(warp_sum(ss) / (float)D + fused.eps) : 1.f;
 #pragma unroll
     for (int i = 0; i < VW; ++i) {
@@ -800,19 +811,6 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
         mine = lane < 16 ? mine * c - other * sn : other * sn + mine * c;
       }
       new_k[i] = __bfloat162float(__float2bfloat16_rn(mine));  // as the cache will hold it
-    }
-    const long long slot = fused.slot_mapping[token];
-    if (slot >= 0 && slot < fused.num_slots) {
-      const long long page = slot / page_size, off = slot % page_size;
-      bf16* k_dst = fused.pages + (((page * 2 + 0) * nkv + kvh) * page_size + off) * D + lane * VW;
-      bf16* v_dst = fused.pages + (((page * 2 + 1) * nkv + kvh) * page_size + off) * D + lane * VW;
-#pragma unroll
-      for (int i = 0; i < VW; ++i) {
-        k_dst[i] = __float2bfloat16_rn(new_k[i]);
-        v_dst[i] = __float2bfloat16_rn(new_v[i]);
-      }
-    } else if (slot >= fused.num_slots && lane == 0) {
-      atomicOr(err, OMNIA_ERR_SLOT);
     }
   }
   float o[NT_O][4];
@@ -867,6 +865,20 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
     }
   }
   cp_async_wait<0>();
+  if (brings_new) {
+    if (new_slot >= 0 && new_slot < fused.num_slots) {
+      const long long page = new_slot / page_size, off = new_slot % page_size;
+      bf16* k_dst = fused.pages + (((page * 2 + 0) * nkv + kvh) * page_size + off) * D + lane * VW;
+      bf16* v_dst = fused.pages + (((page * 2 + 1) * nkv + kvh) * page_size + off) * D + lane * VW;
+#pragma unroll
+      for (int i = 0; i < VW; ++i) {
+        k_dst[i] = __float2bfloat16_rn(new_k[i]);
+        v_dst[i] = __float2bfloat16_rn(new_v[i]);
+      }
+    } else if (new_slot >= fused.num_slots && lane == 0) {
+      atomicOr(err, OMNIA_ERR_SLOT);
+    }
+  }
   OMNIA_TRACE_BLOCK(5);
   if (!beside) pdl_launch_dependents();  // the cache is read: the next kernel may begin its preamble
 
@@ -930,27 +942,20 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
     }
   }
   // Whoever finishes last merges: publish the partial, take a ticket, and if it is the last
-  // one of this (request, head group), read all partials back and write the output. The fences are the ticket thread's: its
-  // own and, through the barrier, the block's writes are released by the first, the other blocks' acquired by the second.
+  // one of this (request, head group), read all partials back and write the output. The ticket is drawn with release
+  // and acquire at once: with it the thread's own and, through the barrier, the block's writes are given out, and the other blocks'
+  // taken in.
   int* counter = tickets + (size_t)request * nkv + kvh;
   int ticket = 0;
   if (WARPS == 1) {
     __syncwarp();
-    if (lane == 0) {
-      __threadfence();
-      ticket = atomicAdd(counter, 1);
-      __threadfence();
-    }
+    if (lane == 0) ticket = draw_ticket(counter);
     ticket = __shfl_sync(0xffffffffu, ticket, 0);
     __syncwarp();
   } else {
     __shared__ int drawn;
     __syncthreads();
-    if (threadIdx.x == 0) {
-      __threadfence();
-      drawn = atomicAdd(counter, 1);
-      __threadfence();
-    }
+    if (threadIdx.x == 0) drawn = draw_ticket(counter);
     __syncthreads();
     ticket = drawn;
   }
