@@ -11,7 +11,8 @@
 //             the final output (optionally times sigmoid(gate)).
 //   decode:   one warp per block owns the g rows of one single-token request and one
 //             chunk of keys (chunks are aligned to absolute key positions; the caller picks
-//             their size from the number of requests and the longest one); it writes an
+//             their size from the number of requests and the longest one), or one piece of a
+//             list that cuts requests of unequal lengths evenly; it writes an
 //             unnormalised partial (max, sum, accumulator) to scratch memory and takes a
 //             ticket; the block that draws the last ticket of a (request, head group)
 //             merges that group's chunks in ascending order (nobody waits for anybody).
@@ -567,6 +568,7 @@ __device__ __forceinline__ void merge_chunks(const float* __restrict__ part_o, c
 // GPU otherwise) the warps take the tiles in turn, one stage each, and their states are merged
 // through shared memory before the block's partial is written. Partials:
 //   part_o  [requests, nq, max_chunks, D] float32 (unnormalised), part_ml [requests, nq, max_chunks, 2]
+//           (by a list of pieces: [nq, pieces, D] and [nq, pieces, 2], grid (nkv, pieces))
 //   tickets [requests, nkv] int32, zero before the first launch; the merging block zeroes its
 //   ticket again, so the array is ready for the next launch.
 // What the decode kernel needs to do the step before it as well (a decode step's QK-norm, rotation
@@ -596,7 +598,8 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
                         const int* __restrict__ seq_lens, const int* __restrict__ seq_ids,
                         float* __restrict__ part_o, float* __restrict__ part_ml,
                         int* __restrict__ tickets, const bf16* __restrict__ gate, int gate_stride,
-                        bf16* __restrict__ out, int chunk_keys, int max_chunks, const Piece* __restrict__ list, int pieces, int listed_before, int max_pages,
+                        bf16* __restrict__ out, int chunk_keys, int max_chunks, const Piece* __restrict__ list, int pieces,
+                        int listed_before, int max_pages,
                         int num_pages, int nq, int nkv, int page_size, int window, float scale,
                         const FusedQK fused, int keep_first, const float* __restrict__ sink, int run, float softcap,
                         const MapDifference difference, int beside, int* err) {

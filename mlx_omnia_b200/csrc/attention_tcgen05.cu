@@ -192,9 +192,9 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   OMNIA_TRACE_BLOCK(3);
 
   if (warp == 0 || warp == 6) {
-    // ---- producers: warp 0 loads Q once, then the K tiles; warp 6 the V tiles. Issuing a box keeps
-    // a warp busy for about 70 ns: one warp for both rings spent more than half a tile's time on it
-    // (2,048 tokens: 61 us with one warp, 52 us with one per ring; two per ring: no faster). ------
+    // ---- producers: warp 0 loads Q once, then the K tiles; warp 6 the V tiles. A warp
+    // to a ring: when its lanes issued a box each, some 70 ns a box, one warp for both rings spent more than half a
+    // tile's time on it (2,048 tokens: 61 us with one warp, 52 us with one per ring; two per ring: no faster). ------
     const int which = warp == 0 ? 0 : 1;  // 0 keys, 1 values
     if (warp == 0 && omnia_elect_one()) {
       mbar_expect_tx(q_full, DH * ROWS * 128);
@@ -277,7 +277,7 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     // ---- issuer of the score products: S[j & 1] = Q K_j^T --------------------------------------------
     // The two kinds of product are issued by two threads (this warp and warp 7). The products of one
     // accumulator depend on one another and run one at a time, some 50 to 100 ns each whatever their
-    // size; a single thread issuing a tile's twelve kept at most one chain in flight and a tile took
+    // size where `lane == 0` issued them; a single thread issuing a tile's twelve kept at most one chain in flight and a tile took
     // 1.27 us, two threads keep the scores' chain and the values' chain going side by side (1.06 us).
     // What one thread's products must wait for of the other's goes through barriers: a score buffer
     // is written again only when the P V product that read P from it is done (v_done, two tiles back).

@@ -19,8 +19,8 @@
 //   O += P V    tcgen05.mma (M 128, N head size), P read from tensor memory, V in stages of 64 keys.
 //               The exponent's offset follows a row's maximum lazily, as in the other kernel
 // Warps 0, 1 feed the ring of K tiles and warps 12, 13 the ring of V stages with TMA, a box of 16 keys
-// x 64 dims per page group (issuing a box keeps a warp busy for some 70 ns whatever its size, so each
-// ring has two warps that take turns); warps 2 and 3 issue the two kinds of product; warps 4-11 are
+// x 64 dims per page group (two warps to a ring, that take turns: when its lanes issued a box each, a
+// box kept a warp busy for some 70 ns whatever its size); warps 2 and 3 issue the two kinds of product; warps 4-11 are
 // the softmax and the epilogue (each team normalises, gates and stores half of the dims). Masking of
 // groups that are not loaded, the cleared tail of the last V stage and the bounded waits are the other
 // kernel's; the work list is the same (tiles counted in 64 keys), but every block does all of its keys:
@@ -158,8 +158,8 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
   OMNIA_TRACE_BLOCK(3);
 
   if ((warp >= WARP_K && warp < WARP_K + FEEDERS) || (warp >= WARP_V && warp < WARP_V + FEEDERS)) {
-    // ---- producers. Issuing a box (16 keys x 64 dims, a page group) keeps a warp busy for about
-    // 70 ns whatever its size, so each ring has two warps that take turns with its stages. ----------
+    // ---- producers: each ring has two warps that take turns with its stages (a box is 16 keys x 64 dims, a page
+    // group). --------------------------------------------------------------------------------------
     const int which = warp >= WARP_V ? 1 : 0;          // 0 keys, 1 values
     const int turn = warp - (which ? WARP_V : WARP_K);  // this warp's stages: turn, turn + 2, ...
     if (warp == WARP_K && omnia_elect_one()) {
