@@ -645,13 +645,13 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
     seq = seq_ids ? seq_ids[request] : request;
     pos = seq_lens[seq] - 1;
     first = first_key(pos);
-    lo = max(first, chunk * chunk_keys), hi = min(pos, (chunk + 1) * chunk_keys - 1);
+    const int c0 = first / chunk_keys;  // blocks count from the first chunk in sight: a window needs a window's worth of them
+    lo = max(first, (c0 + chunk) * chunk_keys), hi = min(pos, (c0 + chunk + 1) * chunk_keys - 1);
     if (pos < 0 || lo > hi) {
       if (early || (beside && pos < 0)) pdl_wait();
       return;
     }
-    const int c0 = first / chunk_keys;
-    chunk -= c0, chunks = pos / chunk_keys - c0 + 1;
+    chunks = pos / chunk_keys - c0 + 1;
     part_o += (size_t)request * nq * max_chunks * D, part_ml += (size_t)request * nq * max_chunks * 2;
   }
   // The chunk that holds the window's first key also takes the kept first positions below the
