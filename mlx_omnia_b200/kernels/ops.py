@@ -370,14 +370,13 @@ def decode_places(requests: int, nkv: int, longest: int, sms: int) -> tuple[int,
 
 def _decode_list(step: StepContext, kv: KVView, run: int, nkv: int, places: int, rounds: int,
                  device: torch.device) -> tuple[torch.Tensor, bool]:
-    """(the step's list of pieces, whether this call has made it: once a pass for all layers that see as far)."""
-    if step.workspace is None:
-        step.workspace = {}
-    made = step.workspace.setdefault("pass", {})
+    """(the step's list of pieces, whether this call has made it: once a pass for all layers that see as far). The list lies in
+    memory of the pass's own: another step's layers may run between this one's."""
+    made = step.workspace["pass"]
     key = ("decode_list", kv.window or 0, run, nkv)
     if key in made:
         return made[key], False
-    (rows,) = _step_buffers(step, device, {f"decode_list_{kv.window or 0}_{run}_{nkv}": (rounds * places * 8, torch.int32, False)})
+    rows = torch.empty(rounds * places * 8, dtype=torch.int32, device=device)
     fn = _function("elementwise", "omnia_decode_pieces",
                    [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
     _check(fn(_ptr(step.seq_lens), step.num_seqs, kv.window or 0, run, nkv, places, rounds, sm_count(device), _ptr(rows), _stream()),
@@ -741,7 +740,10 @@ def paged_attention(q: torch.Tensor | None, kv: KVView, step: StepContext, scale
         sees = min(held, kv.window or held, run or held)
         chunk, warps = decode_plan(count, nkv, sees, sm_count(q.device))
         max_chunks = min(-(-held // chunk), -(-sees // chunk) + 1)
-        places, rounds = decode_places(count, nkv, sees, sm_count(q.device)) if step.decode_only and warps == 1 else (0, 0)
+        # (A list is kept for the layers behind this one, so it takes a pass that begins and ends: a caller that runs a layer by
+        # itself may have moved the lengths on since the last call.)
+        listable = step.decode_only and warps == 1 and in_pass(step)
+        places, rounds = decode_places(count, nkv, sees, sm_count(q.device)) if listable else (0, 0)
         pieces, (listed, now) = rounds * places, _decode_list(step, kv, run, nkv, places, rounds, q.device) if places else (None, False)
         places = pieces or count * max_chunks  # partial results a head
         part_o, part_ml, tickets = _step_buffers(step, q.device, {
@@ -998,8 +1000,19 @@ def begin_pass(step: StepContext) -> None:
     """A pass over the model's layers begins: what kernels keep for the length of one pass (tables
     made from the step's positions, shared by the layers) is made afresh. A captured step is the
     same object from replay to replay, and its capture must hold the kernels that make them."""
-    if isinstance(step.workspace, dict):
-        step.workspace.pop("pass", None)
+    if step.workspace is None:
+        step.workspace = {}
+    step.workspace["pass"] = {"begun": True}
+
+
+def end_pass(step: StepContext) -> None:
+    """The pass is over, and with it what was kept for it."""
+    step.workspace.pop("pass", None)
+
+
+def in_pass(step: StepContext) -> bool:
+    """Whether this step's layers run between `begin_pass` and `end_pass`, on the lengths and positions that it began with."""
+    return (step.workspace or {}).get("pass", {}).get("begun", False)
 
 
 def keep_for_pass(step: StepContext, name: str, value) -> None:

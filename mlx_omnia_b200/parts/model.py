@@ -132,8 +132,14 @@ class DecoderModel:
     # -- the step --------------------------------------------------------------------
     def forward(self, step: StepContext, layers: list[LayerContext]) -> torch.Tensor:
         """Run this step's tokens through the schedule. -> float32 logits [wanted, vocab]"""
-        schedule = self.spec.schedule
         ops.begin_pass(step)
+        try:
+            return self._pass(step, layers)
+        finally:
+            ops.end_pass(step)
+
+    def _pass(self, step: StepContext, layers: list[LayerContext]) -> torch.Tensor:
+        schedule = self.spec.schedule
         if self.embedding.state_spec() is not None:
             x = self.embedding.forward(step.token_ids, step.positions, step)
         else:

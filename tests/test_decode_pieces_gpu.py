@@ -34,11 +34,12 @@ def test_decode_attention_by_pieces(ops, monkeypatch, places, rounds, seq_lens, 
     want = ops.paged_attention(q, view, step, 0.9 * d ** -0.5, gate=gate)
     assert rounds * places >= len(seq_lens)
     monkeypatch.setattr(ops, "decode_places", lambda *a: (places, rounds))
+    ops.begin_pass(step)
     for _ in range(2):  # a second layer reads the first one's list, and the tickets are back at zero
         got = ops.paged_attention(q, view, step, 0.9 * d ** -0.5, gate=gate)
         live = torch.tensor([n > 0 for n in seq_lens], device="cuda")
         assert float((got[live].float() - want[live].float()).abs().max()) <= 2 ** -8 * max(1.0, float(want[live].float().abs().max()))
-    ops.begin_pass(step)
+    ops.end_pass(step)
     ops.raise_on_error(q.device)
 
 

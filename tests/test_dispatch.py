@@ -340,3 +340,42 @@ def test_decode_lists_of_pieces_where_there_is_work_for_every_block():
     assert ops.decode_places(8, 8, 4096, 148) == ops.decode_places(5, 8, 4096, 148) == (111, 1)
     assert ops.decode_places(8, 8, 2000, 148) == (0, 0) and ops.decode_places(256, 8, 4096, 148) == (0, 0)
     assert ops.decode_places(64, 8, 2304, 148) == (111, 2)
+
+
+def _calls_of_decode_attention(monkeypatch):
+    """What is launched, (name, arguments), where decode attention runs on this machine's memory without a kernel behind it."""
+    calls = []
+    monkeypatch.setattr(ops, "_function", lambda library, name, argtypes, defines=None: lambda *args: calls.append((name, args)) or 0)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    monkeypatch.setattr(ops, "error_word", lambda device: torch.zeros(1, dtype=torch.int32))
+    return calls
+
+
+def _decode_step(lengths):
+    step = SimpleNamespace(num_seqs=len(lengths), q_lens=[1] * len(lengths), seq_lens_host=lengths, max_seq_len=max(lengths),
+                           decode_only=True, workspace=None, cu_seqlens=torch.zeros(len(lengths) + 1), seq_lens=torch.tensor(lengths))
+    kv = KVView(torch.zeros(2, 2, 8, 16, 128, dtype=torch.bfloat16), torch.zeros(len(lengths), 300, dtype=torch.int32), None, 16, None)
+    return step, lambda: ops.paged_attention(torch.zeros(len(lengths), 16, 128, dtype=torch.bfloat16), kv, step, 1.0)
+
+
+LIST_ARGUMENT = 32  # of omnia_attention_decode_tc
+
+
+def test_a_list_of_pieces_is_the_passes_own(monkeypatch):
+    """Two steps whose layers run in turn have a list each, made once a pass; and there is none for a layer that is run by
+    itself, whose caller may have moved the lengths on since the last call."""
+    calls = _calls_of_decode_attention(monkeypatch)
+    lists = lambda: [args[LIST_ARGUMENT] for name, args in calls if name == "omnia_attention_decode_tc"]  # noqa: E731
+    made = lambda: [args[8] for name, args in calls if name == "omnia_decode_pieces"]  # noqa: E731
+    (first, a), (second, b) = _decode_step([3000, 70] * 8), _decode_step([1500] * 16)
+    a(), a()
+    assert lists() == [None, None] and not made()
+    ops.begin_pass(first), ops.begin_pass(second)
+    calls.clear()
+    a(), b(), a(), b()
+    assert len(made()) == 2 and lists() == made() * 2 and made()[0] != made()[1] and None not in lists()
+    ops.end_pass(first)
+    calls.clear()
+    a(), b()
+    assert lists()[0] is None and lists()[1] is not None and not made()
