@@ -1032,16 +1032,14 @@ def kept_for_pass(step: StepContext, name: str):
 
 def rope_angles(step: StepContext, inv_freq: torch.Tensor) -> torch.Tensor:
     """(cos, sin)(position * inv_freq) for every token of the step, float32 [len(inv_freq), tokens, 2],
-    made once per pass and per table of frequencies (layers of one base share it)."""
-    if step.workspace is None:
-        step.workspace = {}
-    made = step.workspace.setdefault("pass", {})
+    made once per pass and per table of frequencies (layers of one base share it), in memory of the pass's own; outside of a
+    pass by every call."""
+    made = step.workspace["pass"] if in_pass(step) else {}
     key = ("rope_angles", inv_freq.data_ptr())
     table = made.get(key)
     if table is None:
         half = inv_freq.shape[0]
-        (table,) = _step_buffers(step, inv_freq.device,
-                                 {f"rope_angles_{inv_freq.data_ptr()}": (step.num_tokens * half * 2, torch.float32, False)})
+        table = torch.empty(half, step.num_tokens, 2, dtype=torch.float32, device=inv_freq.device)
         fn = _function("elementwise", "omnia_rope_angles", [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p])
         _check(fn(_ptr(step.positions), _ptr(inv_freq), half, step.num_tokens, _ptr(table), _stream()), "rope_angles")
         made[key] = table

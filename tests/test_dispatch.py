@@ -379,3 +379,21 @@ def test_a_list_of_pieces_is_the_passes_own(monkeypatch):
     calls.clear()
     a(), b()
     assert lists()[0] is None and lists()[1] is not None and not made()
+
+
+def test_a_table_of_angles_is_the_passes_own(monkeypatch):
+    """As the lists: one a pass, whichever steps' layers run between, and none kept outside of one."""
+    calls = []
+    monkeypatch.setattr(ops, "_function", lambda *a, **b: lambda *args: calls.append(args) or 0)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    a, b = (SimpleNamespace(num_tokens=9, positions=torch.arange(9), workspace=None) for _ in range(2))
+    inv = torch.ones(4)
+    ops.rope_angles(a, inv), ops.rope_angles(a, inv)
+    assert len(calls) == 2
+    ops.begin_pass(a), ops.begin_pass(b)
+    tables = [ops.rope_angles(step, inv) for step in (a, b, a, b)]
+    assert len(calls) == 4 and tables[0] is tables[2] and tables[1] is tables[3]
+    assert tables[0].data_ptr() != tables[1].data_ptr() and tables[0].shape == (4, 9, 2)
+    ops.end_pass(a)
+    ops.rope_angles(a, inv)
+    assert len(calls) == 5
