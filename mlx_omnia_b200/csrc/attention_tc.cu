@@ -437,12 +437,15 @@ attention_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pa
 // kernel and nothing but latency, so a round's loads (sixteen chunks' maxima and sums, lane u those of chunk u, the
 // thread's own dims of their accumulators, the gates) all leave together, straight into registers: one trip to L2. One warp
 // that brought them through shared memory by asynchronous copies took 5.5 us behind the last ticket of eight requests.
+// Eight chunks a round where a thread has more than eight dims (two maps of more than 128, one warp): sixteen chunks' loads would
+// be 256 registers, and went by way of 572 bytes of local memory.
 template <int H, int THREADS>
 __device__ __forceinline__ void merge_chunks(const float* __restrict__ part_o, const float* __restrict__ part_ml, size_t base,
                                              int max_chunks, int chunks, const bf16* __restrict__ gate_row, bf16* __restrict__ out_row,
                                              float* stage, const float* __restrict__ sink, const MapDifference difference) {
   const int lane = threadIdx.x & 31, tid = threadIdx.x;
-  constexpr int VEC = H * D >= 4 * THREADS ? 4 : 2, PIECES = H * D / VEC, V = (PIECES + THREADS - 1) / THREADS, ROUND = 16;
+  constexpr int VEC = H * D >= 4 * THREADS ? 4 : 2, PIECES = H * D / VEC, V = (PIECES + THREADS - 1) / THREADS;
+  constexpr int ROUND = V * VEC > 8 ? 8 : 16;
   using Piece = std::conditional_t<VEC == 4, float4, float2>;
   float acc[V][VEC], gates[V][VEC], mx[H], total[H];
 #pragma unroll

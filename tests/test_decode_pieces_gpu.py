@@ -59,6 +59,56 @@ def test_merge_of_many_chunks(ops, monkeypatch, warps, nq, nkv, d, length):  # n
     ops.raise_on_error(q.device)
 
 
+def _reference(q, view, step, scale, gate=None, sink=None, run=0, cap=0.0, difference=None, keep=0):
+    """A decode step's attention in 64 bits, request by request."""
+    nq, nkv = q.shape[1], view.pages.shape[2]
+    out = []
+    for s, n in enumerate(step.seq_lens_host):
+        j = torch.arange(n, device="cuda")
+        sees = (j >= n - view.window) | (j < keep) if view.window else j >= 0
+        if run:
+            sees &= j >= (n - 1) - (n - 1) % run
+        pages = view.block_table[s].long()[j // view.page_size]
+        k, v = (view.pages[pages, w, :, j % view.page_size].double().repeat_interleave(nq // nkv, dim=1) for w in (0, 1))
+        z = torch.einsum("hd,jhd->hj", q[s].double(), k) * scale
+        z = (cap * torch.tanh(z / cap) if cap else z).masked_fill(~sees, -torch.inf)
+        if sink is not None:
+            z = torch.cat([z, sink.double()[:, None]], dim=1)
+        p = torch.softmax(z, dim=1)[:, :n]
+        o = torch.einsum("hj,jhd->hd", p, v)
+        if difference is not None:
+            o = (o[0::2] - difference.lam * o[1::2])[:, : difference.dv]
+            o = o * torch.rsqrt((o * o).sum(1, keepdim=True) / difference.dv + difference.eps) * difference.factor
+        out.append(o.reshape(-1))
+    out = torch.stack(out)
+    return out if gate is None else out * torch.sigmoid(gate.double())
+
+
+def _near(got, want):
+    """Each request within 2^-7 of its own largest value: weights and result are rounded to bfloat16 (2^-9 each), and a sum of
+    weighted values is as uncertain as its largest entry's rounding, some 3 deviations of it."""
+    worst = ((got.double() - want).abs().amax(1) / want.abs().amax(1)).tolist()
+    assert max(worst) <= 2 ** -7, worst
+
+
+@pytest.mark.parametrize("warps", [1, 4])
+@pytest.mark.parametrize("nq,nkv,d,dv", [(2, 1, 256, 250), (16, 2, 128, 128), (2, 1, 64, 64)])
+@pytest.mark.parametrize("length", [128 * 8, 128 * 16 + 1, 128 * 37 + 5])
+def test_merge_of_many_chunks_of_two_maps(ops, monkeypatch, warps, nq, nkv, d, dv, length):  # noqa: F811
+    """Around the eight (rows of more than 128 dims, one warp) and the sixteen chunks that a round takes."""
+    seq_lens, page = [length, 130, 1], 16
+    step = step_of([1] * 3, seq_lens)
+    pages, table = _cache(seq_lens, nkv, d, page, 51)
+    q = rand(3, nq, d, dtype=torch.bfloat16, seed=52)
+    view = KVView(pages, table, torch.zeros(3, dtype=torch.int64, device="cuda"), page, None)
+    difference = ops.MapDifference(lam=0.3, eps=1e-5, factor=0.7, dv=dv)
+    monkeypatch.setattr(ops, "decode_plan", lambda *a: (128, warps))
+    got = ops.paged_attention(q, view, step, 0.9 * d ** -0.5, difference=difference)
+    want = _reference(q, view, step, 0.9 * d ** -0.5, difference=difference)
+    _near(got, want)
+    ops.raise_on_error(q.device)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("nq,nkv,d,rot,whole,interleaved,biased,mixed", [
     (16, 4, 128, 64, True, True, False, False), (4, 2, 64, 64, False, False, True, False), (30, 1, 128, 32, False, False, False, False),
