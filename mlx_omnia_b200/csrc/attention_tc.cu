@@ -594,6 +594,17 @@ struct __align__(16) Piece {
   int request, pos, lo, hi, index, count, before, unused;
 };
 
+// The list may be written while this kernel already runs (its maker is the launch before it), so to the compiler it must be no
+// read-only memory: as a plain load of a `const __restrict__` argument this one was moved above the wait for the maker, and in
+// replayed steps the first layer worked on the pieces of the replay before.
+__device__ __forceinline__ Piece load_piece(const Piece* piece) {
+  Piece p;
+  asm volatile("ld.relaxed.gpu.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(p.request), "=r"(p.pos), "=r"(p.lo), "=r"(p.hi) : "l"(piece) : "memory");
+  asm volatile("ld.relaxed.gpu.global.v4.s32 {%0, %1, %2, %3}, [%4 + 16];"
+               : "=r"(p.index), "=r"(p.count), "=r"(p.before), "=r"(p.unused) : "l"(piece) : "memory");
+  return p;
+}
+
 template <int WARPS, int RING, bool CAPPED>
 __global__ void __launch_bounds__(WARPS * 32)
 attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pages,
@@ -601,7 +612,7 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
                         const int* __restrict__ seq_lens, const int* __restrict__ seq_ids,
                         float* __restrict__ part_o, float* __restrict__ part_ml,
                         int* __restrict__ tickets, const bf16* __restrict__ gate, int gate_stride,
-                        bf16* __restrict__ out, int chunk_keys, int max_chunks, const Piece* __restrict__ list, int pieces,
+                        bf16* __restrict__ out, int chunk_keys, int max_chunks, const Piece* list, int pieces,
                         int listed_before, int max_pages,
                         int num_pages, int nq, int nkv, int page_size, int window, float scale,
                         const FusedQK fused, int keep_first, const float* __restrict__ sink, int run, float softcap,
@@ -634,7 +645,7 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
   int request = blockIdx.z, kvh = blockIdx.y, chunk = blockIdx.x, chunks = 0, seq = 0, pos = -1, first = 0, lo = 0, hi = -1;
   if (WARPS == 1 && pieces > 0) {
     if (listed_before) pdl_wait();  // the list comes from the kernel right before this one
-    const Piece mine = list[blockIdx.y];
+    const Piece mine = load_piece(list + blockIdx.y);
     if (mine.request < 0) {
       if (early) pdl_wait();
       return;

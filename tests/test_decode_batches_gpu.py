@@ -33,9 +33,9 @@ WIDE = {
 DECODED = 3
 
 
-def wide_tensors():
-    architecture = resolve_architecture(WIDE)
-    tensors = architecture.random_tensors(architecture.parse(WIDE), 2)
+def wide_tensors(raw=WIDE):
+    architecture = resolve_architecture(raw)
+    tensors = architecture.random_tensors(architecture.parse(raw), 2)
     # Larger than N(0, 0.02), so that the branches weigh as much as the residual stream and the
     # logits reach the bend of the soft cap.
     tensors = {k: (t * (2.0 if "proj" in k else 1.0) if t.dim() == 2 else t) for k, t in tensors.items()}
@@ -77,9 +77,11 @@ def decode_logits(raw, weights, prompts, dtype, graphs):
     return out
 
 
-def check(raw, weights, count, longest, dtype):
+def check(raw, weights, count, longest, dtype, some=()):
     vocab = raw["text_config"]["vocab_size"]
-    prompts = [tiny_configs.prompt(n, vocab, 700 + i) for i, n in enumerate(lengths(count, longest))]
+    drawn = lengths(count, longest)
+    drawn[1: 1 + len(some)] = some
+    prompts = [tiny_configs.prompt(n, vocab, 700 + i) for i, n in enumerate(drawn)]
     oracle = Oracle(raw, weights, {str(i): p for i, p in enumerate(prompts)},
                     rows=lambda ids: list(range(len(ids) - DECODED, len(ids))))
     eager = decode_logits(raw, weights, prompts, dtype, graphs=False)
@@ -105,3 +107,21 @@ def test_tiny_decode_batches(count, dtype):
 @pytest.mark.parametrize("count,dtype", [(17, "bfloat16"), (64, "bfloat16"), (100, "bfloat16"), (33, "float32")])
 def test_decode_batches_at_the_benchmark_widths(count, dtype):
     check(WIDE, wide_tensors(), count, 120, dtype)
+
+
+def test_decode_steps_by_lists_of_pieces(monkeypatch):
+    """Requests enough and long enough for the decode attention's rule to take a list of pieces, which the second of the two
+    layers that see everything shares; steps that go over tiles' borders, launched one by one and replayed."""
+    text = WIDE["text_config"] | {"hidden_size": 512, "intermediate_size": 1024, "vocab_size": 2048, "num_hidden_layers": 3,
+                                  "layer_types": ["full_attention", "sliding_attention", "full_attention"],
+                                  "layer_rope_theta": [1000000.0] * 3}
+    raw, made, real = WIDE | {"text_config": text}, [], ops._decode_list
+
+    def listed(*args):
+        rows, now = real(*args)
+        made.append(now)
+        return rows, now
+
+    monkeypatch.setattr(ops, "_decode_list", listed)
+    check(raw, wide_tensors(raw), 16, 1203, "bfloat16", some=(323, 642, 961, 34))
+    assert made == [True, False] * (DECODED + 2)  # each step by itself; a captured one's first run, and its capture

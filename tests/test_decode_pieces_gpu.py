@@ -3,6 +3,8 @@ values by 16-byte loads: each against the form that it stands beside."""
 
 from __future__ import annotations
 
+import dataclasses
+
 import pytest
 import torch
 
@@ -99,6 +101,7 @@ def test_merge_of_many_chunks_of_two_maps(ops, monkeypatch, warps, nq, nkv, d, d
     seq_lens, page = [length, 130, 1], 16
     step = step_of([1] * 3, seq_lens)
     pages, table = _cache(seq_lens, nkv, d, page, 51)
+    pages[:, 1, ..., dv:] = 0  # as the cache keeps values narrower than keys
     q = rand(3, nq, d, dtype=torch.bfloat16, seed=52)
     view = KVView(pages, table, torch.zeros(3, dtype=torch.int64, device="cuda"), page, None)
     difference = ops.MapDifference(lam=0.3, eps=1e-5, factor=0.7, dv=dv)
@@ -144,3 +147,104 @@ def test_heads_prepared_side_by_side(ops, dtype, nq, nkv, d, rot, whole, interle
         scale = b.float().abs().clamp(min=1.0)
         assert float(((a.float() - b.float()).abs() / scale).max()) <= bound
     ops.raise_on_error(wide.device)
+
+
+@pytest.mark.parametrize("nq,nkv,d", [(6, 3, 128), (4, 2, 64), (4, 2, 256)])
+@pytest.mark.parametrize("places,rounds", [(9, 1), (12, 2)])
+def test_layers_that_share_a_list_in_a_replayed_step(ops, monkeypatch, nq, nkv, d, places, rounds):  # noqa: F811
+    """Two layers of a captured pass, each behind the product that makes its projected rows; the second reads the list ahead of its
+    wait. Replayed on other inputs and on lengths that go over tiles' borders, beside the form by chunks on caches of its own: the
+    same new keys and values, and results that are a rounding apart. (A replay that found what the one before left, lists, rows or
+    gates, would show here.)"""
+    page, seq_lens, layers = 16, [1, 31, 700, 32, 257, 1023, 64, 95, 1500], 2
+    table = _cache([n + 4 for n in seq_lens], nkv, d, page, 61)[1]
+    step = step_of([1] * len(seq_lens), seq_lens)
+    step.workspace, step.max_seq_len = {"private": True}, 1504
+    plain = dataclasses.replace(step, workspace=None)
+    slots = torch.zeros(len(seq_lens), dtype=torch.int64, device="cuda")
+    inputs = [rand(len(seq_lens), 256, dtype=torch.bfloat16, seed=62 + i) for i in range(layers)]
+    weights = [rand((2 * nq + 2 * nkv) * d, 256, dtype=torch.bfloat16, scale=1 / 16, seed=65 + i) for i in range(layers)]
+    caches = [rand(int(table.max()) + 1, 2, nkv, page, d, dtype=torch.bfloat16, seed=70 + i) for i in range(layers)]
+    by_list, by_chunk = ([KVView(c.clone(), table, slots, page, None) for c in caches] for _ in range(2))
+    inv_freq = (10000.0 ** (-torch.arange(d // 2, dtype=torch.float64) * 2 / d)).float().cuda()
+    monkeypatch.setattr(ops, "decode_plan", lambda *a: (128, 1))
+    monkeypatch.setattr(ops, "decode_places", lambda *a: (places, rounds))
+
+    def layer(views, i, step):
+        rows = ops.linear(inputs[i], weights[i])
+        p = ops.Projection(rows, 0, 2 * nq * d, (2 * nq + nkv) * d, nq, d, 1e-6, inv_freq)
+        return ops.paged_attention(None, views[i], step, 0.9 * d ** -0.5, gate=rows, gate_col=nq * d, projection=p)
+
+    def one_pass():
+        ops.begin_pass(step)
+        out = [layer(by_list, i, step) for i in range(layers)]
+        ops.end_pass(step)
+        return out
+
+    def lengths(more):
+        held = [n + more for n in seq_lens]
+        step.seq_lens.copy_(torch.tensor(held, dtype=torch.int32))
+        slots.copy_(torch.tensor([int(table[s, (n - 1) // page]) * page + (n - 1) % page for s, n in enumerate(held)]))
+
+    lengths(0)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        one_pass()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = one_pass()
+    for more in range(4):
+        lengths(more)
+        for i, x in enumerate(inputs):
+            x.copy_(rand(*x.shape, dtype=torch.bfloat16, seed=80 + 10 * more + i))
+        want = [layer(by_chunk, i, plain) for i in range(layers)]  # outside of a pass: by chunks
+        graph.replay()
+        for i in range(layers):
+            assert torch.equal(by_list[i].pages, by_chunk[i].pages)
+            _near(got[i], want[i].double())
+    ops.raise_on_error(inputs[0].device)
+
+
+@pytest.mark.parametrize("tokens", [9, 300])
+@pytest.mark.parametrize("nq,nkv,d,whole", [(16, 4, 128, True), (6, 2, 64, False), (2, 1, 256, False)])
+def test_heads_prepared_behind_a_product_in_a_replayed_step(ops, nq, nkv, d, whole, tokens):  # noqa: F811
+    """The product and the preparation in a captured chain, replayed on other inputs and positions: bit for bit what the two give
+    with a pause between them. (The preparation begins beside the product, and may read nothing of it before its wait.)"""
+    page, width = 16, 256
+    x, weight = rand(tokens, width, dtype=torch.bfloat16, seed=91), rand((nq + 2 * nkv) * d, width, dtype=torch.bfloat16, scale=1 / 16, seed=92)
+    wq, wk = (1 + rand((n if whole else 1) * d, scale=0.1, seed=93 + n) for n in (nq, nkv))
+    inv = (10000.0 ** (-torch.arange(d // 2, dtype=torch.float64) * 2 / d)).float().cuda()
+    positions = torch.zeros(tokens, device="cuda", dtype=torch.int32)
+    slots = torch.zeros(tokens, device="cuda", dtype=torch.int64)
+    caches = [torch.zeros(-(-tokens // page) + 2, 2, nkv, page, d, dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+
+    def product():
+        out = torch.empty(tokens, weight.shape[0], dtype=torch.bfloat16, device="cuda")
+        return ops.linear(x, weight) if tokens <= 16 else ops._gemm_tcgen05(x, weight, out, 0, pair=False)
+
+    def prepare(rows, pages):
+        kv = KVView(pages, torch.zeros(1, 1, dtype=torch.int32, device="cuda"), slots, page, None, spec=KVSpec(((nkv, d), (nkv, d)), None))
+        return ops.qkv_prepare(rows, 0, nq * d, (nq + nkv) * d, nq, d, None, wq, wk, 1e-5, inv, positions, kv, True, whole=whole)
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        prepare(product(), caches[0])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = prepare(product(), caches[0])
+    for again in range(4):
+        x.copy_(rand(*x.shape, dtype=torch.bfloat16, seed=95 + again))
+        positions.copy_(torch.randint(0, 5000, (tokens,), dtype=torch.int32))
+        slots.copy_(torch.randperm(tokens + page)[:tokens])
+        for pages in caches:
+            pages.zero_()
+        graph.replay()
+        rows = product()
+        torch.cuda.synchronize()
+        want = prepare(rows, caches[1])
+        assert torch.equal(got, want) and torch.equal(*caches)
+    ops.raise_on_error(x.device)

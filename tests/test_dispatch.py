@@ -345,6 +345,8 @@ def test_decode_lists_of_pieces_where_there_is_work_for_every_block():
 def _calls_of_decode_attention(monkeypatch):
     """What is launched, (name, arguments), where decode attention runs on this machine's memory without a kernel behind it."""
     calls = []
+    monkeypatch.setattr(ops, "_scratch", {})  # (what this machine's memory stands in for is not left to the tests of a GPU)
+    monkeypatch.setattr(ops, "_zeroed", set())
     monkeypatch.setattr(ops, "_function", lambda library, name, argtypes, defines=None: lambda *args: calls.append((name, args)) or 0)
     monkeypatch.setattr(ops, "_stream", lambda: 0)
     monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
