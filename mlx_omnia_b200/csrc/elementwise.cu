@@ -1123,17 +1123,22 @@ extern "C" int omnia_fill_slots(const void* const* to, const void* const* from, 
 // A decode step's requests cut into pieces for the decode attention kernel, a block a piece and key/value head. Chunks at
 // fixed positions give a short request's only chunk as much of the GPU as a long one's, and the last blocks run alone. Here a
 // request is cut into equal parts of at most `size` tiles of 32 keys, `size` the least with which the parts of all
-// requests fit into one, two or three times `places` (the blocks a head that the GPU holds at a time), and the parts are
-// listed largest first: SMs are given blocks in turn, so each gets its share of every size. Which of the three is estimated
-// from blocks an SM times their mean size, and WAVE tiles of an SM's time for each further round of blocks (their starts).
+// requests fit into one or two times `places` (the blocks a head that the GPU holds at a time), and the parts are
+// listed largest first: SMs are given blocks in turn, so each gets its share of every size. Which of the two is estimated:
+// blocks an SM times their mean size, but no less than `chain` times the largest (a block's tiles come one after another, and an
+// SM with fewer blocks than `chain` waits for memory most of the time), and PIECE_WAVE tiles of an SM's time for a
+// second round of blocks (their starts). Without `chain`, 64 requests of 1,000 positions were 64 pieces: steps of eight
+// layers with heads of 64 took 755 us, with it 648 (by chunks 652); heads of 128: 918, 867 (884).
+// PIECE_WAVE from 0 to 52 and PIECE_LEAST from 1 to 8 made no difference beyond 1 % (16 to 100 requests of unequal lengths,
+// two models), PIECE_LEAST 16 cost 6 to 12 %.
 // Lengths are on the device alone in a replayed step, hence a kernel, once for all layers that see as far: one block, a warp
-// for each of the three to find its size, a thread for each request to list its parts.
-constexpr int PIECE_LEAST = 4, PIECE_ROUNDS = 3, PIECE_WAVE = 13, PIECE_THREADS = 256;
+// for each of the two to find its size, a thread for each request to list its parts.
+constexpr int PIECE_LEAST = 4, PIECE_ROUNDS = 2, PIECE_WAVE = 13, PIECE_THREADS = 256;
 struct __align__(16) Piece {  // (as attention_tc.cu reads it)
   int request, pos, lo, hi, index, count, before, unused;
 };
 __global__ void __launch_bounds__(PIECE_THREADS)
-decode_pieces_kernel(const int* __restrict__ seq_lens, int requests, int window, int run, int nkv, int places, int rounds, int sms,
+decode_pieces_kernel(const int* __restrict__ seq_lens, int requests, int window, int run, int nkv, int places, int rounds, int chain, int sms,
                      Piece* __restrict__ list) {
   __shared__ int tiles[PIECE_THREADS], parts[PIECE_THREADS], sizes[PIECE_THREADS];
   __shared__ int found[PIECE_ROUNDS], cost[PIECE_ROUNDS];
@@ -1165,7 +1170,8 @@ decode_pieces_kernel(const int* __restrict__ seq_lens, int requests, int window,
     if (lane == 0) {
       found[warp] = lo;
       const int blocks = count * nkv;
-      cost[warp] = live > room || count == 0 ? 0x7fffffff : (int)((long long)((blocks + sms - 1) / sms) * total / count) + PIECE_WAVE * warp;
+      cost[warp] = live > room || count == 0 ? 0x7fffffff
+                                             : max((int)((long long)((blocks + sms - 1) / sms) * total / count), chain * lo) + PIECE_WAVE * warp;
     }
   }
   __syncthreads();
@@ -1189,12 +1195,12 @@ decode_pieces_kernel(const int* __restrict__ seq_lens, int requests, int window,
   for (int i = all + r; i < places * rounds; i += PIECE_THREADS) list[i].request = -1;
 }
 
-// list: room for rounds * places pieces of eight ints, on 16 bytes. At most 256 requests, no more than that room, and 3 rounds.
-extern "C" int omnia_decode_pieces(const int* seq_lens, int requests, int window, int run, int nkv, int places, int rounds, int sms, void* list,
-                                   cudaStream_t stream) {
-  if (requests < 1 || requests > PIECE_THREADS || places < 1 || rounds < 1 || rounds > PIECE_ROUNDS || requests > rounds * places || sms < 1 || nkv < 1 ||
-      ((uintptr_t)list & 15))
+// list: room for rounds * places pieces of eight ints, on 16 bytes. At most 256 requests, no more than that room, and 2 rounds.
+extern "C" int omnia_decode_pieces(const int* seq_lens, int requests, int window, int run, int nkv, int places, int rounds, int chain, int sms,
+                                   void* list, cudaStream_t stream) {
+  if (requests < 1 || requests > PIECE_THREADS || places < 1 || rounds < 1 || rounds > PIECE_ROUNDS || requests > rounds * places || chain < 0 || sms < 1 ||
+      nkv < 1 || ((uintptr_t)list & 15))
     return (int)cudaErrorInvalidValue;
-  launch_pdl(decode_pieces_kernel, 1, PIECE_THREADS, 0, stream, seq_lens, requests, window, run, nkv, places, rounds, sms, (Piece*)list);
+  launch_pdl(decode_pieces_kernel, 1, PIECE_THREADS, 0, stream, seq_lens, requests, window, run, nkv, places, rounds, chain, sms, (Piece*)list);
   return OMNIA_LAUNCH_RESULT();
 }

@@ -349,37 +349,43 @@ PIECE_REQUESTS, PIECE_TILES = 256, 5
 attention runs by such a list."""
 
 
-def decode_places(requests: int, nkv: int, longest: int, sms: int) -> tuple[int, int]:
+def decode_places(requests: int, nkv: int, longest: int, sms: int, d: int = 128) -> tuple[int, int]:
     """(blocks a key/value head that the GPU holds at a time, rounds of them that there may be) where a decode step's
     attention runs by a list of pieces (`omnia_decode_pieces`); (0, 0) where it keeps to `decode_plan`'s chunks. `requests` is
-    rounded up to a power of two, `longest` bounds the positions that a request sees.
+    rounded up to a power of two, `longest` bounds the positions that a request sees, `d` is the head size.
 
     Whole decode steps, chunks against the list (B200, us): 16 requests of 190 to 3,000 positions 2,057 / 1,782, 24 through the
     8-billion model 5,820 / 5,050, 32 of up to 600 2,006 / 1,890, 64 of up to 2,304 3,364 / 3,160; of equal lengths, 8 of 4,096
-    1,751 / 1,750, 64 of 2,000 4,077 / 4,100. Below five tiles a block (the smallest of these has 5.5) the pieces are as short
-    as chunks are at their shortest, and the list's launch would be all it gives. Two rounds of blocks cost some 5 us a layer in
-    starts, so there is one while a request has two places a head; mixed steps, whose single tokens share the GPU with
+    1,751 / 1,750. Steps of eight layers, 64 requests of 500 / 1,000 / 2,000 positions: heads of 128 709 / 716, 884 / 867,
+    1,188 / 1,176, heads of 64 555 / 557, 652 / 651, 829 / 828. Below five tiles a block (the smallest of the first has 5.5) the pieces
+    are as short as chunks are at their shortest, and the list's launch would be all it gives. Two rounds of blocks cost some
+    5 us a layer in starts, so there is one while a request has two places a head. More requests than places keep to
+    chunks: what does not fit the first round is a few long pieces behind it (the same steps, 128 requests of 700: 1,076 / 1,152 to 1,184). So do few
+    requests with heads of more than 128, of which an SM holds three blocks and not six (heads of 256, 16 requests of up to 3,000:
+    622 / 652; 24 of up to 2,304 854 / 822, 64 1,299 / 1,055). Mixed steps, whose single tokens share the GPU with
     prompts, keep to chunks (a list there: 7.8 -> 8.1 to 8.5 ms)."""
     batch = 1 << max(requests - 1, 0).bit_length()
     places = 6 * sms // max(nkv, 1)
-    rounds = 1 if 2 * batch <= places else 2
-    if batch * nkv * 8 <= sms or batch > min(PIECE_REQUESTS, rounds * places):
+    if batch * nkv * 8 <= sms or batch > min(PIECE_REQUESTS, places) or (d > 128 and batch * nkv < 128):
         return 0, 0
-    return (places, rounds) if batch * nkv * -(-longest // 32) >= PIECE_TILES * 6 * sms else (0, 0)
+    return (places, 1 if 2 * batch <= places else 2) if batch * nkv * -(-longest // 32) >= PIECE_TILES * 6 * sms else (0, 0)
 
 
-def _decode_list(step: StepContext, kv: KVView, run: int, nkv: int, places: int, rounds: int,
+def _decode_list(step: StepContext, kv: KVView, run: int, nkv: int, d: int, places: int, rounds: int,
                  device: torch.device) -> tuple[torch.Tensor, bool]:
     """(the step's list of pieces, whether this call has made it: once a pass for all layers that see as far). The list lies in
     memory of the pass's own: another step's layers may run between this one's."""
     made = step.workspace["pass"]
-    key = ("decode_list", kv.window or 0, run, nkv)
+    # How many blocks keep an SM busy: a tile of a narrow head is half the bytes. (48 requests of 1,000 positions, heads of 64: 618 us
+    # with six, 607 with nine, by chunks 603; heads of 128 770 and 787, 810.)
+    chain = 9 if d <= 64 else 6
+    key = ("decode_list", kv.window or 0, run, nkv, chain)
     if key in made:
         return made[key], False
     rows = torch.empty(rounds * places * 8, dtype=torch.int32, device=device)
     fn = _function("elementwise", "omnia_decode_pieces",
-                   [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
-    _check(fn(_ptr(step.seq_lens), step.num_seqs, kv.window or 0, run, nkv, places, rounds, sm_count(device), _ptr(rows), _stream()),
+                   [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
+    _check(fn(_ptr(step.seq_lens), step.num_seqs, kv.window or 0, run, nkv, places, rounds, chain, sm_count(device), _ptr(rows), _stream()),
            "decode_pieces")
     made[key] = rows
     return rows, True
@@ -743,8 +749,8 @@ def paged_attention(q: torch.Tensor | None, kv: KVView, step: StepContext, scale
         # (A list is kept for the layers behind this one, so it takes a pass that begins and ends: a caller that runs a layer by
         # itself may have moved the lengths on since the last call.)
         listable = step.decode_only and warps == 1 and in_pass(step)
-        places, rounds = decode_places(count, nkv, sees, sm_count(q.device)) if listable else (0, 0)
-        pieces, (listed, now) = rounds * places, _decode_list(step, kv, run, nkv, places, rounds, q.device) if places else (None, False)
+        places, rounds = decode_places(count, nkv, sees, sm_count(q.device), d) if listable else (0, 0)
+        pieces, (listed, now) = rounds * places, _decode_list(step, kv, run, nkv, d, places, rounds, q.device) if places else (None, False)
         places = pieces or count * max_chunks  # partial results a head
         part_o, part_ml, tickets = _step_buffers(step, q.device, {
             "attention_part_o": (nq * places * d, torch.float32, False),

@@ -340,6 +340,10 @@ def test_decode_lists_of_pieces_where_there_is_work_for_every_block():
     assert ops.decode_places(8, 8, 4096, 148) == ops.decode_places(5, 8, 4096, 148) == (111, 1)
     assert ops.decode_places(8, 8, 2000, 148) == (0, 0) and ops.decode_places(256, 8, 4096, 148) == (0, 0)
     assert ops.decode_places(64, 8, 2304, 148) == (111, 2)
+    # More requests than places, and few with heads of which an SM holds three blocks, were slower by a list.
+    assert ops.decode_places(100, 8, 700, 148) == ops.decode_places(128, 8, 4096, 148) == (0, 0)
+    assert ops.decode_places(16, 4, 3000, 148, 256) == (0, 0) and ops.decode_places(16, 4, 3000, 148, 128) == (222, 1)
+    assert ops.decode_places(24, 4, 2304, 148, 256) == (222, 1)
 
 
 def _calls_of_decode_attention(monkeypatch):
@@ -369,7 +373,7 @@ def test_a_list_of_pieces_is_the_passes_own(monkeypatch):
     itself, whose caller may have moved the lengths on since the last call."""
     calls = _calls_of_decode_attention(monkeypatch)
     lists = lambda: [args[LIST_ARGUMENT] for name, args in calls if name == "omnia_attention_decode_tc"]  # noqa: E731
-    made = lambda: [args[8] for name, args in calls if name == "omnia_decode_pieces"]  # noqa: E731
+    made = lambda: [args[9] for name, args in calls if name == "omnia_decode_pieces"]  # noqa: E731
     (first, a), (second, b) = _decode_step([3000, 70] * 8), _decode_step([1500] * 16)
     a(), a()
     assert lists() == [None, None] and not made()
