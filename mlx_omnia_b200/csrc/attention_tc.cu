@@ -441,7 +441,7 @@ attention_prefill_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pa
 // be 256 registers, and went by way of 572 bytes of local memory.
 template <int H, int THREADS>
 __device__ __forceinline__ void merge_chunks(const float* __restrict__ part_o, const float* __restrict__ part_ml, size_t base,
-                                             int max_chunks, int chunks, const bf16* __restrict__ gate_row, bf16* __restrict__ out_row,
+                                             int max_chunks, int chunks, const bf16* gate_row, bf16* __restrict__ out_row,
                                              float* stage, const float* __restrict__ sink, const MapDifference difference) {
   const int lane = threadIdx.x & 31, tid = threadIdx.x;
   constexpr int VEC = H * D >= 4 * THREADS ? 4 : 2, PIECES = H * D / VEC, V = (PIECES + THREADS - 1) / THREADS;
@@ -587,18 +587,11 @@ struct FusedQK {
   long long num_slots;
 };
 
-// A piece of a request's keys, as the list that omnia_decode_pieces (elementwise.cu) makes of a step holds it: request of
-// the call (-1: none), its position, the piece's first and last key, its number among the request's pieces and how many
-// these are, and the pieces listed ahead of the request's first.
-struct __align__(16) Piece {
-  int request, pos, lo, hi, index, count, before, unused;
-};
-
 // The list may be written while this kernel already runs (its maker is the launch before it), so to the compiler it must be no
 // read-only memory: as a plain load of a `const __restrict__` argument this one was moved above the wait for the maker, and in
 // replayed steps the first layer worked on the pieces of the replay before.
-__device__ __forceinline__ Piece load_piece(const Piece* piece) {
-  Piece p;
+__device__ __forceinline__ DecodePiece load_piece(const DecodePiece* piece) {
+  DecodePiece p;
   asm volatile("ld.relaxed.gpu.global.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(p.request), "=r"(p.pos), "=r"(p.lo), "=r"(p.hi) : "l"(piece) : "memory");
   asm volatile("ld.relaxed.gpu.global.v4.s32 {%0, %1, %2, %3}, [%4 + 16];"
                : "=r"(p.index), "=r"(p.count), "=r"(p.before), "=r"(p.unused) : "l"(piece) : "memory");
@@ -607,12 +600,12 @@ __device__ __forceinline__ Piece load_piece(const Piece* piece) {
 
 template <int WARPS, int RING, bool CAPPED>
 __global__ void __launch_bounds__(WARPS * 32)
-attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pages,
+attention_decode_kernel(const bf16* q, const bf16* __restrict__ pages,
                         const int* __restrict__ block_table, const int* __restrict__ cu_seqlens,
                         const int* __restrict__ seq_lens, const int* __restrict__ seq_ids,
                         float* __restrict__ part_o, float* __restrict__ part_ml,
-                        int* __restrict__ tickets, const bf16* __restrict__ gate, int gate_stride,
-                        bf16* __restrict__ out, int chunk_keys, int max_chunks, const Piece* list, int pieces,
+                        int* __restrict__ tickets, const bf16* gate, int gate_stride,
+                        bf16* __restrict__ out, int chunk_keys, int max_chunks, const DecodePiece* list, int pieces,
                         int listed_before, int max_pages,
                         int num_pages, int nq, int nkv, int page_size, int window, float scale,
                         const FusedQK fused, int keep_first, const float* __restrict__ sink, int run, float softcap,
@@ -645,7 +638,7 @@ attention_decode_kernel(const bf16* __restrict__ q, const bf16* __restrict__ pag
   int request = blockIdx.z, kvh = blockIdx.y, chunk = blockIdx.x, chunks = 0, seq = 0, pos = -1, first = 0, lo = 0, hi = -1;
   if (WARPS == 1 && pieces > 0) {
     if (listed_before) pdl_wait();  // the list comes from the kernel right before this one
-    const Piece mine = load_piece(list + blockIdx.y);
+    const DecodePiece mine = load_piece(list + blockIdx.y);
     if (mine.request < 0) {
       if (early) pdl_wait();
       return;
@@ -1038,7 +1031,7 @@ extern "C" int omnia_attention_prefill_tc(const void* q, const void* pages, cons
 }
 
 typedef void (*DecodeKernel)(const bf16*, const bf16*, const int*, const int*, const int*, const int*, float*, float*, int*, const bf16*,
-                             int, bf16*, int, int, const Piece*, int, int, int, int, int, int, int, int, float, const FusedQK, int, const float*, int, float,
+                             int, bf16*, int, int, const DecodePiece*, int, int, int, int, int, int, int, int, float, const FusedQK, int, const float*, int, float,
                              const MapDifference, int, int*);
 
 // Shared memory of an SM, the most a block may ask for, and what a block costs beside its dynamic
@@ -1111,7 +1104,8 @@ extern "C" int omnia_attention_decode_tc(const void* q, const void* pages, const
     if (room > smem + BLOCK_OVERHEAD) smem = (room > BLOCK_MOST ? BLOCK_MOST : room) - BLOCK_OVERHEAD;
   }
   // Scores without a cap take kernels without its tanh: 16 of them stand in a tile's straight line of code, and a decode
-  // step fetches every kernel's code anew (a layer's weights have pushed it out of the caches).
+  // step fetches every kernel's code anew (a layer's weights have pushed it out of the caches). One request of 4,096 positions,
+  // eight layers: 347.1 -> 342.2 us a step; eight requests, no difference.
   const DecodeKernel kernel =
       softcap > 0.f ? (warps == 1 ? attention_decode_kernel<1, DECODE_STAGES, true>
                                   : deep ? attention_decode_kernel<4, 2, true> : attention_decode_kernel<4, 1, true>)
@@ -1119,7 +1113,7 @@ extern "C" int omnia_attention_decode_tc(const void* q, const void* pages, const
                                   : deep ? attention_decode_kernel<4, 2, false> : attention_decode_kernel<4, 1, false>);
   launch_pdl(kernel, pieces > 0 ? dim3(nkv, pieces) : dim3(max_chunks, nkv, requests), warps * 32, smem, stream,
       (const bf16*)q, (const bf16*)pages, block_table, cu_seqlens, seq_lens, seq_ids, part_o, part_ml,
-      tickets, (const bf16*)gate, gate_stride, (bf16*)out, chunk_keys, max_chunks, (const Piece*)list, pieces, listed_before, max_pages,
+      tickets, (const bf16*)gate, gate_stride, (bf16*)out, chunk_keys, max_chunks, (const DecodePiece*)list, pieces, listed_before, max_pages,
       num_pages, nq, nkv, page_size, window, scale, fused, keep_first, sink, run, softcap, difference, beside, err);
   return OMNIA_LAUNCH_RESULT();
 }

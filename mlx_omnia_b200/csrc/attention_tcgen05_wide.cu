@@ -8,8 +8,9 @@
 // head and one request, has all of its SM's tensor memory (three score buffers of 128 columns and
 // the accumulator) and walks the visible keys in score tiles of 128:
 //   S = Q K^T   tcgen05.mma (M 128, N 128) over the head size. A product with its 128-row operand in
-//               shared memory occupies the tensor core for 65 to 80 ns however few columns it has, so
-//               a tile of 128 keys costs the eight products that a tile of 64 would
+//               shared memory took 65 to 80 ns however few columns it had (issued by `lane == 0`; not
+//               measured again behind an elected lane), so a tile of 128 keys costs the eight
+//               products that a tile of 64 would
 //   softmax     two teams of four warps, a thread per row in each, take turns with the tiles: one
 //               team's exponentials run while the other reads its scores and finds its maximum. What
 //               a tile needs of the tile before, the exponent's offset, goes through shared memory
@@ -241,8 +242,8 @@ attention_prefill_tcgen05_kernel(const __grid_constant__ CUtensorMap map_q, cons
     }
   } else if (warp == WARP_QK) {
     // ---- issuer of the score products: S[j & 1] = Q K_j^T, 128 keys a tile ----------------------------
-    // A product with the 128-row operand in shared memory occupies the tensor core for 65 to 80 ns
-    // however few columns it has, so a tile of 128 keys costs the eight products that a tile of 64
+    // A product with the 128-row operand in shared memory took 65 to 80 ns however few columns it
+    // had (where `lane == 0` issued it), so a tile of 128 keys costs the eight products that a tile of 64
     // did. The two kinds of product are issued by two threads (this warp and the next), so the scores'
     // chain and the values' chain run side by side. What one thread's products must wait for of the
     // other's goes through barriers: a score buffer is written again only when the products that read

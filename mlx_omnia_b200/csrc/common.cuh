@@ -117,11 +117,10 @@ __device__ __forceinline__ bool omnia_mbar_test(uint32_t bar, uint32_t parity) {
 }
 
 // One lane of the warp (the same one every time). Whoever issues tensor-core products or bulk copies branches on this and not on
-// `lane == 0`: those instructions take their descriptors and addresses from registers that a warp shares, and only of a
-// branch on an elected lane does the compiler know that one thread runs it; for any other it writes a loop over the lanes
-// that may be there, around every one of them. (So, against `lane == 0`, of the cases of whole steps: a prompt of 2,048 tokens 7,190 -> 6,870 us,
-// 8,192 tokens through the 8-billion model in portions 128.4 -> 124.0 ms; attention of 1,082 ragged rows 24.1 -> 19.6 us a layer,
-// the one-SM product of 1,082 x 12,288 x 2,048 59 -> 51.)
+// `lane == 0`: those instructions take their descriptors and addresses from registers that a warp shares, and of a branch on an
+// elected lane the compiler knows that one thread runs it. What was timed is the effect: by this alone
+// a prompt of 2,048 tokens 7,222 -> 7,033 us (median of three runs each, 1 % apart), 8,192 tokens through the 8-billion model in
+// portions 130.6 -> 126.3 ms, five short prompts no difference; attention of 1,082 ragged rows 24.1 -> 19.6 us a layer.
 __device__ __forceinline__ bool omnia_elect_one() {
   uint32_t one;
   asm volatile(
@@ -135,12 +134,23 @@ __device__ __forceinline__ bool omnia_elect_one() {
 __device__ __forceinline__ int omnia_warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 
 // The cache policy of what is read once a step, a product's weights and the cache's keys and values: such lines leave L2
-// first, so that a step's stream of gigabytes does not push out what the next layer needs again.
+// first, so that a step's stream of gigabytes does not push out what the next layer needs again. (On the products' weights alone:
+// eight layers of 2,048, eight requests of 4,096 positions 526 -> 514 us a step, one request 344 -> 342. Models that L2 could hold
+// lose less than they gain: three of 30 to 100 MB, one, eight and sixteen requests of 500 positions, 1.1 % slower to 2.8 % faster;
+// a matrix of 50 MB read again and again by nothing but its product 8.5 -> 8.9. Experts whose matrix is read again for more rows
+// than an entry has: 62.1 -> 59.8, 78.2 -> 75.5, 54.0 -> 54.7.)
 __device__ __forceinline__ uint64_t omnia_read_once_policy() {
   uint64_t policy;
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(policy));
   return policy;
 }
+
+// A piece of a request's keys, as decode_pieces_kernel (elementwise.cu) lists those of a step and the decode attention kernel
+// (attention_tc.cu) takes them, a block each: request of the call (-1: none), its position, the piece's first and last key, its
+// number among the request's pieces and how many these are, and the pieces listed ahead of the request's first.
+struct __align__(16) DecodePiece {
+  int request, pos, lo, hi, index, count, before, unused;
+};
 
 // Programmatic dependent launch. A kernel launched through launch_pdl may begin while the kernel
 // before it in the stream is still running; it must call pdl_wait() before it touches anything an
@@ -152,6 +162,8 @@ __device__ __forceinline__ uint64_t omnia_read_once_policy() {
 // an SM where the first kernel still runs, and later find in L1, through a cached load, lines
 // that the first kernel's blocks fetched from memory which has since been freed, handed out
 // again and rewritten. That was seen as a rare wrong token.)
+// What an earlier kernel writes is no `const __restrict__` argument where the wait for that kernel stands under a condition: the
+// compiler may take such memory as never written and load from it ahead of the wait. That was seen too.
 #ifndef OMNIA_TIMELINE
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 #define OMNIA_TRACE_BLOCK(phase) do { } while (0)

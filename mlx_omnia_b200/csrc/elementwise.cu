@@ -1134,12 +1134,9 @@ extern "C" int omnia_fill_slots(const void* const* to, const void* const* from, 
 // Lengths are on the device alone in a replayed step, hence a kernel, once for all layers that see as far: one block, a warp
 // for each of the two to find its size, a thread for each request to list its parts.
 constexpr int PIECE_LEAST = 4, PIECE_ROUNDS = 2, PIECE_WAVE = 13, PIECE_THREADS = 256;
-struct __align__(16) Piece {  // (as attention_tc.cu reads it)
-  int request, pos, lo, hi, index, count, before, unused;
-};
 __global__ void __launch_bounds__(PIECE_THREADS)
 decode_pieces_kernel(const int* __restrict__ seq_lens, int requests, int window, int run, int nkv, int places, int rounds, int chain, int sms,
-                     Piece* __restrict__ list) {
+                     DecodePiece* __restrict__ list) {
   __shared__ int tiles[PIECE_THREADS], parts[PIECE_THREADS], sizes[PIECE_THREADS];
   __shared__ int found[PIECE_ROUNDS], cost[PIECE_ROUNDS];
   pdl_wait();
@@ -1190,7 +1187,7 @@ decode_pieces_kernel(const int* __restrict__ seq_lens, int requests, int window,
   const int base = count > 0 ? mine / count : 0, longer = count > 0 ? mine - base * count : 0;  // the first `longer` parts have a tile more
   for (int i = 0; i < count; ++i) {
     const int tile = first / 32 + i * base + min(i, longer), next = tile + base + (i < longer);
-    list[before + i] = Piece{r, pos, max(first, tile * 32), min(pos, next * 32 - 1), i, count, before, 0};
+    list[before + i] = DecodePiece{r, pos, max(first, tile * 32), min(pos, next * 32 - 1), i, count, before, 0};
   }
   for (int i = all + r; i < places * rounds; i += PIECE_THREADS) list[i].request = -1;
 }
@@ -1201,6 +1198,6 @@ extern "C" int omnia_decode_pieces(const int* seq_lens, int requests, int window
   if (requests < 1 || requests > PIECE_THREADS || places < 1 || rounds < 1 || rounds > PIECE_ROUNDS || requests > rounds * places || chain < 0 || sms < 1 ||
       nkv < 1 || ((uintptr_t)list & 15))
     return (int)cudaErrorInvalidValue;
-  launch_pdl(decode_pieces_kernel, 1, PIECE_THREADS, 0, stream, seq_lens, requests, window, run, nkv, places, rounds, chain, sms, (Piece*)list);
+  launch_pdl(decode_pieces_kernel, 1, PIECE_THREADS, 0, stream, seq_lens, requests, window, run, nkv, places, rounds, chain, sms, (DecodePiece*)list);
   return OMNIA_LAUNCH_RESULT();
 }

@@ -120,8 +120,8 @@ __device__ __forceinline__ void tmem_load32(uint32_t addr, uint32_t* v) {
 
 
 constexpr int STAGES = 6;
-// The accumulator has 256 columns whatever the shape: an instruction of 256 rows takes some 80 ns with 256, 192, 128 or
-// 64 columns alike (a wave of tiles 2,048 deep 10.4 / 12.2 / 10.0 / 9.6 us), so narrower tiles only add waves
+// The accumulator has 256 columns whatever the shape: an instruction of 256 rows took some 80 ns with 256, 192, 128 or
+// 64 columns alike where `lane == 0` issued it (a wave of tiles 2,048 deep 10.4 / 12.2 / 10.0 / 9.6 us), so narrower tiles only add waves
 // (2,048 x 12,288 x 2,048: 86 us with tiles of 192, whose last wave is fuller, 78 with 256; x 24,576 x 4,096: 313 and 280).
 // Clusters of two pairs that share a's rows by multicast, a quarter less out of L2, measured the same a wave (and the
 // device holds 33 of them, 66 pairs of 74). Each block stages TILE_N / 2 rows of w.

@@ -325,10 +325,12 @@ def decode_plan(requests: int, nkv: int, longest: int, sms: int) -> tuple[int, i
     tile counts one and a half); at some 244 registers a thread two such blocks fit an SM (plans
     made for three ran in one and a half waves, and badly). The cost of a plan, in tile times:
     waves x (4 for a block's start and its partial result + tiles per warp), for four-warp blocks
-    divided by the share of the SMs' places that they fill, + a round trip of the merge per eight
-    chunks; the plan is the cheapest chunk (a multiple of 64 keys, 128 to 1024), the shorter on a
-    tie. Its pick was the best or within 2 % of the best of the plans tried at 4,096 positions
-    (batches 1 to 16) and at 16,000 and 32,000 (batches 1 and 2), on a GPU of 148 SMs (`sms`)."""
+    divided by the share of the SMs' places that they fill, + one per eight chunks for their merge (a
+    weight that was fitted; the merge takes sixteen chunks a round); the plan is the cheapest chunk (a
+    multiple of 64 keys, 128 to 1024), the shorter on a tie. Whole steps of eight layers, its pick against
+    the best of fourteen chunk lengths, on a GPU of 148 SMs (`sms`): the best or within 1.2 % at 4,096 positions (batches 1, 2, 4
+    and 8), 4 requests of 1,000, 8 of 500, 1 of 16,000, 1 and 2 of 32,000; 2.1 % behind at 2 of 16,000, 5.3 % at 16 of 4,096 (which
+    a decode-only step runs by a list, `decode_places`)."""
     pairs = (1 << max(requests - 1, 0).bit_length()) * max(nkv, 1)
     longest = max(longest, 1)
     warps, per_sm, tile = (4, 2, 1.5) if pairs * 8 <= sms else (1, 6, 1.0)
@@ -579,13 +581,14 @@ def wide_prefill_pays(q_lens, seq_lens, tokens_per_block: int, nkv: int, window:
     SM and cuts long blocks into parts (attention_tcgen05.cu).
 
     Measured on a B200 (16 query and 8 key/value heads of 128, with the gate; us, wide against two to
-    an SM; a prompt of n tokens makes n / 64 blocks per key/value head): one whole prompt of 512 / 1,024
-    / 2,048 / 2,304 tokens 17 / 19 / 37 / 42 against 22 / 24 / 44 / 52 (few blocks, each a long chain of
-    tiles, which a block alone on its SM walks at 1.16 us for 128 keys against 1.06 us for 64), of
-    2,560 / 2,816 / 3,072: 53 / 61 / 68 against 57 / 60 / 65, of 4,096 / 8,192: 101 / 323 against 88 / 290
-    (a block's 7 us of start and epilogue overlap nothing when it has its SM alone); 2 prompts of 768
-    or of 1,024, 4 of 512: even; 2 of 1,536, 3 of 1,024 (384 blocks): 48 / 40 against 39 / 31; 8
-    portions of 256 over 1,024: 36 against 31; 512 over 8,192 cut into parts: 75 against 57. So:
+    an SM; a prompt of n tokens makes n / 64 blocks per key/value head), products and boxes issued by an
+    elected lane: one whole prompt of 512 / 1,024 / 2,048 / 2,304 tokens 15.7 / 18.6 / 34.6 / 38.2 against
+    16.2 / 24.8 / 41.2 / 47.1 (few blocks, each a long chain of tiles), of 2,560 / 2,816 / 3,072: 49 / 56 / 62
+    against 50 / 54 / 59, of 4,096 / 8,192: 94 / 326 against 81 / 311 (a block's start and epilogue
+    overlap nothing when it has its SM alone); 2 of 1,536, 3 of 1,024 (384 blocks): 44 / 37 against 36 / 30.
+    The line was drawn where `lane == 0` issued, when 2 prompts of 768 or of 1,024 and 4 of 512 were even; now
+    these are 23.9 / 27.6 / 22.1 against 22.1 / 26.9 / 18.5, and it could be drawn closer. Measured then only:
+    8 portions of 256 over 1,024 36 against 31; 512 over 8,192 cut into parts 75 against 57. So:
     prompts from their first token, each of at least WIDE_MIN_TOKENS tokens, at most two blocks to an
     SM, and no window shorter than WIDE_MIN_WINDOW. The answer depends on the step's lengths and on
     whether its prompts start at zero, both of which a captured step's key holds."""
@@ -900,22 +903,25 @@ SKINNY_ROWS = 16
 FUSED_GATE_ROWS = 320
 FUSED_CAP_ROWS = 129
 """From these many rows on, the products that have an epilogue fused into them (gate‖up with SwiGLU;
-the head with its soft cap) run on this package's tcgen05 kernels. Measured on B200 inside replayed
-graphs (weights of 8 to 50 MB, fresh for every launch): gate‖up with SwiGLU takes 46.7 us at 1,024
-rows, 87.5 at 2,048 and 305 at 8,192, against 58.7, 112 and 408 for the vendor library's product
-followed by the SwiGLU kernel; at 384 / 512 / 640 / 768 / 896 rows 24.3 / 31.0 / 34.6 / 35.0 / 46.3
-against 26.7 / 33.8 / 41.5 / 43.0 / 55.5 (the kernel with one SM or two to a tile, whichever runs fewer
-waves: `_pair_pays`); at 264 rows the library's pair is the faster one (23.3 against 24.1 us).
+the head with its soft cap) run on this package's tcgen05 kernels. Measured on B200 in captured chains
+of one product (12,288 x 2,048, eight matrices in turn), products issued by an elected lane: gate‖up with SwiGLU
+takes 40.1 us at 1,024 rows, 74.2 at 2,048 and 284 at 8,192, against 46.3, 86.1 and 374 for the vendor library's
+product followed by the SwiGLU kernel; at 320 / 384 / 512 / 640 / 768 / 896 rows 23.9 / 23.9 / 27.2 / 29.9 / 32.1 / 40.0
+against 20.4 / 20.6 / 25.3 / 32.2 / 34.2 / 49.7 (the kernel with one SM or two to a tile, whichever `_pair_pays`
+names), at 264 23.6 against 18.0. The line of 320 comes from whole replayed steps, before the lane was elected
+(384 / 512 rows 24.3 / 31.0 against 26.7 / 33.8); alone in a chain the library is ahead up to 512 rows, and the line is
+due to be drawn again in whole steps. The head with its cap (151,936 x 2,048): 256 / 512 rows 197 / 333 us against 214 / 329;
+at 129 and 192 rows, where one SM has a tile, 317 / 347 against 153 / 174 for the library's: that line, too.
 
 A product with nothing fused into it is the vendor library's above the streaming kernel's rows, as the
 reference's is MLX's. The tcgen05 kernels take the same products (`_gemm_tcgen05`, tested), but the
-library is ahead at every size measured: by 3 to 10 % at 2,048 to 4,096 rows (38.5 against 39.6 us
-for 2,048 x 6,144 x 2,048), by 1.3 to 2.8 times between 129 and 1,024 rows, where 128 x 256 tiles
-are too few for the SMs (12.1 against 33.8 us for 264 x 2,048 x 6,144), and by 10 to 28 % at 8,192.
+library is ahead up to 2,048 rows: 37.3 against 42.6 us for 2,048 x 6,144 x 2,048, 21.0 against 27.6 for
+1,082, and 16.2 against 28.0 for 264 x 2,048 x 6,144, where 128 x 256 tiles are too few for the SMs. With the lane elected
+the pair kernel is now ahead at 4,096 rows (80.8 against 83.0) and 8,192 (145 against 165); the rule has not followed.
 Two kernels of this package's own for the rows in between were built, right and deterministic, and
-not kept: the weights as the 128-row operand of tcgen05.mma with the few activation rows as its
-columns (a tcgen05.mma with M = 128 occupies the tensor core for some 80 ns however few columns it
-has, so the weights stream at half the rate of 256-column tiles), and the k range of a 128 x 256 tile
+not kept, both where `lane == 0` issued the products: the weights as the 128-row operand of tcgen05.mma with the
+few activation rows as its columns (a product with M = 128 took some 80 ns however few columns it
+had, so the weights streamed at half the rate of 256-column tiles), and the k range of a 128 x 256 tile
 cut over a thread-block cluster (the exchange of partial sums, 128 KB a block, costs what the cut
 saves: 10.6 to 32 us against the library's 8 to 12)."""
 
@@ -939,19 +945,20 @@ def _tensor_core(a: torch.Tensor, weight: torch.Tensor, rows: int) -> bool:
 def _pair_pays(rows: int, n: int, k: int, epilogue: int, sms: int) -> bool:
     """Whether the two-SM kernel is the faster one: it brings in a third less per step of k, but
     has half as many (twice as large) tiles to hand out and a longer start. Measured on a GPU of
-    148 SMs it wins by 4 to 13 % where a pair of SMs gets at least 64 steps of k of a 256 x 256
-    tile to do (2,048 rows of 2,048 columns times 6,144 or more; 8,192 rows: all), and loses where
-    the work is less (2,048 x 2,048 x 2,048; 512 rows)."""
+    148 SMs it wins by 6 to 21 % where a pair of SMs gets at least 64 steps of k of a 256 x 256
+    tile to do (rows x columns x depth, one SM / a pair, us, 2,048 x 6,144 x 2,048 49.3 / 42.6, 2,048 x 2,048 x 6,144 46.1 / 43.3,
+    8,192 x 6,144 x 2,048 182.7 / 145.2), and is even or loses where the work is less (2,048 x 2,048 x 2,048 17.1 / 16.6,
+    512 x 6,144 x 2,048 18.4 / 17.8, 264 x 6,144 x 2,048 11.5 / 17.0, 1,082 x 2,048 x 6,144 25.9 / 45.3)."""
     if rows < 256:
         return False
     if epilogue == 1:
         # gate|up with SwiGLU: tiles of 128 output columns, 128 rows to an SM or 256 to a pair. What
-        # decides is how many waves of tiles each kernel runs (measured, 12,288 weight rows of 2,048:
-        # some 10 us and 14 a wave for one SM, 9 and 11 a wave for a pair; 512 / 1,082 rows: 38 / 53 us
-        # against 29.6 / 52). A pair's wave counts as 12, and the depth is not asked: where pairs run one wave more than
+        # decides is how many waves of tiles each kernel runs (fitted where `lane == 0` issued, 12,288 weight rows of 2,048:
+        # some 10 us and 14 a wave for one SM, 9 and 11 a wave for a pair; now 512 / 1,082 rows 37.0 / 53 to 55 us
+        # against 27.2 / 50 to 52). A pair's wave counts as 12, and the depth is not asked: where pairs run one wave more than
         # a few, shallow products would gain by them and deep ones lose, and one SM keeps them all (one SM / a pair, us,
-        # 1,024, 2,048, 4,096 and 8,192 deep: 1,082 x 12,288 39 / 32, 53 / 52, 93 / 99, 194 / 209; 896 x 24,576 63 / 44,
-        # 93 / 80, 167 / 163, 342 / 335).
+        # 1,024, 2,048, 4,096 and 8,192 deep: 1,082 x 12,288 37.5 / 29.6, 53.0 / 51.5, 93.9 / 98.2, 176 / 179; 896 x 24,576
+        # 66.7 / 44.5, 91.6 / 74.7, 163 / 145, 311 / 292).
         tiles = -(-(n // 2) // 128)
         one = -(-(-(-rows // 128) * tiles) // sms)
         two = -(-(-(-rows // 256) * tiles) // (sms // 2))
@@ -1056,10 +1063,9 @@ FUSED_QKV_ROWS = 1280
 """From how many rows on the attention input projection runs on the two-SM tcgen05 kernel with the
 head norms, the rotation and the cache write in its epilogue, instead of the library's product and
 the kernel that reads its result back. B200, rows x 2,048 -> 6,144, us for the two against the one
-(without the 3 us of the angles' table, which a pass makes once for all its layers): 768 rows 22.7
-against 23.2, 1,024: 29.4 against 29.7, 1,280: 34.8 against 31.2, 1,536: 37.2 against 31.7, 2,048:
-50.7 against 42.9, 4,096: 94.0 against 80.8, 8,192: 182.7 against 154.8 (the bare products at
-2,048 rows: 38.8 us for this kernel, 37.3 for the library's)."""
+(without the 2 to 7 us of the angles' table, which a pass makes once for all its layers), products issued by an
+elected lane: 512 rows 18.2 against 20.2, 640: 20.0 / 20.2, 768: 21.7 / 20.4, 896: 27.4 / 27.8, 1,024: 27.8 / 27.9, 1,082:
+28.2 / 28.2, 1,280: 33.8 / 28.8, 1,536: 36.0 / 31.0, 2,048: 51.0 / 43.3, 4,096: 101 / 78, 8,192: 213 / 175."""
 
 
 def linear_qkv(x, weight: torch.Tensor, q_col: int, k_col: int, v_col: int, nq: int, nkv: int, d: int,
@@ -2076,10 +2082,11 @@ would leave most of every tile empty); below, on the mma.sync kernel with tiles 
 def _moe_pair_pays(pairs: int, experts: int, columns: int, sms: int) -> bool:
     """Whether the experts' grouped tcgen05 products take tiles of 256 rows, two SMs to a tile, rather than of 128
     (`columns`: 128 of the first product's per tile). A wave of them brings in a third less, but an expert's last tile
-    is twice as empty. Experts of 137 to 256 rows fill one such tile or two of the others: 0.86 to 0.98 of the time with
-    8 to 128 experts of 512 to 1,536; at 112 to 128 rows, one tile of either, 1.00 to 1.08, at 280 to 350 rows, two
-    against three, 1.0 to 1.07. Further up (0.81 to 0.98) what is left is the waves, as for a dense product: with 8
-    experts of 512 rows three of these against two of the others, 84 us and 78."""
+    is twice as empty. Experts of 137 to 256 rows fill one such tile or two of the others: 0.81 to 0.96 of the time with
+    8 to 128 experts of 512 to 1,536; at 112 to 128 rows, one tile of either, 0.99 and 0.83 with 8 experts, 1.07 and 1.02 with 32, at
+    300 to 350 rows, two against three, 0.93 to 0.94 and 0.96 to 1.02. Further up what is left is the waves, as for a dense
+    product: 400 rows 0.83 and 0.84, 512 rows 0.98 with 8 experts (left to one SM) and 1.07 with 32 (given to two: the fit of
+    the waves is from before the products' lane was elected, as is the line at 136)."""
     rows = pairs / experts
     if rows < 384:
         return 136 <= rows <= 256
@@ -2092,10 +2099,10 @@ def _moe_stream_rows(rows: int, pairs: int, experts: int, hidden: int, inner: in
     """Rows of an entry (8 or 16) where the experts' bfloat16 products stream the weights as a decode step's dense
     products do, 0 where they take mma.sync tiles. An expert with more rows than an entry has its matrix read again for
     the next one; entries of 16 multiply twice as much for every weight and take 1.1 to 1.2 times as long, until second
-    entries come often: from 7 pairs an expert on (8 of 32 experts of 2,048 x 768: 78 us with eight, 73 with sixteen, 81
-    on mma.sync tiles; 6: 65, 71, 78), and not at all above 8, unless 16 rows in all leave no expert more than an entry.
-    Small matrices pay for an entry's start: above 6 pairs they stay with the tiles (64 experts of 512 x 512 at 8: 51
-    and 47 us), and inner widths under 512, which fill less than half of the second product's stages, stream only
+    entries come often: from 7 pairs an expert on (8 of 32 experts of 2,048 x 768, weights loaded evict-first: 7 pairs 72.0 us with eight,
+    71.8 with sixteen, 79.7 on mma.sync tiles; 8: 75.5, 72.1, 80.3; 6: 65.1, 70.8, 79.5), and not at all above 8, unless 16 rows in
+    all leave no expert more than an entry. Small matrices pay for an entry's start: above 6 pairs they stay with the tiles (64
+    experts of 512 x 512 at 8: 49.5 and 45.6 us), and inner widths under 512, which fill less than half of the second product's stages, stream only
     few pairs (256 of 1,024 x 256, 64 pairs: 49 against 51, 128: 67 against 60; 64 of 4,096 x 256, 256 pairs: 124, 110)."""
     if inner < 512 and pairs > inner // 4:
         return 0
