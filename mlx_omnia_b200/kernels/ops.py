@@ -302,6 +302,14 @@ def _step_buffers(step: StepContext, device: torch.device, wanted: dict) -> list
     return buffers
 
 
+def _pass_buffer(step: StepContext, device: torch.device, name: str, numel: int, dtype: torch.dtype) -> torch.Tensor:
+    """Memory for what a kernel makes once for the layers of a pass, which no other step may write: a tensor of its own, or, for a
+    step captured into a graph, one that its workspace has kept since the pass before the capture."""
+    if (step.workspace or {}).get("private"):
+        return _step_buffers(step, device, {name: (numel, dtype, False)})[0]
+    return torch.empty(numel, dtype=dtype, device=device)
+
+
 def width_bucket(pages: int) -> int:
     """`pages` (of the longest block table of a step) rounded up to three significant bits, at
     least 8: the widths that captured decode graphs are made for, and the bound that the decode
@@ -346,9 +354,9 @@ def decode_plan(requests: int, nkv: int, longest: int, sms: int) -> tuple[int, i
     return best
 
 
-PIECE_REQUESTS, PIECE_TILES = 256, 5
-"""The most requests a list of pieces is made for (the kernel's), and the tiles of 32 keys a block from which on decode
-attention runs by such a list."""
+PIECE_REQUESTS, PIECE_TILES, PIECE_INTS = 256, 5, 8
+"""The most requests a list of pieces is made for (the kernel's), the tiles of 32 keys a block from which on decode
+attention runs by such a list, and the ints of a piece (`DecodePiece` in common.cuh)."""
 
 
 def decode_places(requests: int, nkv: int, longest: int, sms: int, d: int = 128) -> tuple[int, int]:
@@ -384,7 +392,7 @@ def _decode_list(step: StepContext, kv: KVView, run: int, nkv: int, d: int, plac
     key = ("decode_list", kv.window or 0, run, nkv, chain)
     if key in made:
         return made[key], False
-    rows = torch.empty(rounds * places * 8, dtype=torch.int32, device=device)
+    rows = _pass_buffer(step, device, "_".join(map(str, key)), rounds * places * PIECE_INTS, torch.int32)
     fn = _function("elementwise", "omnia_decode_pieces",
                    [c_void_p, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p])
     _check(fn(_ptr(step.seq_lens), step.num_seqs, kv.window or 0, run, nkv, places, rounds, chain, sm_count(device), _ptr(rows), _stream()),
@@ -1052,7 +1060,7 @@ def rope_angles(step: StepContext, inv_freq: torch.Tensor) -> torch.Tensor:
     table = made.get(key)
     if table is None:
         half = inv_freq.shape[0]
-        table = torch.empty(half, step.num_tokens, 2, dtype=torch.float32, device=inv_freq.device)
+        table = _pass_buffer(step, inv_freq.device, f"rope_angles_{inv_freq.data_ptr()}", half * step.num_tokens * 2, torch.float32)
         fn = _function("elementwise", "omnia_rope_angles", [c_void_p, c_void_p, c_int, c_int, c_void_p, c_void_p])
         _check(fn(_ptr(step.positions), _ptr(inv_freq), half, step.num_tokens, _ptr(table), _stream()), "rope_angles")
         made[key] = table

@@ -399,7 +399,21 @@ def test_a_table_of_angles_is_the_passes_own(monkeypatch):
     ops.begin_pass(a), ops.begin_pass(b)
     tables = [ops.rope_angles(step, inv) for step in (a, b, a, b)]
     assert len(calls) == 4 and tables[0] is tables[2] and tables[1] is tables[3]
-    assert tables[0].data_ptr() != tables[1].data_ptr() and tables[0].shape == (4, 9, 2)
+    assert tables[0].data_ptr() != tables[1].data_ptr() and tables[0].numel() == 4 * 9 * 2
     ops.end_pass(a)
     ops.rope_angles(a, inv)
     assert len(calls) == 5
+
+
+def test_a_captured_step_keeps_what_a_pass_makes_where_the_pass_before_made_it(monkeypatch):
+    """Nothing that a graph's kernels share between layers is allocated by the capture."""
+    monkeypatch.setattr(ops, "_function", lambda *a, **b: lambda *args: 0)
+    monkeypatch.setattr(ops, "_stream", lambda: 0)
+    monkeypatch.setattr(ops, "sm_count", lambda device=None: 148)
+    step = SimpleNamespace(num_tokens=9, num_seqs=9, positions=torch.arange(9), seq_lens=torch.arange(9), workspace={"private": True})
+    kv, inv, made = KVView(torch.zeros(1, 2, 8, 16, 128), None, None, 16, None), torch.ones(4), []
+    for _ in range(2):
+        ops.begin_pass(step)
+        made.append((ops.rope_angles(step, inv), ops._decode_list(step, kv, 0, 8, 128, 111, 1, torch.device("cpu"))[0]))
+        ops.end_pass(step)
+    assert all(a is b for a, b in zip(*made))
