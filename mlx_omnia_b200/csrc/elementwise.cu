@@ -1131,6 +1131,7 @@ extern "C" int omnia_fill_slots(const void* const* to, const void* const* from, 
 // layers with heads of 64 took 755 us, with it 648 (by chunks 652); heads of 128: 918, 867 (884).
 // PIECE_WAVE from 0 to 52 and PIECE_LEAST from 1 to 8 made no difference beyond 1 % (16 to 100 requests of unequal lengths,
 // two models), PIECE_LEAST 16 cost 6 to 12 %.
+// (Positions kept in sight below a window are not counted: a request's first piece has their few tiles on top of its own.)
 // Lengths are on the device alone in a replayed step, hence a kernel, once for all layers that see as far: one block, a warp
 // for each of the two to find its size, a thread for each request to list its parts.
 constexpr int PIECE_LEAST = 4, PIECE_ROUNDS = 2, PIECE_WAVE = 13, PIECE_THREADS = 256;
